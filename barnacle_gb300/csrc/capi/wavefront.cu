@@ -1,5 +1,5 @@
 // Wavefront render orchestration: path-state buffers, the CUDA graph whose while-node runs the
-// whole bounce loop on the device, the host-driven fallback loop, and the launch autotuner.
+// whole bounce loop on the device, the host-driven fallback loop, and the rule for the pool's size.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -24,9 +24,6 @@ struct WfState {
   bool graph_failed = false;
   bn::WfLaunch shape{};
   int shape_cap = -1;
-  // autotuned choice per uploaded scene and triangle test (index: watertight)
-  long long tuned_generation[2] = {-1, -1};
-  int tuned_pool[2] = {0, 0}, tuned_cap[2] = {0, 0}, tuned_refill[2] = {16, 16};
   // the PSSMLT iteration's second stream and its fork / join events (made on first use)
   bn::WfFork fork{nullptr, nullptr, nullptr};
 
@@ -88,6 +85,17 @@ cudaError_t ensure_pool(WfState* w, int pool) {
   return cudaSuccess;
 }
 
+// Path slots of a render that does not choose them: one per path, up to 64 M (15 GB).  Every path
+// then starts at once, the queues are as long and the sorted rays as coherent as they can be, and
+// a bounce is one iteration; fewer slots cost more, short iterations, more slots only add rows to
+// scan.  Measured (kernel ms by log2 of the slots, the render's paths in brackets): Cornell box
+// [2^22] 20: 7.04, 21: 6.47, 22: 6.17, 23: 6.70; Cornell with objects [2^23] 21: 25.2, 22: 23.1,
+// 23: 22.7, 24: 23.8; 16 instanced views [2^25.8] 23: 292, 24: 283, 25: 278, 26: 278.  A cap of 2
+// blocks per SM was 1.8 times slower at every one of them.
+int default_pool(long long paths) {
+  return static_cast<int>(std::min<long long>(1LL << 26, (paths + 1023) / 1024 * 1024));
+}
+
 // the while-node graph of the path tracer: body = one iteration (regen, extend, shade, shadow,
 // control)
 int build_graph(bn_context* ctx, WfState* w) {
@@ -124,9 +132,9 @@ int build_graph(bn_context* ctx, WfState* w) {
   return BN_OK;
 }
 
-// One render (or a truncated tuning render) into w->film_acc / ctx->film.
+// One render into w->film_acc / ctx->film.
 int run(bn_context* ctx, WfState* w, const bn_render_desc* d, long long n_pixels, long long total_paths, int n_views,
-        int pool, int cap, int refill, bool use_graph, float* ms_out) {
+        int pool, int cap, bool use_graph) {
   cudaError_t e;
   if ((e = ensure_pool(w, pool)) != cudaSuccess) return ctx->cuda_fail(e, "wavefront path-state allocation");
   if ((e = w->film_acc.reserve(static_cast<size_t>(n_pixels) * 3 * sizeof(double))) != cudaSuccess)
@@ -158,9 +166,10 @@ int run(bn_context* ctx, WfState* w, const bn_render_desc* d, long long n_pixels
   p.frame_id = d->frame_id;
   p.integrator = d->integrator;
   p.pool = pool;
-  // refill thresholds (lanes of 32 still walking; autotuned, 16 unless told otherwise)
-  p.refill_extend = refill;
-  p.refill_shadow = refill;
+  // lanes of 32 still walking when a traversal warp refills (12 / 16 / 20 / 24 measured 192.9 /
+  // 193.7 / 191.6 / 187.8 M paths/s on the instanced workload, when the mode vote came in)
+  p.refill_extend = 16;
+  p.refill_shadow = 16;
   p.total_paths = total_paths;
   p.n_pixels = n_pixels;
   p.max_iters = static_cast<int>(std::min<long long>(1LL << 30, (total_paths / pool + 2) * (d->max_depth + 2) + 64));
@@ -241,7 +250,6 @@ int run(bn_context* ctx, WfState* w, const bn_render_desc* d, long long n_pixels
   ctx->stats.last_kernel_ms = ms_all;
   ctx->stats.last_dominant_ms = ms_loop;
   ctx->stats.last_launches = launches + 1;
-  if (ms_out) *ms_out = ms_all;
   return BN_OK;
 }
 
@@ -367,51 +375,19 @@ int render_wavefront(bn_context* ctx, const bn_render_desc* d, const std::vector
     total += static_cast<long long>(v.width) * v.height * d->spp;
   }
   const bool use_graph = !(d->flags & BN_RENDER_NO_GRAPH);
-  int pool = d->queue_capacity, cap = d->block_size;  // block_size doubles as the blocks/SM cap
-  int refill = 16;
-  if (pool <= 0 && cap <= 0 && !(d->flags & BN_RENDER_COUNT)) {  // a counting render is a one-off: no tuning
-    const int wt = (d->flags & BN_RENDER_WATERTIGHT) ? 1 : 0;
-    if (w->tuned_generation[wt] != ctx->scene_generation) {
-      // autotune on a truncated render of the same views: pool size (the queue width) x
-      // blocks-per-SM cap, then the lanes a traversal warp refills at (the width of its batch)
-      const int pools[7] = {1 << 20, 1 << 21, 1 << 22, 1 << 23, 1 << 24, 1 << 25, 1 << 26};
-      const int caps[2] = {0, 2};
-      const int refills[3] = {16, 12, 20};
-      const long long sample = std::min<long long>(total, 128LL << 20);  // two fills of the largest pool
-      float best = 1e30f;
-      w->tuned_refill[wt] = 16;
-      for (int pi : pools)
-        for (int ci : caps) {
-          // a pool larger than the paths it would hold only adds slots to scan
-          if (pi > (1 << 20) && pi > sample) continue;
-          float ms = 0.f;
-          const int rc = run(ctx, w, d, pixels, sample, static_cast<int>(views.size()), pi, ci, 16, use_graph, &ms);
-          if (rc) return rc;
-          if (ms < best) {
-            best = ms;
-            w->tuned_pool[wt] = pi;
-            w->tuned_cap[wt] = ci;
-          }
-        }
-      for (int k = 1; k < 3; ++k) {
-        float ms = 0.f;
-        const int rc = run(ctx, w, d, pixels, sample, static_cast<int>(views.size()), w->tuned_pool[wt],
-                           w->tuned_cap[wt], refills[k], use_graph, &ms);
-        if (rc) return rc;
-        if (ms < best) {
-          best = ms;
-          w->tuned_refill[wt] = refills[k];
-        }
-      }
-      w->tuned_generation[wt] = ctx->scene_generation;
-    }
-    pool = w->tuned_pool[wt];
-    cap = w->tuned_cap[wt];
-    refill = w->tuned_refill[wt];
-  }
-  if (pool <= 0) pool = 1 << 20;
+  const int cap = d->block_size;  // block_size doubles as the blocks/SM cap
+  int pool = d->queue_capacity;
+  if (pool <= 0) pool = default_pool(total);
   pool = std::max(pool, 1024);
-  const int rc = run(ctx, w, d, pixels, total, static_cast<int>(views.size()), pool, cap, refill, use_graph, nullptr);
+  if (d->queue_capacity <= 0) {
+    // a default pool gives way on a GPU whose memory others hold
+    cudaError_t e;
+    while ((e = ensure_pool(w, pool)) == cudaErrorMemoryAllocation && pool > (1 << 20)) {
+      cudaGetLastError();
+      pool >>= 1;
+    }
+  }
+  const int rc = run(ctx, w, d, pixels, total, static_cast<int>(views.size()), pool, cap, use_graph);
   if (rc) return rc;
   ctx->stats.paths += static_cast<uint64_t>(total);
   return BN_OK;

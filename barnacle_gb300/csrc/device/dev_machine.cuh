@@ -1,0 +1,170 @@
+// The path machine: whole paths on persistent lanes.
+//
+// A loop that runs a path per thread (trace, shade, trace a shadow ray, next bounce) keeps a warp
+// at every step until its slowest lane is through: on the Cornell box 6 of 32 lanes were active
+// per instruction, in PSSMLT's chains 4.  Here each lane is a small state machine that always
+// holds a walk (a closest hit or a shadow ray, of whatever bounce of whatever path), and the warp
+// alternates two things:
+//   * walk     the walking lanes vote on the kind of unit (trav_vote_full) and the winners take one
+//              step of their walk;
+//   * service  once at most `refill` lanes still walk, every lane whose walk has ended is served
+//              together: a shadow ray's answer is added, a hit is shaded, an ended path is handed
+//              to the task and the lane's next path is begun, and the lane's next walk is set up.
+// So a lane with a short path goes on to its next one instead of waiting, and both the walk and
+// the shading run with most of the warp.  Each lane's sequence of walks, draws and float
+// operations is that of the plain loop, so the results are too, bit for bit.
+//
+// A path's shadow term is evaluated when its light sample is (Ln, the radiance if the ray gets
+// through) and the ray is traced only if it can change L (shadow_contributes).
+//
+// Task: what the paths are.  start(&ray, &smp) begins this lane's next path (false: none left),
+// finish(L) takes the radiance of the one that ended; both are called by the lanes concerned
+// together.  Smp is the task's sampler type.
+#pragma once
+#define BN_SYNC 1
+#define NI_NORM 1
+#define NI_SIN 1
+#ifndef BN_MT
+#define BN_MT 384
+#endif
+#include "dev_shading.cuh"
+
+namespace bn {
+
+// the vote of trav_vote for whole warps (every lane calls it)
+__device__ __forceinline__ bool trav_vote_full(bool walking, int mode) {
+  const unsigned b0 = __ballot_sync(0xffffffffu, !walking || (mode & 1));
+  const unsigned b1 = __ballot_sync(0xffffffffu, !walking || (mode & 2));
+  const int cn = 2 * __popc(~(b0 | b1));
+  const int ct = 2 * __popc(b0 & ~b1);
+  const int ci = 3 * __popc(b1 & ~b0);
+  const int pick = (cn >= ct && cn >= ci) ? kTravNode : (ct >= ci ? kTravTri : kTravInst);
+  return walking && mode == pick;
+}
+
+// Lanes of a warp that take paths: n paths spread over every warp of the grid when there are
+// fewer of them than lanes (short renders are bound by the latency of one path's walks, which
+// more warps with fewer lanes hide better).
+__host__ __device__ __forceinline__ int machine_lanes(long long n, long long warps) {
+  const long long l = (n + warps - 1) / warps;
+  return l < 1 ? 1 : (l > 32 ? 32 : static_cast<int>(l));
+}
+
+constexpr int kMachineStack = 16;  // stack entries per lane in shared memory
+
+enum : int { kLaneNew = 0, kLaneClosest = 1, kLaneShadow = 2, kLaneIdle = 3 };
+
+template <bool kWT, int kWalk, bool kSimple, bool kFixed7, class Task, class Smp>
+__device__ __forceinline__ void path_machine(const DevScene& s, Task& task, Smp& smp, int max_depth, int rr_depth,
+                                             int lanes, int refill) {
+  static_assert(kWalk != kWalkCount, "counting walks run the plain loop");
+  __shared__ int2 stack_block[kMachineStack * BN_MT];
+  SharedStack<kMachineStack, BN_MT> stk(stack_block);
+  TraceCounters tc{0, 0, 0};
+  Trav tr;
+  tr.mode = kTravDone;
+  tr.any = false;
+  int phase = static_cast<int>(threadIdx.x & 31) < lanes ? kLaneNew : kLaneIdle;
+  V3 L = mk(0.f, 0.f, 0.f), Ln = L, beta = L, nd = L;
+  float pdf = 0.f;
+  int depth = 0;
+  bool ends = false;
+  for (;;) {
+    const bool walking = tr.mode != kTravDone;
+    const unsigned wm = __ballot_sync(0xffffffffu, walking);
+    const unsigned im = __ballot_sync(0xffffffffu, phase == kLaneIdle);
+#ifdef BN_SYNC
+    {
+#ifdef BN_NOBAR
+      if (im == 0xffffffffu) break;
+#else
+      if (__syncthreads_and(phase == kLaneIdle)) break;
+#endif
+#else
+    if (im == 0xffffffffu) break;
+    if (__popc(wm) <= refill && (wm | im) != 0xffffffffu) {
+#endif
+      bool over = false;
+      V3 org = mk(0.f, 0.f, 0.f), dir = org;  // the next walk
+      float tmax = CUDART_INF_F;
+      if (!walking && phase == kLaneClosest) {
+        if (!tr.found) {
+          over = true;
+        } else {
+          Bounce b;
+          PathState ps;
+          ps.ray = tr.wr;
+          ps.L = L;
+          ps.beta = beta;
+          ps.pdf_bsdf = pdf;
+          ps.depth = depth;
+          bounce_shade<kFixed7, kSimple>(s, ps, tr.hit, smp, max_depth, rr_depth, &b);
+          L = ps.L;
+          beta = ps.beta;
+          pdf = ps.pdf_bsdf;
+          depth = ps.depth;
+          ends = b.ends;
+          org = b.p;
+          if (b.shadow) {
+            Ln = b.Ln;
+            nd = ps.ray.d;
+            dir = b.sh_d;
+            tmax = b.sh_t;
+            phase = kLaneShadow;
+          } else {
+            dir = ps.ray.d;
+            over = ends;
+          }
+        }
+      } else if (!walking && phase == kLaneShadow) {
+        if (!tr.found) L = Ln;
+        org = tr.wr.o;
+        dir = nd;
+        phase = kLaneClosest;
+        over = ends;
+      }
+      if (over) task.finish(L);
+      if (!walking && (over || phase == kLaneNew)) {
+        Ray ray;
+        if (task.start(&ray, &smp)) {
+          org = ray.o;
+          dir = ray.d;
+          L = mk(0.f, 0.f, 0.f);
+          beta = mk(1.f, 1.f, 1.f);
+          pdf = 0.f;
+          depth = 0;
+          phase = kLaneClosest;
+        } else {
+          phase = kLaneIdle;
+        }
+      }
+      if (!walking && phase != kLaneIdle) {
+        Ray ray;
+        ray.o = org;
+        ray.d = dir;
+        tr.any = phase == kLaneShadow;
+        trav_init<kWalk>(tr, s, ray, tmax, &tc);  // may end at once (the root box missed)
+      }
+    }
+#ifdef BN_SYNC
+#ifdef BN_SYNC2
+    __syncthreads();
+#endif
+    const int stop = refill * __popc(__ballot_sync(0xffffffffu, phase != kLaneIdle)) / 32;
+    while (__popc(__ballot_sync(0xffffffffu, tr.mode != kTravDone)) > stop)
+#endif
+    if (trav_vote_full(tr.mode != kTravDone, tr.mode)) trav_step<kAnyRuntime, kWT, kWalk, 4, true>(tr, s, stk, &tc);
+  }
+}
+
+// a grid-wide counter handed out to the lanes that call together, one atomic per group
+__device__ __forceinline__ unsigned long long claim_next(unsigned long long* counter) {
+  const unsigned act = __activemask();
+  const int lane = threadIdx.x & 31, leader = __ffs(act) - 1;
+  unsigned long long base = 0;
+  if (lane == leader) base = atomicAdd(counter, static_cast<unsigned long long>(__popc(act)));
+  base = __shfl_sync(act, base, leader);
+  return base + __popc(act & ((1u << lane) - 1u));
+}
+
+}  // namespace bn

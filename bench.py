@@ -392,8 +392,8 @@ def main():
     ap.add_argument("--no-extras", action="store_true",
                     help="skip the Cornell-box CPU ratio, PSSMLT and adjoint/forward measurements")
     ap.add_argument("--no-count", action="store_true", help="skip the instrumented visit-counting render")
-    ap.add_argument("--pool", type=int, default=0, help="wavefront path slots (0 = autotuned)")
-    ap.add_argument("--cap", type=int, default=0, help="wavefront blocks per SM cap (0 = autotuned)")
+    ap.add_argument("--pool", type=int, default=0, help="wavefront path slots (0 = default)")
+    ap.add_argument("--cap", type=int, default=0, help="wavefront blocks per SM cap (0 = none)")
     ap.add_argument("--bvh-width", type=int, default=0, choices=[0, 2, 4],
                     help="BVH walk: 0 = auto (wide records for BVHs of 1,024+ nodes), 2 = binary, 4 = wide")
     ap.add_argument("--profile-case", choices=["pssmlt", "adjoint"], default=None,
