@@ -95,6 +95,7 @@ __global__ void __launch_bounds__(256) k_mlt_regen(const WfParams* __restrict__ 
         m.cur_iter = 0;
         m.index = 0;
         m.initialized = 0;
+        m.fresh = 0;
         c0 = make_float4(0.f, 0.f, 0.f, 0.f);
         c1 = make_float4(0.f, 0.f, 0.f, __int_as_float(0));
         c2 = make_float4(__uint_as_float(cs.state), __int_as_float(-1), __int_as_float(0), __int_as_float(bid));

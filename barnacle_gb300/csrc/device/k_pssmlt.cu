@@ -57,6 +57,7 @@ __global__ void __launch_bounds__(128) k_mlt_chains(MltParams p) {
     m.cur_iter = 0;
     m.index = 0;
     m.initialized = 0;
+    m.fresh = 0;
     m.p_large = p.large_step_prob;
     m.kelemen = kKelemen;
     m.sigma = p.sigma;
