@@ -41,6 +41,7 @@ struct bn_context {
   // scene
   bool has_scene = false;
   bn::DevScene scene{};
+  // error_word: 256 bytes, the BN_DEVERR_* word at 0 and the path machine's item counter at 64
   DevBuf nodes, nodes4, tris, inst, mats, lights, light_inst, tri_pdf, tri_lights, error_word, counters;
   std::vector<int32_t> inst_order;     // TLAS order -> descriptor index
   std::vector<bn::DevMaterial> host_mats;
@@ -92,6 +93,10 @@ MegaChunks mega_chunks(long long pixels, int spp, long long max_items);
 // offsets, partial sums, film and counting are filled in by the caller).
 bn::MegaParams mega_params(const bn_context* ctx, const bn_render_desc* d, const std::vector<bn::DevView>& views,
                            const MegaChunks& ck, long long items, long long pixels);
+// A megakernel-mode render (p: its launch parameters) whose paths run in the wavefront's queues and
+// are summed in the mode's order.  *ran stays false, with nothing rendered, when the path state
+// does not fit the GPU's free memory.
+int render_ordered(bn_context* ctx, const bn_render_desc* d, const bn::MegaParams& p, bool* ran);
 int render_wavefront(bn_context* ctx, const bn_render_desc* d, const std::vector<bn::DevView>& views);
 // BVHNode.Build on the GPU (bvh_gpu.cu): the host builder's nodes and permutation
 int gpu_bvh_build(bn_context* ctx, const float* bounds, int32_t n, std::vector<bn_bvh_node>* nodes,

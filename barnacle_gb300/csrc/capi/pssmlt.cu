@@ -78,9 +78,10 @@ int render_pssmlt(bn_context* ctx, const bn_render_desc* d, const std::vector<bn
   p.eps_max = d->eps_max;
   p.watertight = d->flags & BN_RENDER_WATERTIGHT;
   p.weights = ctx->mlt_boot.as<float>();
-  p.X = ctx->mlt_state.as<float4>();  // [dimension][chain] (lockstep) or [chain][dimension] (wavefront)
+  p.X = ctx->mlt_state.as<float4>();
   p.film = ctx->film.as<float>();
   p.accepted = reinterpret_cast<unsigned long long*>(ctx->mlt_chain.ptr);
+  p.next = p.accepted + 8;
   cudaMemsetAsync(ctx->film.ptr, 0, static_cast<size_t>(pixels) * 3 * sizeof(float), st);
   cudaMemsetAsync(ctx->mlt_chain.ptr, 0, 256, st);
   cudaEventRecord(ctx->ev0, st);

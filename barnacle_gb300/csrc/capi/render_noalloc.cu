@@ -125,7 +125,6 @@ extern "C" int bn_render_noalloc(bn_context* ctx, const bn_render_desc* d, const
   p.views = scratch->views;
   p.item_offsets = scratch->item_offsets;
   p.count = false;
-  p.cull = d->flags & BN_RENDER_CULL_SHADOW;
   p.partial = scratch->partial;
   p.film = film_device;
   cudaEventRecord(ctx->ev0, ctx->stream);

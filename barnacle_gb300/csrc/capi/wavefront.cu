@@ -17,6 +17,7 @@ struct WfState {
   DevBuf params, ray, bl, hit, meta, q_active, q_bins, shadow, counters, work_next, film_acc;
   DevBuf mlt_smp, mlt_chain;  // PSSMLT chains: sampler state and chain records
   DevBuf slot_key, q_key, q_ray, sh_key, q_shadow, hist, off;
+  DevBuf path_L;              // radiance per path of a batch (ordered renders)
   // captured graph (one per launch shape)
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
@@ -38,7 +39,7 @@ struct WfState {
   void release() {
     DevBuf* b[] = {&params, &ray, &bl, &hit, &meta, &q_active, &q_bins, &shadow, &counters,
                    &work_next, &film_acc, &slot_key, &q_key, &q_ray, &sh_key, &q_shadow, &hist, &off,
-                   &mlt_smp, &mlt_chain};
+                   &mlt_smp, &mlt_chain, &path_L};
     for (DevBuf* x : b) x->release();
     if (exec) cudaGraphExecDestroy(exec);
     if (graph) cudaGraphDestroy(graph);
@@ -132,12 +133,13 @@ int build_graph(bn_context* ctx, WfState* w) {
   return BN_OK;
 }
 
-// One render into w->film_acc / ctx->film.
-int run(bn_context* ctx, WfState* w, const bn_render_desc* d, long long n_pixels, long long total_paths, int n_views,
-        int pool, int cap, bool use_graph) {
+// The bounce loop over path ids [first, end): into w->film_acc and ctx->film, or with `ordered` into
+// w->path_L.
+int run(bn_context* ctx, WfState* w, const bn_render_desc* d, long long n_pixels, long long first, long long end,
+        int n_views, int pool, int cap, bool use_graph, bool ordered) {
   cudaError_t e;
   if ((e = ensure_pool(w, pool)) != cudaSuccess) return ctx->cuda_fail(e, "wavefront path-state allocation");
-  if ((e = w->film_acc.reserve(static_cast<size_t>(n_pixels) * 3 * sizeof(double))) != cudaSuccess)
+  if (!ordered && (e = w->film_acc.reserve(static_cast<size_t>(n_pixels) * 3 * sizeof(double))) != cudaSuccess)
     return ctx->cuda_fail(e, "wavefront film allocation");
   const bool wt = d->flags & BN_RENDER_WATERTIGHT;
   const bool wide = ctx->scene.wide != 0;
@@ -170,10 +172,12 @@ int run(bn_context* ctx, WfState* w, const bn_render_desc* d, long long n_pixels
   // 193.7 / 191.6 / 187.8 M paths/s on the instanced workload, when the mode vote came in)
   p.refill_extend = 16;
   p.refill_shadow = 16;
-  p.total_paths = total_paths;
+  p.first_path = first;
+  p.total_paths = end;
   p.n_pixels = n_pixels;
-  p.max_iters = static_cast<int>(std::min<long long>(1LL << 30, (total_paths / pool + 2) * (d->max_depth + 2) + 64));
-  if (ctx->limit_iters > 0) p.max_iters = ctx->limit_iters;
+  p.max_iters = static_cast<int>(std::min<long long>(1LL << 30, ((end - first) / pool + 2) * (d->max_depth + 2) + 64));
+  // bn_set_limits' cap is the wavefront mode's
+  if (ctx->limit_iters > 0 && !ordered) p.max_iters = ctx->limit_iters;
   p.ray = w->ray.as<float4>();
   p.bl = w->bl.as<float4>();
   p.hit = w->hit.as<float4>();
@@ -205,6 +209,7 @@ int run(bn_context* ctx, WfState* w, const bn_render_desc* d, long long n_pixels
   p.trace_counters = ctx->counters.ptr;
   p.work_next = w->work_next.as<unsigned long long>();
   p.film_acc = w->film_acc.as<double>();
+  p.path_L = ordered ? w->path_L.as<float4>() : nullptr;
   p.film_out = ctx->film.as<float>();
   if (use_graph && !w->exec && !w->graph_failed) {
     if (build_graph(ctx, w) != BN_OK) {
@@ -220,7 +225,7 @@ int run(bn_context* ctx, WfState* w, const bn_render_desc* d, long long n_pixels
   cudaMemsetAsync(w->hist.ptr, 0, bn::kSortBins * sizeof(unsigned), st);
   cudaMemsetAsync(w->work_next.ptr, 0, sizeof(unsigned long long), st);
   cudaMemsetAsync(w->meta.ptr, 0, static_cast<size_t>(pool) * sizeof(int4), st);
-  cudaMemsetAsync(w->film_acc.ptr, 0, static_cast<size_t>(n_pixels) * 3 * sizeof(double), st);
+  if (!ordered) cudaMemsetAsync(w->film_acc.ptr, 0, static_cast<size_t>(n_pixels) * 3 * sizeof(double), st);
   cudaEventRecord(ctx->ev0, st);
   int launches = 0;
   if (use_graph) {
@@ -237,7 +242,7 @@ int run(bn_context* ctx, WfState* w, const bn_render_desc* d, long long n_pixels
     }
   }
   cudaEventRecord(ctx->ev1, st);
-  if ((e = bn::wf_launch_resolve(w->params.as<bn::WfParams>(), st)) != cudaSuccess)
+  if (!ordered && (e = bn::wf_launch_resolve(w->params.as<bn::WfParams>(), st)) != cudaSuccess)
     return ctx->cuda_fail(e, "wavefront resolve");
   cudaEventRecord(ctx->ev2, st);
   if ((e = cudaEventSynchronize(ctx->ev2)) != cudaSuccess) return ctx->cuda_fail(e, "wavefront render");
@@ -249,7 +254,7 @@ int run(bn_context* ctx, WfState* w, const bn_render_desc* d, long long n_pixels
   if (use_graph) launches = (5 + (sort ? 3 : 0) + (sort_shadow ? 3 : 0)) * counters[bn::kCntIter];
   ctx->stats.last_kernel_ms = ms_all;
   ctx->stats.last_dominant_ms = ms_loop;
-  ctx->stats.last_launches = launches + 1;
+  ctx->stats.last_launches = launches + (ordered ? 0 : 1);
   return BN_OK;
 }
 
@@ -367,6 +372,47 @@ int render_pssmlt_wavefront(bn_context* ctx, const bn_render_desc* d, const bn::
   return rc;
 }
 
+int render_ordered(bn_context* ctx, const bn_render_desc* d, const bn::MegaParams& p, bool* ran) {
+  // batches of whole pixels with at most 128 M paths (2 GB of radiances; half a second of work)
+  const long long per = std::min<long long>(p.n_pixels, std::max<long long>(1, (1LL << 27) / d->spp));
+  WfState* w = state(ctx);
+  const int pool = std::max(default_pool(per * d->spp), 1024);
+  cudaError_t e = w->path_L.reserve(static_cast<size_t>(per) * d->spp * sizeof(float4));
+  if (e == cudaSuccess) e = ensure_pool(w, pool);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    return BN_OK;  // *ran is false: the caller renders without path state
+  }
+  if (e != cudaSuccess) return ctx->cuda_fail(e, "wavefront path-state allocation");
+  *ran = true;
+  float loop_ms = 0.f, sum_ms = 0.f;
+  int launches = 0;
+  for (long long first = 0; first < p.n_pixels; first += per) {
+    const long long n = std::min(per, p.n_pixels - first);
+    const int rc = run(ctx, w, d, p.n_pixels, first * d->spp, (first + n) * d->spp, p.n_views, pool, 0, true, true);
+    if (rc) return rc;
+    loop_ms += ctx->stats.last_dominant_ms;
+    launches += ctx->stats.last_launches + 1;
+    cudaEventRecord(ctx->ev0, ctx->stream);
+    if ((e = bn::launch_mega_chunks(p, w->path_L.as<float4>(), first, n, ctx->stream)) != cudaSuccess)
+      return ctx->cuda_fail(e, "ordered sums");
+    if (first + n == p.n_pixels) {
+      ++launches;
+      if ((e = bn::launch_mega_reduce(p, ctx->stream)) != cudaSuccess) return ctx->cuda_fail(e, "reduce launch");
+    }
+    cudaEventRecord(ctx->ev2, ctx->stream);
+    if ((e = cudaEventSynchronize(ctx->ev2)) != cudaSuccess) return ctx->cuda_fail(e, "ordered sums");
+    float ms = 0.f;
+    cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev2);
+    sum_ms += ms;
+  }
+  ctx->stats.last_dominant_ms = loop_ms;
+  ctx->stats.last_kernel_ms = loop_ms + sum_ms;
+  ctx->stats.last_launches = launches;
+  ctx->stats.paths += static_cast<uint64_t>(p.n_paths);
+  return BN_OK;
+}
+
 int render_wavefront(bn_context* ctx, const bn_render_desc* d, const std::vector<bn::DevView>& views) {
   WfState* w = state(ctx);
   long long pixels = 0, total = 0;
@@ -387,7 +433,7 @@ int render_wavefront(bn_context* ctx, const bn_render_desc* d, const std::vector
       pool >>= 1;
     }
   }
-  const int rc = run(ctx, w, d, pixels, total, static_cast<int>(views.size()), pool, cap, use_graph);
+  const int rc = run(ctx, w, d, pixels, 0, total, static_cast<int>(views.size()), pool, cap, use_graph, false);
   if (rc) return rc;
   ctx->stats.paths += static_cast<uint64_t>(total);
   return BN_OK;

@@ -14,6 +14,16 @@
 
 namespace bn {
 
+// Functions of IEEE divisions and roots that shading calls at many places.  A kernel that holds a
+// whole path loop defines BN_COMPACT before its includes and calls them (same results): its warps
+// stand at different places in more code than the instruction cache holds, and fetch is what they
+// wait for.  Inline in kernels that do one thing at a time.
+#ifdef BN_COMPACT
+#define BN_SHADE_FN static __device__ __noinline__
+#else
+#define BN_SHADE_FN __device__ __forceinline__
+#endif
+
 // ------------------------------------------------------------------ exact vector math
 struct V3 {
   float x, y, z;
@@ -33,7 +43,7 @@ __device__ __forceinline__ V3 cross(V3 a, V3 b) {
           __fsub_rn(__fmul_rn(a.x, b.y), __fmul_rn(a.y, b.x))};
 }
 __device__ __forceinline__ float length(V3 a) { return __fsqrt_rn(dot(a, a)); }
-__device__ __forceinline__ V3 normalize(V3 a) { return divs(a, length(a)); }
+BN_SHADE_FN V3 normalize(V3 a) { return divs(a, length(a)); }
 // Vector3.FusedMultiplyAdd(a, b, c)
 __device__ __forceinline__ V3 fma3(V3 a, V3 b, V3 c) { return {fmaf(a.x, b.x, c.x), fmaf(a.y, b.y, c.y), fmaf(a.z, b.z, c.z)}; }
 __device__ __forceinline__ float comp(V3 a, int i) { return i == 0 ? a.x : (i == 1 ? a.y : a.z); }

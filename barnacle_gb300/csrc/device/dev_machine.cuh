@@ -7,7 +7,7 @@
 // alternates two things:
 //   * walk     the walking lanes vote on the kind of unit (trav_vote_full) and the winners take one
 //              step of their walk;
-//   * service  once at most `refill` lanes still walk, every lane whose walk has ended is served
+//   * service  once at most a quarter of the lanes still walk, every lane whose walk has ended is served
 //              together: a shadow ray's answer is added, a hit is shaded, an ended path is handed
 //              to the task and the lane's next path is begun, and the lane's next walk is set up.
 // So a lane with a short path goes on to its next one instead of waiting, and both the walk and
@@ -18,15 +18,9 @@
 // through) and the ray is traced only if it can change L (shadow_contributes).
 //
 // Task: what the paths are.  start(&ray, &smp) begins this lane's next path (false: none left),
-// finish(L) takes the radiance of the one that ended; both are called by the lanes concerned
+// finish(L, smp) takes the radiance of the one that ended; both are called by the lanes concerned
 // together.  Smp is the task's sampler type.
 #pragma once
-#define BN_SYNC 1
-#define NI_NORM 1
-#define NI_SIN 1
-#ifndef BN_MT
-#define BN_MT 384
-#endif
 #include "dev_shading.cuh"
 
 namespace bn {
@@ -50,16 +44,23 @@ __host__ __device__ __forceinline__ int machine_lanes(long long n, long long war
   return l < 1 ? 1 : (l > 32 ? 32 : static_cast<int>(l));
 }
 
+// Launch shape.  Blocks of 128, 4 per SM (128 registers): 64 spp of the Cornell box / 32 spp of
+// Cornell with objects / two instanced views of 4 spp took 10.0 / 45.7 / 35.8 ms, at 5 blocks 10.4 /
+// 48.4 / 35.5, at 6 blocks 11.6 / 50.1 / 36.1 (spills), at 3 up to 15 % more than at 4.  Service when 20, 16,
+// 12, 8 or 4 of the 32 lanes still walk: 12.4 10.6 10.2 10.1 9.9 / 60.2 56.1 53.2 51.1 51 / 47.6
+// 42.6 39.8 38.6 40 (before the inner walk loop): a quarter of the lanes.
+constexpr int kMachineThreads = 128, kMachineBlocks = 4;
+constexpr int kMachineRefill = 8;
 constexpr int kMachineStack = 16;  // stack entries per lane in shared memory
 
 enum : int { kLaneNew = 0, kLaneClosest = 1, kLaneShadow = 2, kLaneIdle = 3 };
 
 template <bool kWT, int kWalk, bool kSimple, bool kFixed7, class Task, class Smp>
 __device__ __forceinline__ void path_machine(const DevScene& s, Task& task, Smp& smp, int max_depth, int rr_depth,
-                                             int lanes, int refill) {
+                                             int lanes) {
   static_assert(kWalk != kWalkCount, "counting walks run the plain loop");
-  __shared__ int2 stack_block[kMachineStack * BN_MT];
-  SharedStack<kMachineStack, BN_MT> stk(stack_block);
+  __shared__ int2 stack_block[kMachineStack * kMachineThreads];
+  SharedStack<kMachineStack, kMachineThreads> stk(stack_block);
   TraceCounters tc{0, 0, 0};
   Trav tr;
   tr.mode = kTravDone;
@@ -71,23 +72,12 @@ __device__ __forceinline__ void path_machine(const DevScene& s, Task& task, Smp&
   bool ends = false;
   for (;;) {
     const bool walking = tr.mode != kTravDone;
-    const unsigned wm = __ballot_sync(0xffffffffu, walking);
-    const unsigned im = __ballot_sync(0xffffffffu, phase == kLaneIdle);
-#ifdef BN_SYNC
-    {
-#ifdef BN_NOBAR
-      if (im == 0xffffffffu) break;
-#else
-      if (__syncthreads_and(phase == kLaneIdle)) break;
-#endif
-#else
-    if (im == 0xffffffffu) break;
-    if (__popc(wm) <= refill && (wm | im) != 0xffffffffu) {
-#endif
+    // service every lane whose walk has ended
+    if (!walking && phase != kLaneIdle) {
       bool over = false;
       V3 org = mk(0.f, 0.f, 0.f), dir = org;  // the next walk
       float tmax = CUDART_INF_F;
-      if (!walking && phase == kLaneClosest) {
+      if (phase == kLaneClosest) {
         if (!tr.found) {
           over = true;
         } else {
@@ -116,15 +106,15 @@ __device__ __forceinline__ void path_machine(const DevScene& s, Task& task, Smp&
             over = ends;
           }
         }
-      } else if (!walking && phase == kLaneShadow) {
+      } else if (phase == kLaneShadow) {
         if (!tr.found) L = Ln;
         org = tr.wr.o;
         dir = nd;
         phase = kLaneClosest;
         over = ends;
       }
-      if (over) task.finish(L);
-      if (!walking && (over || phase == kLaneNew)) {
+      if (over) task.finish(L, smp);
+      if (over || phase == kLaneNew) {
         Ray ray;
         if (task.start(&ray, &smp)) {
           org = ray.o;
@@ -138,7 +128,7 @@ __device__ __forceinline__ void path_machine(const DevScene& s, Task& task, Smp&
           phase = kLaneIdle;
         }
       }
-      if (!walking && phase != kLaneIdle) {
+      if (phase != kLaneIdle) {
         Ray ray;
         ray.o = org;
         ray.d = dir;
@@ -146,14 +136,12 @@ __device__ __forceinline__ void path_machine(const DevScene& s, Task& task, Smp&
         trav_init<kWalk>(tr, s, ray, tmax, &tc);  // may end at once (the root box missed)
       }
     }
-#ifdef BN_SYNC
-#ifdef BN_SYNC2
-    __syncthreads();
-#endif
-    const int stop = refill * __popc(__ballot_sync(0xffffffffu, phase != kLaneIdle)) / 32;
+    // walk until few lanes still do
+    const unsigned busy = __ballot_sync(0xffffffffu, phase != kLaneIdle);
+    if (!busy) break;
+    const int stop = __popc(busy) * kMachineRefill / 32;
     while (__popc(__ballot_sync(0xffffffffu, tr.mode != kTravDone)) > stop)
-#endif
-    if (trav_vote_full(tr.mode != kTravDone, tr.mode)) trav_step<kAnyRuntime, kWT, kWalk, 4, true>(tr, s, stk, &tc);
+      if (trav_vote_full(tr.mode != kTravDone, tr.mode)) trav_step<kAnyRuntime, kWT, kWalk, 4, true>(tr, s, stk, &tc);
   }
 }
 

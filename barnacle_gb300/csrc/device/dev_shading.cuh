@@ -102,7 +102,7 @@ struct BsdfSample {
 };
 
 // Extensions/Material/PBR.fs:108-131
-__device__ __forceinline__ float pbr_lambda(float alpha, V3 w) {
+BN_SHADE_FN float pbr_lambda(float alpha, V3 w) {
   const float sin2 = fmaf(w.x, w.x, __fmul_rn(w.y, w.y));
   if (sin2 == 0.f) return 0.f;
   const float tan2 = __fdiv_rn(sin2, __fmul_rn(w.z, w.z));
@@ -429,30 +429,36 @@ __device__ __forceinline__ void path_begin(PathState& ps, const Ray& ray) {
   ps.depth = 0;
 }
 
-// One iteration of PathTracingIntegrator.Li's bounce loop (Extensions/Integrator/PathTracing.fs:
-// 14-81) and, with kFixed7, of PSSMLTIntegrator.Li (PSSMLT.fs:172-245), which draws 7 samples per
-// bounce in a fixed order; returns true once the path has ended (ps.L holds its radiance).
-// Draw order per bounce: u_select, u_light.xy (NEE), u_lobe, u_bsdf.xy, then u_rr if depth >=
-// rr_depth (PathTracing) / always (PSSMLT).  Reciprocal estimates are exact reciprocals here.
-// kOutline: one out-of-line walk for both queries (see trace_walk_outline).
-// kCull: evaluate the light sample first and trace its shadow ray only if it can contribute
-// (shadow_contributes); the result is the same, the plain megakernel keeps the reference's order.
-template <bool kWT, bool kFixed7, int kWalk, class Smp, bool kOutline = false, bool kSimple = false,
-          bool kCull = false>
-__device__ __forceinline__ bool li_bounce(const DevScene& s, PathState& ps, Smp& smp, int max_depth, int rr_depth,
-                                          PathCounters* pc) {
-  constexpr bool kCount = kWalk == kWalkCount;
-  if (ps.depth >= max_depth) return true;
-  Ray& ray = ps.ray;
-  HitRec h;
-  if (kCount) pc->rays++;
-  if (!trace_closest<kWT, kWalk, kOutline>(s, ray, CUDART_INF_F, &h, &pc->tc)) return true;
-  const Interaction it = make_interaction<kSimple>(s, ray, h);
+// What a bounce's shading leaves to do: the light sample's shadow ray and the radiance if it gets
+// through, whether the path ends here.  The path's next ray is in PathState.
+struct Bounce {
+  V3 p;          // the hit point: origin of the shadow ray and of the next ray
+  V3 sh_d;       // shadow ray direction and length
+  float sh_t;
+  V3 Ln;         // L with the light sample's term (the shadow ray unoccluded)
+  bool sampled;  // a light sample with a pdf
+  bool shadow;   // its shadow ray can change the radiance (shadow_contributes)
+  bool ends;     // the path ends once the shadow ray is answered
+};
+
+// The shading of one iteration of PathTracingIntegrator.Li's bounce loop (Extensions/Integrator/
+// PathTracing.fs:14-81) and, with kFixed7, of PSSMLTIntegrator.Li (PSSMLT.fs:172-245), which draws
+// 7 samples per bounce in a fixed order.  Draw order per bounce: u_select, u_light.xy (NEE),
+// u_lobe, u_bsdf.xy, then u_rr if depth >= rr_depth (PathTracing) / always (PSSMLT).  Reciprocal
+// estimates are exact reciprocals here.  No draw depends on the shadow ray, so it may be traced
+// after all of this.
+template <bool kFixed7, bool kSimple, class Smp>
+__device__ __forceinline__ void bounce_shade(const DevScene& s, PathState& ps, const HitRec& h, Smp& smp, int max_depth,
+                                             int rr_depth, Bounce* out) {
+  out->sampled = out->shadow = false;
+  out->ends = true;
+  const Interaction it = make_interaction<kSimple>(s, ps.ray, h);
+  out->p = it.p;
   const DevInstance* I = s.inst + it.inst;
   if (__ldg(&I->light) >= 0) {
     V3 le;
     float pdf_l;
-    eval_light<kSimple>(s, ray.o, it, &le, &pdf_l);
+    eval_light<kSimple>(s, ps.ray.o, it, &le, &pdf_l);
     const float mis = ps.depth == 0 ? 1.f : __fmul_rn(ps.pdf_bsdf, __frcp_rn(__fadd_rn(pdf_l, ps.pdf_bsdf)));
     ps.L = fma3(ps.beta, scale(mis, le), ps.L);
   }
@@ -464,55 +470,67 @@ __device__ __forceinline__ bool li_bounce(const DevScene& s, PathState& ps, Smp&
     u_sel = u7[0]; ulx = u7[1]; uly = u7[2];
     u_lobe = u7[3]; ubx = u7[4]; uby = u7[5]; u_rr = u7[6];
   }
-  if (mat < 0) return true;
+  if (mat < 0) return;
   if (!kFixed7) { u_sel = smp.next(); ulx = smp.next(); uly = smp.next(); }
   const DevMaterial m = s.mats[mat];
-  const V3 wo_w = neg(ray.d);
+  const V3 wo_l = to_local(it.f, neg(ps.ray.d));
   const LightSample ls = sample_light<kSimple>(s, it.p, u_sel, ulx, uly);
-  const float dist = length(sub(ls.p, it.p));
   if (ls.pdf != 0.f) {
-    Ray sh;
-    sh.o = it.p;
-    sh.d = ls.wi;
-    if (kCull) {
-      const BsdfEval be = bsdf_eval<kSimple>(m, to_local(it.f, wo_w), to_local(it.f, ls.wi));
-      const V3 a = mul(ps.beta, be.f), b = scale(__frcp_rn(__fadd_rn(be.pdf, ls.pdf)), ls.L);
-      if (shadow_contributes(a, b, ps.L)) {
-        if (kCount) pc->rays++;
-        if (!trace_any<kWT, kWalk, kOutline>(s, sh, __fsub_rn(dist, 1e-3f), &pc->tc)) ps.L = fma3(a, b, ps.L);
-      }
-    } else {
-      if (kCount) pc->rays++;
-      if (!trace_any<kWT, kWalk, kOutline>(s, sh, __fsub_rn(dist, 1e-3f), &pc->tc)) {
-        const BsdfEval be = bsdf_eval<kSimple>(m, to_local(it.f, wo_w), to_local(it.f, ls.wi));
-        ps.L = fma3(mul(ps.beta, be.f), scale(__frcp_rn(__fadd_rn(be.pdf, ls.pdf)), ls.L), ps.L);
-      }
-    }
+    const BsdfEval be = bsdf_eval<kSimple>(m, wo_l, to_local(it.f, ls.wi));
+    const V3 a = mul(ps.beta, be.f), b = scale(__frcp_rn(__fadd_rn(be.pdf, ls.pdf)), ls.L);
+    out->sampled = true;
+    out->shadow = shadow_contributes(a, b, ps.L);
+    out->Ln = fma3(a, b, ps.L);
+    out->sh_d = ls.wi;
+    out->sh_t = __fsub_rn(length(sub(ls.p, it.p)), 1e-3f);
   }
   if (!kFixed7) { u_lobe = smp.next(); ubx = smp.next(); uby = smp.next(); }
-  const BsdfSample bs = bsdf_sample<kSimple>(m, to_local(it.f, wo_w), u_lobe, ubx, uby);
-  if (bs.pdf == 0.f) return true;
+  const BsdfSample bs = bsdf_sample<kSimple>(m, wo_l, u_lobe, ubx, uby);
+  if (bs.pdf == 0.f) return;
   ps.pdf_bsdf = bs.pdf;
-  ray.o = it.p;
-  ray.d = to_world(it.f, bs.wi);
+  ps.ray.o = it.p;
+  ps.ray.d = to_world(it.f, bs.wi);
   ps.beta = scale(__frcp_rn(bs.pdf), mul(ps.beta, bs.f));
   if (ps.depth >= rr_depth) {
     const float q = fminf(1.f, fmaxf(ps.beta.x, fmaxf(ps.beta.y, ps.beta.z)));
     if (!kFixed7) u_rr = smp.next();
     if (u_rr < q) ps.beta = scale(__frcp_rn(q), ps.beta);
-    else return true;
+    else return;
   }
   ps.depth++;
-  return false;
+  out->ends = ps.depth >= max_depth;
+}
+
+// One iteration of the bounce loop with both walks in line; returns true once the path has ended
+// (ps.L holds its radiance).  A counting walk traces the shadow ray of every light sample, as the
+// reference does; the others only those that can contribute.  kOutline: one out-of-line walk for
+// both queries (see trace_walk_outline).
+template <bool kWT, bool kFixed7, int kWalk, class Smp, bool kOutline = false, bool kSimple = false>
+__device__ __forceinline__ bool li_bounce(const DevScene& s, PathState& ps, Smp& smp, int max_depth, int rr_depth,
+                                          PathCounters* pc) {
+  constexpr bool kCount = kWalk == kWalkCount;
+  if (ps.depth >= max_depth) return true;
+  HitRec h;
+  if (kCount) pc->rays++;
+  if (!trace_closest<kWT, kWalk, kOutline>(s, ps.ray, CUDART_INF_F, &h, &pc->tc)) return true;
+  Bounce b;
+  bounce_shade<kFixed7, kSimple>(s, ps, h, smp, max_depth, rr_depth, &b);
+  if (kCount ? b.sampled : b.shadow) {
+    Ray sh;
+    sh.o = b.p;
+    sh.d = b.sh_d;
+    if (kCount) pc->rays++;
+    if (!trace_any<kWT, kWalk, kOutline>(s, sh, b.sh_t, &pc->tc)) ps.L = b.Ln;
+  }
+  return b.ends;
 }
 
 // the whole path: PathTracingIntegrator.Li / PSSMLTIntegrator.Li
-template <bool kWT, bool kFixed7, int kWalk, class Smp, bool kOutline = false, bool kSimple = false,
-          bool kCull = false>
+template <bool kWT, bool kFixed7, int kWalk, class Smp, bool kOutline = false, bool kSimple = false>
 __device__ __forceinline__ V3 li_path(const DevScene& s, Ray ray, Smp& smp, int max_depth, int rr_depth, PathCounters* pc) {
   PathState ps;
   path_begin(ps, ray);
-  while (!li_bounce<kWT, kFixed7, kWalk, Smp, kOutline, kSimple, kCull>(s, ps, smp, max_depth, rr_depth, pc)) {
+  while (!li_bounce<kWT, kFixed7, kWalk, Smp, kOutline, kSimple>(s, ps, smp, max_depth, rr_depth, pc)) {
   }
   return ps.L;
 }

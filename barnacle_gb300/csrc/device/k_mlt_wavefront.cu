@@ -17,7 +17,7 @@
 //               chain is not finished.
 // A chain whose path is short starts its next mutation at once instead of waiting for the
 // longest path of its warp, and every traversal runs compacted and binned by material.  Each
-// chain draws exactly the random numbers of the lockstep kernel (k_mlt_chains) in the same order
+// chain draws exactly the random numbers of the chain kernel (k_mlt_chains) in the same order
 // and adds its path's terms to L in the same order (a bounce's emission, then its shadow term),
 // so both forms give every chain the same mutations and decisions; only the film's summation
 // order differs.  Primary samples are chain-major here: the 7 draws of a bounce read one chain's

@@ -121,6 +121,11 @@ __global__ void __launch_bounds__(256) k_wf_regen(const WfParams* __restrict__ p
 #pragma unroll
     for (int k = 0; k < kRegenRows; ++k) {
       if (valid[k] && m[k].w == kStatusDone) {
+        if (p.path_L) {  // kept path by path, summed in order afterwards (k_mega_chunks)
+          __stcs(p.path_L + m[k].x, L[k]);
+          m[k].w = kStatusFree;
+          continue;
+        }
         double* f = p.film_acc + 3LL * m[k].x;
         atomicAdd(f, static_cast<double>(__fmul_rn(L[k].x, inv_spp)));
         atomicAdd(f + 1, static_cast<double>(__fmul_rn(L[k].y, inv_spp)));
@@ -142,7 +147,7 @@ __global__ void __launch_bounds__(256) k_wf_regen(const WfParams* __restrict__ p
       first = __shfl_sync(0xffffffffu, first, 0);
 #pragma unroll
       for (int k = 0; k < kRegenRows; ++k) {
-        const long long id = static_cast<long long>(first) + __popc(wmask[k] & below);
+        const long long id = p.first_path + static_cast<long long>(first) + __popc(wmask[k] & below);
         first += __popc(wmask[k]);
         if (!((wmask[k] >> lane) & 1u) || id >= p.total_paths) continue;
         const int vi = find_view(p, id);
@@ -166,7 +171,7 @@ __global__ void __launch_bounds__(256) k_wf_regen(const WfParams* __restrict__ p
         bl[0] = make_float4(1.f, 1.f, 1.f, 0.f);
         bl[1] = make_float4(0.f, 0.f, 0.f, 0.f);
         const long long film_pix = v.pixel_offset + static_cast<long long>(v.height - y - 1) * v.width + x;
-        m[k] = make_int4(static_cast<int>(film_pix), 0, static_cast<int>(smp.state), kStatusActive);
+        m[k] = make_int4(static_cast<int>(p.path_L ? id - p.first_path : film_pix), 0, static_cast<int>(smp.state), kStatusActive);
         // PathTracing: while (depth < maxDepth) never runs; Normal and Direct ignore maxDepth
         if (p.max_depth <= 0 && p.integrator == BN_INTEGRATOR_PATH) m[k].w = kStatusDone;
       }
@@ -625,7 +630,7 @@ __global__ void __launch_bounds__(256) k_wf_sort_scatter(const WfParams* __restr
 __global__ void k_wf_control(WfParams* pp, int use_graph) {
   WfParams& p = *pp;
   int* c = p.counters;
-  const bool more_work = *p.work_next < static_cast<unsigned long long>(p.total_paths);
+  const bool more_work = *p.work_next < static_cast<unsigned long long>(p.total_paths - p.first_path);
   // PSSMLT chains: the chain regen counted the chains that are not finished into kCntDone
   bool again = p.mlt ? c[kCntDone] > 0 : (c[kCntCont] > 0 || c[kCntDone] > 0 || more_work);
   const int iter = ++c[kCntIter];
@@ -659,15 +664,6 @@ __global__ void k_wf_resolve(const WfParams* __restrict__ pp) {
   for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
        i += static_cast<long long>(gridDim.x) * blockDim.x)
     p.film_out[i] = static_cast<float>(p.film_acc[i]);
-}
-
-template <class K>
-int resident_grid(K kernel, int block) {
-  int dev = 0, sms = 0, per = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, block, 0);
-  return sms * (per > 0 ? per : 1);
 }
 
 }  // namespace

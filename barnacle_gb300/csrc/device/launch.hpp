@@ -34,6 +34,16 @@ void dispatch_walk(const DevScene& s, bool watertight, bool count, F&& f) {
   }
 }
 
+// blocks of a persistent kernel that fill the current device
+template <class K>
+int resident_grid(K kernel, int block) {
+  int dev = 0, sms = 0, per = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, block, 0);
+  return sms * (per > 0 ? per : 1);
+}
+
 // per-launch counters written by kernels that count (BN_TRACE_COUNT, stats renders)
 struct DevCounters {
   unsigned long long rays, nodes, tris, insts, paths, accepted, proposed, pad;
@@ -45,20 +55,21 @@ cudaError_t launch_bsdf(const DevScene& s, const bn_bsdf_query* q, bn_bsdf_resul
                         cudaStream_t st);
 cudaError_t launch_sampler_stream(const uint32_t* seeds, long long n_streams, int n_draws, float* out, cudaStream_t st);
 
-// Plain megakernel: one thread per (view, pixel, sample chunk); partial sums per chunk, then a
+// Megakernel: work items of one (view, pixel, sample chunk); partial sums per chunk, then a
 // reduction in chunk order into the FP32 film (rows flipped as Film.SetPixel does).
 struct MegaParams {
   const DevView* views;
   int n_views;
   long long n_items;         // sum over views of pixels * chunks
   const long long* item_offsets;  // per view: first item (device)
+  long long n_paths;         // pixels * spp
   int spp, chunks, spc;      // samples per pixel, chunks per pixel, samples per chunk
   int max_depth, rr_depth, frame_id;
   int integrator;            // bn_integrator_type: PATH, NORMAL or DIRECT
   bool simple;               // Lambertian meshes, uniform light sampler, pinhole views only
   bool watertight;
   bool count;
-  bool cull;                 // trace a light sample's shadow ray only if it can change L
+  unsigned long long* next;  // the next item a lane of the path machine claims (scratch)
   float4* partial;           // n_items partial sums (scratch)
   float* film;               // concatenated views, 3 floats per pixel
   long long n_pixels;
@@ -66,7 +77,8 @@ struct MegaParams {
 };
 cudaError_t launch_megakernel(const DevScene& s, const MegaParams& p, cudaStream_t st);
 cudaError_t launch_megakernel_simple(const DevScene& s, const MegaParams& p, cudaStream_t st);  // NORMAL, DIRECT
-cudaError_t launch_megakernel_cull(const DevScene& s, const MegaParams& p, cudaStream_t st);    // PATH + cull
+// chunk sums of path radiances (n pixels from `first` on, spp float4 each) that the wavefront left
+cudaError_t launch_mega_chunks(const MegaParams& p, const float4* path_L, long long first, long long n, cudaStream_t st);
 cudaError_t launch_mega_reduce(const MegaParams& p, cudaStream_t st);
 
 // Film.PostProcess + Rgba32 packing over n_pixels RGB floats into 4-byte RGBA

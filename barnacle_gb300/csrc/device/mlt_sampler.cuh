@@ -1,4 +1,4 @@
-// The PSSMLT sampler and splats shared by the lockstep chain kernel (k_pssmlt.cu) and the
+// The PSSMLT sampler and splats shared by the chain kernel (k_pssmlt.cu) and the
 // wavefront chains (k_mlt_wavefront.cu): MLTSampler (Extensions/Integrator/PSSMLT.fs:36-150) over
 // primary samples at X[dim * stride] (float4: value, backup, last modification, its backup),
 // the luminance and camera draws of PSSMLTIntegrator, and warp-aggregated film splats.
@@ -37,7 +37,7 @@ __device__ __forceinline__ float erfinv_giles(float x) {
   return __fmul_rn(fmaf(p, w, 2.83297682f), x);
 }
 
-// MLTSampler (PSSMLT.fs:36-150); primary samples at X[dim * stride + chain]
+// MLTSampler (PSSMLT.fs:36-150); primary samples at X[dim * stride]
 struct MltSampler {
   uint32_t inner;
   bool large_step;
@@ -75,6 +75,7 @@ struct MltSampler {
     } else if (kelemen) {
       v = x.x;
       const float a = log_eps;
+#pragma unroll 1
       for (int k = last_mod; k < cur_iter; ++k) {
         const float u1 = __fsub_rn(lcg_next(inner), 0.5f);
         const float u2 = u1 < 0.f ? __fadd_rn(1.f, __fmul_rn(2.f, u1)) : __fmul_rn(2.f, u1);
@@ -110,25 +111,26 @@ struct MltSampler {
     else x = record(min(i, max_dims - 1), fresh);
     return draw(i, x);
   }
-  // the next N draws (Next1D N times), their primary samples loaded together first: one memory
-  // round trip instead of N dependent ones, the same values in the same order
+  // the next N draws (Next1D N times), the same values in the same order
   template <int N>
   __device__ __forceinline__ void next_n(float* u) {
     const int i0 = index, init0 = initialized, fresh0 = fresh;
     if (i0 + N > max_dims) {  // past the vector's end: one at a time, as Next1D
-#pragma unroll
+#pragma unroll 1
       for (int k = 0; k < N; ++k) u[k] = next();
       return;
     }
-    float4 x[N];
-#pragma unroll
-    for (int k = 0; k < N; ++k)
-      x[k] = i0 + k < init0 ? record(i0 + k, fresh0) : make_float4(0.f, 0.f, __int_as_float(0), __int_as_float(0));
-#pragma unroll
+    // one copy of the draw's code, run N times: unrolled, the draws were half of a chain kernel's
+    // code.  The records' lines are asked for first, so the loop does not wait for them one by one.
+    const float4* x = X + static_cast<long long>(i0) * stride;
+    asm volatile("prefetch.global.L1 [%0];" ::"l"(x));
+    asm volatile("prefetch.global.L1 [%0];" ::"l"(x + (N - 1) * stride));
+#pragma unroll 1
     for (int k = 0; k < N; ++k) {
       const int i = index++;
+      const float4 r = i < init0 ? record(i, fresh0) : make_float4(0.f, 0.f, __int_as_float(0), __int_as_float(0));
       if (initialized <= i) initialized = i + 1;
-      u[k] = draw(i, x[k]);
+      u[k] = draw(i, r);
     }
   }
   // Reject restores every initialised dimension (value and last modification from their backups).

@@ -21,7 +21,8 @@ struct MltParams {
   float* weights;               // n_bootstrap luminances
   const float* alias_prob;      // proportional start table, or null: uniform as the reference
   const int* alias_idx;
-  float4* X;                    // n_dims x n_chains primary samples
+  unsigned long long* next;     // the next bootstrap path or chain a lane claims (scratch)
+  float4* X;                    // n_dims primary samples per chain, chain-major
   float* film;                  // W * H * 3
   unsigned long long* accepted;
 };

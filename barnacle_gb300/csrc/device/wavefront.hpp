@@ -66,6 +66,7 @@ struct WfParams {
   int max_iters;                // watchdog
   int refill_extend;            // extend lanes refill when at most this many of a warp still walk
   int refill_shadow;            // the same for the shadow kernel
+  long long first_path;         // path ids [first_path, total_paths)
   long long total_paths;
   long long n_pixels;
   // per slot
@@ -74,7 +75,7 @@ struct WfParams {
   float4* bl;                   // 2 per slot: (beta, -), (L, -)
   float4* hit;                  // 2 per slot: (t, u, v, instance | -1 as int bits),
                                 //             (triangle or sphere root as int bits, -, -, -)
-  int4* meta;                   // (film pixel, depth, sampler state, status)
+  int4* meta;                   // (film pixel, or path - first_path with path_L; depth, sampler state, status)
   // queues
   int* q_active;                // pool entries
   int* q_bins;                  // kNumBins x pool entries
@@ -94,6 +95,7 @@ struct WfParams {
   void* trace_counters;         // DevCounters (rays, nodes, triangles, instances) of counting walks
   unsigned long long* work_next;
   double* film_acc;             // 3 doubles per pixel
+  float4* path_L;               // or, if not null, the radiance of path first_path + i at i
   float* film_out;              // 3 floats per pixel
   cudaGraphConditionalHandle cond;
   int mlt;                      // 1: the slots hold PSSMLT chains (mlt_p), 0: camera paths

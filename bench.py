@@ -13,10 +13,10 @@ render per step, depth 8).
 value  = paths / device time (CUDA events on the library's stream around its kernels).
 e2e    = the same metric through bn_render with a host output buffer: the views' descriptors
          go host->device and the FP32 film comes back device->host inside the timed region.
-compare: the plain megakernel in the reference's order (trace every shadow ray, then evaluate),
-         the megakernel that traces only shadow rays that can change the radiance (the test the
-         wavefront applies), and the wavefront with the watertight triangle test; each timed the
-         same way on the same step (fewer steps: --compare-steps).
+compare: megakernel mode (whose long renders run their paths through the wavefront's queues and sum
+         them in order), the same as one kernel (megakernel_cull), and the wavefront with the
+         watertight triangle test; each timed the same way on the same step (fewer steps:
+         --compare-steps).
 roofline: the dominant kernel's algorithmic bytes (32 per BVH node tested, 48 per triangle
          tested, 152 per instance visited, counted by an instrumented run of the same step) over
          its event-timed duration, against the measured HBM copy bandwidth; traffic = DRAM bytes
@@ -200,7 +200,7 @@ def run_extras(ctx, args, torch, flush):
     from oracle import pyoracle
 
     out = {}
-    # Cornell box: plain megakernel vs the CPU restatement (same workload, bounded CPU sample)
+    # Cornell box: megakernel mode vs the CPU restatement (same workload, bounded CPU sample)
     c0 = Bundle.generate("cornell", 1)
     c0.scene.contents.bvh_width = args.bvh_width
     ctx.upload(c0)

@@ -175,8 +175,11 @@ enum bn_integrator_type {
                             /* and one BSDF sample that scores a light it hits                     */
 };
 enum bn_render_mode {
-  BN_MODE_MEGAKERNEL = 0, /* one thread per pixel-sample path (PSSMLT: per chain, in   */
-                          /* lockstep), the plain form                               */
+  BN_MODE_MEGAKERNEL = 0, /* each pixel's samples summed in order (the film is the     */
+                          /* same on every run); one kernel of lanes that run whole   */
+                          /* paths, from 1 M paths on the wavefront's queues (2 GB    */
+                          /* and 224 B per slot of device memory at most; without it, */
+                          /* the one kernel).  PSSMLT: a lane per chain               */
   BN_MODE_WAVEFRONT = 1   /* persistent queues compacted every bounce, many views per */
                           /* launch (PSSMLT: one path slot per chain, same decisions) */
 };
@@ -189,10 +192,10 @@ enum bn_mutation_type { BN_MUTATION_GAUSSIAN = 0, BN_MUTATION_KELEMEN = 1 };
                                     /* (PSSMLT chains always run host-driven iterations)       */
 #define BN_RENDER_COUNT 0x8u        /* count rays / BVH nodes / triangles / instances visited  */
                                     /* into bn_stats (a slower instrumented kernel variant)     */
-#define BN_RENDER_CULL_SHADOW 0x10u /* megakernel: evaluate a light sample first and trace its   */
-                                    /* shadow ray only if it can change the radiance (the same  */
-                                    /* image; the wavefront always does this, the plain form    */
-                                    /* keeps the reference's trace-then-evaluate order)          */
+#define BN_RENDER_CULL_SHADOW 0x10u /* megakernel mode: one kernel whatever the render's length (the */
+                                    /* same image).  Every form evaluates a light sample first and */
+                                    /* traces its shadow ray only if it can change the radiance;   */
+                                    /* a counting render traces all of them, as the reference does */
 
 typedef struct bn_view {
   bn_camera_desc camera;
