@@ -184,7 +184,7 @@ int bn_destroy(bn_context* ctx) {
                     &ctx->tri_pdf, &ctx->tri_lights, &ctx->error_word, &ctx->counters, &ctx->q_in, &ctx->q_out,
                     &ctx->views, &ctx->item_offsets, &ctx->partial, &ctx->film, &ctx->wf_state, &ctx->mlt_state,
                     &ctx->mlt_boot, &ctx->mlt_chain, &ctx->adj_params, &ctx->adj_image, &ctx->adj_target,
-                    &ctx->adj_grad, &ctx->adj_aux};
+                    &ctx->adj_grad, &ctx->adj_aux, &ctx->adj_scene, &ctx->adj_rec};
   for (DevBuf* b : bufs) b->release();
   if (ctx->wf && ctx->wf_release) ctx->wf_release(ctx->wf);
   cudaEventDestroy(ctx->ev0);

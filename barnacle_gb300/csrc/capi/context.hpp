@@ -62,7 +62,7 @@ struct bn_context {
   bn_stats stats{};
 
   // pssmlt / adjoint scratch
-  DevBuf mlt_state, mlt_boot, mlt_chain, adj_params, adj_image, adj_target, adj_grad, adj_aux;
+  DevBuf mlt_state, mlt_boot, mlt_chain, adj_params, adj_image, adj_target, adj_grad, adj_aux, adj_scene, adj_rec;
 
   // wavefront path state, captured graph and launch shape (owned by wavefront.cu)
   void* wf = nullptr;
@@ -97,6 +97,16 @@ bn::MegaParams mega_params(const bn_context* ctx, const bn_render_desc* d, const
 // are summed in the mode's order.  *ran stays false, with nothing rendered, when the path state
 // does not fit the GPU's free memory.
 int render_ordered(bn_context* ctx, const bn_render_desc* d, const bn::MegaParams& p, bool* ran);
+// Where an ordered run of the wavefront leaves its paths (WfParams::path_L, rec, lit).
+struct PathRecords {
+  float4* L;
+  float4* rec;
+  unsigned char* lit;
+};
+// The n_paths camera paths of the one view in ctx->views through the wavefront's queues.  *ran stays
+// false when the path state does not fit the GPU's free memory.
+int wavefront_paths(bn_context* ctx, const bn::DevScene& scene, const bn_render_desc* d, long long n_paths,
+                    const PathRecords& out, bool* ran);
 int render_wavefront(bn_context* ctx, const bn_render_desc* d, const std::vector<bn::DevView>& views);
 // BVHNode.Build on the GPU (bvh_gpu.cu): the host builder's nodes and permutation
 int gpu_bvh_build(bn_context* ctx, const float* bounds, int32_t n, std::vector<bn_bvh_node>* nodes,

@@ -134,15 +134,15 @@ int build_graph(bn_context* ctx, WfState* w) {
 }
 
 // The bounce loop over path ids [first, end): into w->film_acc and ctx->film, or with `ordered` into
-// w->path_L.
-int run(bn_context* ctx, WfState* w, const bn_render_desc* d, long long n_pixels, long long first, long long end,
-        int n_views, int pool, int cap, bool use_graph, bool ordered) {
+// its buffers.
+int run(bn_context* ctx, WfState* w, const bn::DevScene& scene, const bn_render_desc* d, long long n_pixels,
+        long long first, long long end, int n_views, int pool, int cap, bool use_graph, const bnc::PathRecords* ordered) {
   cudaError_t e;
   if ((e = ensure_pool(w, pool)) != cudaSuccess) return ctx->cuda_fail(e, "wavefront path-state allocation");
   if (!ordered && (e = w->film_acc.reserve(static_cast<size_t>(n_pixels) * 3 * sizeof(double))) != cudaSuccess)
     return ctx->cuda_fail(e, "wavefront film allocation");
   const bool wt = d->flags & BN_RENDER_WATERTIGHT;
-  const bool wide = ctx->scene.wide != 0;
+  const bool wide = scene.wide != 0;
   // both queues sorted by ray key: on the 1,024-instance workload 111.5 M paths/s against 110.0
   // (ray queue only) and 107.9 (neither)
   const bool sort = true, sort_shadow = true;
@@ -159,7 +159,7 @@ int run(bn_context* ctx, WfState* w, const bn_render_desc* d, long long n_pixels
     }
   }
   bn::WfParams p{};
-  p.scene = ctx->scene;
+  p.scene = scene;
   p.views = ctx->views.as<bn::DevView>();
   p.n_views = n_views;
   p.spp = d->spp;
@@ -209,7 +209,11 @@ int run(bn_context* ctx, WfState* w, const bn_render_desc* d, long long n_pixels
   p.trace_counters = ctx->counters.ptr;
   p.work_next = w->work_next.as<unsigned long long>();
   p.film_acc = w->film_acc.as<double>();
-  p.path_L = ordered ? w->path_L.as<float4>() : nullptr;
+  if (ordered) {
+    p.path_L = ordered->L;
+    p.rec = ordered->rec;
+    p.lit = ordered->lit;
+  }
   p.film_out = ctx->film.as<float>();
   if (use_graph && !w->exec && !w->graph_failed) {
     if (build_graph(ctx, w) != BN_OK) {
@@ -389,7 +393,9 @@ int render_ordered(bn_context* ctx, const bn_render_desc* d, const bn::MegaParam
   int launches = 0;
   for (long long first = 0; first < p.n_pixels; first += per) {
     const long long n = std::min(per, p.n_pixels - first);
-    const int rc = run(ctx, w, d, p.n_pixels, first * d->spp, (first + n) * d->spp, p.n_views, pool, 0, true, true);
+    const PathRecords out{w->path_L.as<float4>(), nullptr, nullptr};
+    const int rc = run(ctx, w, ctx->scene, d, p.n_pixels, first * d->spp, (first + n) * d->spp, p.n_views, pool, 0, true,
+                       &out);
     if (rc) return rc;
     loop_ms += ctx->stats.last_dominant_ms;
     launches += ctx->stats.last_launches + 1;
@@ -413,6 +419,20 @@ int render_ordered(bn_context* ctx, const bn_render_desc* d, const bn::MegaParam
   return BN_OK;
 }
 
+int wavefront_paths(bn_context* ctx, const bn::DevScene& scene, const bn_render_desc* d, long long n_paths,
+                    const PathRecords& out, bool* ran) {
+  WfState* w = state(ctx);
+  const int pool = std::max(default_pool(n_paths), 1024);
+  const cudaError_t e = ensure_pool(w, pool);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    return BN_OK;
+  }
+  if (e != cudaSuccess) return ctx->cuda_fail(e, "wavefront path-state allocation");
+  *ran = true;
+  return run(ctx, w, scene, d, n_paths / d->spp, 0, n_paths, 1, pool, 0, true, &out);
+}
+
 int render_wavefront(bn_context* ctx, const bn_render_desc* d, const std::vector<bn::DevView>& views) {
   WfState* w = state(ctx);
   long long pixels = 0, total = 0;
@@ -433,7 +453,7 @@ int render_wavefront(bn_context* ctx, const bn_render_desc* d, const std::vector
       pool >>= 1;
     }
   }
-  const int rc = run(ctx, w, d, pixels, 0, total, static_cast<int>(views.size()), pool, cap, use_graph, false);
+  const int rc = run(ctx, w, ctx->scene, d, pixels, 0, total, static_cast<int>(views.size()), pool, cap, use_graph, nullptr);
   if (rc) return rc;
   ctx->stats.paths += static_cast<uint64_t>(total);
   return BN_OK;

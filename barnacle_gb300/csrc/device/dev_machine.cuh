@@ -19,7 +19,11 @@
 //
 // Task: what the paths are.  start(&ray, &smp) begins this lane's next path (false: none left),
 // finish(L, smp) takes the radiance of the one that ended; both are called by the lanes concerned
-// together.  Smp is the task's sampler type.
+// together.  hit(depth, found, h) and lit() hear of every closest hit and, for the vertex in
+// task.vertex, of a shadow ray that got through (kRecord).  Smp is the task's sampler type.
+//
+// kRecord: the paths are to be replayed from those records (k_adjoint.cu), so a shadow ray is also
+// traced when only the derivative of its term can be other than zero (Bounce::lit).
 #pragma once
 #include "dev_shading.cuh"
 
@@ -55,7 +59,7 @@ constexpr int kMachineStack = 16;  // stack entries per lane in shared memory
 
 enum : int { kLaneNew = 0, kLaneClosest = 1, kLaneShadow = 2, kLaneIdle = 3 };
 
-template <bool kWT, int kWalk, bool kSimple, bool kFixed7, class Task, class Smp>
+template <bool kWT, int kWalk, bool kSimple, bool kFixed7, bool kRecord = false, class Task, class Smp>
 __device__ __forceinline__ void path_machine(const DevScene& s, Task& task, Smp& smp, int max_depth, int rr_depth,
                                              int lanes) {
   static_assert(kWalk != kWalkCount, "counting walks run the plain loop");
@@ -78,6 +82,7 @@ __device__ __forceinline__ void path_machine(const DevScene& s, Task& task, Smp&
       V3 org = mk(0.f, 0.f, 0.f), dir = org;  // the next walk
       float tmax = CUDART_INF_F;
       if (phase == kLaneClosest) {
+        if constexpr (kRecord) task.hit(depth, tr.found, tr.hit);
         if (!tr.found) {
           over = true;
         } else {
@@ -88,6 +93,7 @@ __device__ __forceinline__ void path_machine(const DevScene& s, Task& task, Smp&
           ps.beta = beta;
           ps.pdf_bsdf = pdf;
           ps.depth = depth;
+          const int vertex = depth;
           bounce_shade<kFixed7, kSimple>(s, ps, tr.hit, smp, max_depth, rr_depth, &b);
           L = ps.L;
           beta = ps.beta;
@@ -95,7 +101,8 @@ __device__ __forceinline__ void path_machine(const DevScene& s, Task& task, Smp&
           depth = ps.depth;
           ends = b.ends;
           org = b.p;
-          if (b.shadow) {
+          if (b.shadow || (kRecord && b.lit)) {
+            if constexpr (kRecord) task.vertex = vertex;
             Ln = b.Ln;
             nd = ps.ray.d;
             dir = b.sh_d;
@@ -107,7 +114,10 @@ __device__ __forceinline__ void path_machine(const DevScene& s, Task& task, Smp&
           }
         }
       } else if (phase == kLaneShadow) {
-        if (!tr.found) L = Ln;
+        if (!tr.found) {
+          L = Ln;
+          if constexpr (kRecord) task.lit();
+        }
         org = tr.wr.o;
         dir = nd;
         phase = kLaneClosest;

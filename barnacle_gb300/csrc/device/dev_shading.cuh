@@ -438,6 +438,7 @@ struct Bounce {
   V3 Ln;         // L with the light sample's term (the shadow ray unoccluded)
   bool sampled;  // a light sample with a pdf
   bool shadow;   // its shadow ray can change the radiance (shadow_contributes)
+  bool lit;      // light would arrive through it, whatever the BSDF's value
   bool ends;     // the path ends once the shadow ray is answered
 };
 
@@ -450,7 +451,7 @@ struct Bounce {
 template <bool kFixed7, bool kSimple, class Smp>
 __device__ __forceinline__ void bounce_shade(const DevScene& s, PathState& ps, const HitRec& h, Smp& smp, int max_depth,
                                              int rr_depth, Bounce* out) {
-  out->sampled = out->shadow = false;
+  out->sampled = out->shadow = out->lit = false;
   out->ends = true;
   const Interaction it = make_interaction<kSimple>(s, ps.ray, h);
   out->p = it.p;
@@ -480,6 +481,7 @@ __device__ __forceinline__ void bounce_shade(const DevScene& s, PathState& ps, c
     const V3 a = mul(ps.beta, be.f), b = scale(__frcp_rn(__fadd_rn(be.pdf, ls.pdf)), ls.L);
     out->sampled = true;
     out->shadow = shadow_contributes(a, b, ps.L);
+    out->lit = b.x != 0.f || b.y != 0.f || b.z != 0.f;
     out->Ln = fma3(a, b, ps.L);
     out->sh_d = ls.wi;
     out->sh_t = __fsub_rn(length(sub(ls.p, it.p)), 1e-3f);

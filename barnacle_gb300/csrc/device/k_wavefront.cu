@@ -392,7 +392,9 @@ __global__ void __launch_bounds__(128) k_wf_shade(const WfParams* __restrict__ p
       int4 m = p.meta[slot];
       const float4 hf = p.hit[2 * slot];
       const int hinst = __float_as_int(hf.w);
+      const long long vertex = static_cast<long long>(m.y) * (p.total_paths - p.first_path) + m.x;
       if (hinst < 0) {
+        if (p.rec) p.rec[vertex] = make_float4(0.f, __int_as_float(-1), 0.f, 0.f);
         done = true;
       } else {
         const float4 o = p.ray[2 * slot], d = p.ray[2 * slot + 1];
@@ -401,6 +403,7 @@ __global__ void __launch_bounds__(128) k_wf_shade(const WfParams* __restrict__ p
         ray.d = mk(d.x, d.y, d.z);
         const float pdf_bsdf = d.w;
         const int hprim = __float_as_int(p.hit[2 * slot + 1].x);
+        if (p.rec) p.rec[vertex] = make_float4(hf.x, hf.w, __int_as_float(hprim), 0.f);
         HitRec h;
         h.t = hf.x; h.u = hf.y; h.v = hf.z;
         h.inst = hinst;
@@ -444,9 +447,9 @@ __global__ void __launch_bounds__(128) k_wf_shade(const WfParams* __restrict__ p
             const V3 bb = scale(__frcp_rn(__fadd_rn(be.pdf, ls.pdf)), ls.L);
             sh_o = make_float4(it.p.x, it.p.y, it.p.z, __fsub_rn(dist, 1e-3f));
             sh_d = make_float4(ls.wi.x, ls.wi.y, ls.wi.z, __int_as_float(slot));
-            sh_a = make_float4(a.x, a.y, a.z, 0.f);
-            sh_b = make_float4(bb.x, bb.y, bb.z, 0.f);
-            shadow = shadow_contributes(a, bb, L);
+            sh_a = make_float4(a.x, a.y, a.z, __int_as_float(static_cast<int>(vertex)));
+            sh_b = make_float4(bb.x, bb.y, bb.z, __int_as_float(static_cast<int>(vertex >> 32)));
+            shadow = shadow_contributes(a, bb, L) || (p.rec && (bb.x != 0.f || bb.y != 0.f || bb.z != 0.f));
           }
           const float u_lobe = smp.next(), ubx = smp.next(), uby = smp.next();
           const BsdfSample bs = bsdf_sample(mt, to_local(it.f, wo_w), u_lobe, ubx, uby);
@@ -528,6 +531,8 @@ __global__ void __launch_bounds__(128, kShadowBlocks) k_wf_shadow(const WfParams
           L.y = fmaf(a.y, b.y, L.y);
           L.z = fmaf(a.z, b.z, L.z);
           p.bl[2 * slot + 1] = L;
+          if (p.lit)
+            p.lit[static_cast<long long>(__float_as_uint(a.w)) | (static_cast<long long>(__float_as_int(b.w)) << 32)] = 1;
         }
       }
       const int qi = fetch_next(&p.counters[kCntFetchShadow], !have);

@@ -96,6 +96,12 @@ struct WfParams {
   unsigned long long* work_next;
   double* film_acc;             // 3 doubles per pixel
   float4* path_L;               // or, if not null, the radiance of path first_path + i at i
+  // records of an ordered render's vertices, or null: (t, instance | -1, triangle or sphere root, -)
+  // of path first_path + i's hit at depth k at k * n + i, n = total_paths - first_path, and 1 in lit
+  // where the vertex's shadow ray got through.  With them a shadow ray is also traced when only
+  // the derivative of its term can be other than zero.
+  float4* rec;
+  unsigned char* lit;
   float* film_out;              // 3 floats per pixel
   cudaGraphConditionalHandle cond;
   int mlt;                      // 1: the slots hold PSSMLT chains (mlt_p), 0: camera paths
