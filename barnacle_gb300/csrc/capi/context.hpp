@@ -32,6 +32,16 @@ struct DevBuf {
   T* as() const { return static_cast<T*>(ptr); }
 };
 
+namespace bnc {
+// the GPU BVH builder's buffers (bvh_gpu.cu)
+struct BvhWork {
+  DevBuf bounds, items, ranges, level, nodes, out, perm, odd, counters;
+  void* host_counters = nullptr;  // pinned
+  void trim();                    // frees what is too large to keep
+  void release();
+};
+}  // namespace bnc
+
 struct bn_context {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -60,6 +70,8 @@ struct bn_context {
   DevBuf views, item_offsets, partial, film, wf_state, rgba;
   long long film_floats = 0;
   bn_stats stats{};
+
+  bnc::BvhWork bvh;
 
   // pssmlt / adjoint scratch
   DevBuf mlt_state, mlt_boot, mlt_chain, adj_params, adj_image, adj_target, adj_grad, adj_aux, adj_scene, adj_rec;
@@ -110,7 +122,10 @@ int wavefront_paths(bn_context* ctx, const bn::DevScene& scene, const bn_render_
 int render_wavefront(bn_context* ctx, const bn_render_desc* d, const std::vector<bn::DevView>& views);
 // BVHNode.Build on the GPU (bvh_gpu.cu): the host builder's nodes and permutation
 int gpu_bvh_build(bn_context* ctx, const float* bounds, int32_t n, std::vector<bn_bvh_node>* nodes,
-                  std::vector<int32_t>* perm, int small);
+                  std::vector<int32_t>* perm);
+// the same from n > 0 boxes in device memory, left there: ctx->bvh.out, perm, and with `odd` the
+// parity of each node's depth in ctx->bvh.odd.  *nan: not built, a box is for the host builder.
+int gpu_bvh_build_resident(bn_context* ctx, const float* bounds_device, int32_t n, bool odd, bool* nan, int* n_nodes);
 int render_pssmlt(bn_context* ctx, const bn_render_desc* d, const std::vector<bn::DevView>& views);
 // the PSSMLT chains in the wavefront (wavefront.cu), after the bootstrap
 int render_pssmlt_wavefront(bn_context* ctx, const bn_render_desc* d, const bn::MltParams& mp, int* launches);

@@ -244,7 +244,7 @@ extern "C" int bn_scene_upload(bn_context* ctx, const bn_scene_desc* d) {
       b[0] = lo.x; b[1] = lo.y; b[2] = lo.z; b[3] = hi.x; b[4] = hi.y; b[5] = hi.z;
     }
     if (on_device(m.n_triangles)) {
-      const int rc = bnc::gpu_bvh_build(ctx, boxes.data(), m.n_triangles, &mp[i].nodes, &mp[i].perm, 256);
+      const int rc = bnc::gpu_bvh_build(ctx, boxes.data(), m.n_triangles, &mp[i].nodes, &mp[i].perm);
       if (rc) return rc;
     } else if (!bnh::bvh_build(boxes.data(), m.n_triangles, &mp[i].nodes, &mp[i].perm)) {
       return ctx->fail(BN_ERR_UNSUPPORTED, "mesh " + std::to_string(i) + ": BVH leaf larger than 127 triangles");
@@ -304,7 +304,7 @@ extern "C" int bn_scene_upload(bn_context* ctx, const bn_scene_desc* d) {
   std::vector<bn_bvh_node> tlas;
   std::vector<int32_t> order;
   if (on_device(ni)) {
-    const int rc = bnc::gpu_bvh_build(ctx, ibox.data(), ni, &tlas, &order, 256);
+    const int rc = bnc::gpu_bvh_build(ctx, ibox.data(), ni, &tlas, &order);
     if (rc) return rc;
   } else if (!bnh::bvh_build(ibox.data(), ni, &tlas, &order)) {
     return ctx->fail(BN_ERR_UNSUPPORTED, "TLAS leaf larger than 127 instances");
