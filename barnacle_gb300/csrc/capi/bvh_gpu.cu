@@ -5,7 +5,7 @@
 // coordinate or centroid, where the fold's order decides the bounds, are built by the host builder.
 //
 // The buffers (about 230 bytes per box) belong to the context and are kept from build to build up
-// to 256 MB; larger ones are freed when the call that needed them returns.
+// to 256 MB; larger ones are freed when the C call that needed them returns.
 #include <algorithm>
 #include <string>
 #include <vector>
@@ -17,14 +17,16 @@
 namespace bnc {
 
 void BvhWork::release() {
-  for (DevBuf* b : {&bounds, &items, &ranges, &level, &nodes, &out, &perm, &odd, &counters}) b->release();
+  for (DevBuf* b : {&bounds, &items, &ranges, &level, &nodes, &out, &perm, &odd, &counters, &vertices, &indices, &slots,
+                    &scene_odd, &wide}) b->release();
   if (host_counters) cudaFreeHost(host_counters);
   host_counters = nullptr;
 }
 
 void BvhWork::trim() {
   size_t total = 0;
-  DevBuf* all[] = {&bounds, &items, &ranges, &level, &nodes, &out, &perm, &odd};
+  DevBuf* all[] = {&bounds, &items, &ranges, &level, &nodes, &out, &perm, &odd, &vertices, &indices, &slots, &scene_odd,
+                   &wide};
   for (DevBuf* b : all) total += b->bytes;
   if (total > (256u << 20))
     for (DevBuf* b : all) b->release();
@@ -121,7 +123,6 @@ int gpu_bvh_build(bn_context* ctx, const float* bounds, int32_t n, std::vector<b
   cudaMemcpyAsync(nodes->data(), ctx->bvh.out.ptr, nodes->size() * sizeof(bn_bvh_node), cudaMemcpyDeviceToHost, ctx->stream);
   cudaMemcpyAsync(perm->data(), ctx->bvh.perm.ptr, perm->size() * sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream);
   const cudaError_t e = cudaStreamSynchronize(ctx->stream);
-  ctx->bvh.trim();
   return e == cudaSuccess ? BN_OK : ctx->cuda_fail(e, "BVH download");
 }
 

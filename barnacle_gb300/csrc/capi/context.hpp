@@ -36,6 +36,7 @@ namespace bnc {
 // the GPU BVH builder's buffers (bvh_gpu.cu)
 struct BvhWork {
   DevBuf bounds, items, ranges, level, nodes, out, perm, odd, counters;
+  DevBuf vertices, indices, slots, scene_odd, wide;  // bn_scene_upload's meshes
   void* host_counters = nullptr;  // pinned
   void trim();                    // frees what is too large to keep
   void release();

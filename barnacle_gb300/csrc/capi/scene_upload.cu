@@ -2,7 +2,9 @@
 //
 //  1. BLAS per mesh over the triangle AABBs (MeshPrimitive.BVHNodes, Mesh.fs:159-169), which
 //     permutes the mesh's triangles in place; triangles are stored in that order.  Built on the
-//     GPU (bvh_gpu.cu) or the host (bvh_build.cpp), which give the same trees.
+//     GPU (bvh_gpu.cu) or the host (bvh_build.cpp), which give the same trees.  A mesh built on the
+//     GPU stays there: its boxes, permuted triangles, pdfs and wide records are made from its
+//     vertices and indices by kernels (k_scene.cu).
 //  2. the reference AliasTable of each mesh over triangle areas in permuted order
 //     (Mesh.fs:181-186, Util/AliasTable.fs:14-27): entry pdf = area / (sequential float sum).
 //  3. instance world bounds = AxisAlignedBoundingBox.Transform(BLAS root bounds, ObjectToWorld)
@@ -14,9 +16,11 @@
 #include <cmath>
 #include <cstring>
 #include <limits>
+#include <map>
 #include <string>
 #include <vector>
 
+#include "../device/scene_gpu.hpp"
 #include "../host/bvh_build.hpp"
 #include "../host/host_math.hpp"
 #include "context.hpp"
@@ -50,6 +54,7 @@ struct MeshPrep {
   std::vector<bn_bvh_node> nodes;
   std::vector<int32_t> perm;
   int node_base = 0, tri_base = 0, node4_root = -1;
+  bool on_device = false;  // nodes holds the root only, perm nothing
 };
 
 // The wide records of one binary BVH (layout in dev_types.cuh).  A record stands for an
@@ -178,6 +183,189 @@ cudaError_t upload(DevBuf& b, const std::vector<T>& v, cudaStream_t st) {
   return e;
 }
 
+void mesh_boxes(const bn_mesh_desc& m, std::vector<float>* boxes) {
+  boxes->resize(6 * static_cast<size_t>(m.n_triangles));
+  for (int t = 0; t < m.n_triangles; ++t) {
+    const V3 p0 = vtx(m, m.indices[3 * t]), p1 = vtx(m, m.indices[3 * t + 1]), p2 = vtx(m, m.indices[3 * t + 2]);
+    const V3 lo = bnh::min_native(bnh::min_native(p0, p1), p2), hi = bnh::max_native(bnh::max_native(p0, p1), p2);
+    float* b = &(*boxes)[6 * static_cast<size_t>(t)];
+    b[0] = lo.x; b[1] = lo.y; b[2] = lo.z; b[3] = hi.x; b[4] = hi.y; b[5] = hi.z;
+  }
+}
+
+// the mesh's triangles in permuted order and their reference alias pdfs, appended
+void mesh_tris(const bn_mesh_desc& m, const std::vector<int32_t>& perm, std::vector<float4>* tris, std::vector<float>* pdf) {
+  std::vector<float> areas(m.n_triangles);
+  float sum = 0.f;
+  for (int k = 0; k < m.n_triangles; ++k) {
+    const int t = perm[k];
+    const V3 p0 = vtx(m, m.indices[3 * t]), p1 = vtx(m, m.indices[3 * t + 1]), p2 = vtx(m, m.indices[3 * t + 2]);
+    const int slot = m.tri_material ? m.tri_material[t] : -1;
+    float slotf, tf;
+    std::memcpy(&slotf, &slot, 4);
+    std::memcpy(&tf, &t, 4);
+    tris->push_back(make_float4(p0.x, p0.y, p0.z, slotf));
+    tris->push_back(make_float4(p1.x, p1.y, p1.z, tf));
+    tris->push_back(make_float4(p2.x, p2.y, p2.z, 0.f));
+    areas[k] = 0.5f * bnh::length(bnh::cross(p1 - p0, p2 - p0));
+    sum = sum + areas[k];
+  }
+  for (int k = 0; k < m.n_triangles; ++k)
+    pdf->push_back(sum == 0.f ? 1.f / static_cast<float>(m.n_triangles) : areas[k] / sum);
+}
+
+// n bytes of b with its first `used` kept
+cudaError_t grow(DevBuf& b, size_t used, size_t n, cudaStream_t st) {
+  if (n <= b.bytes) return cudaSuccess;
+  DevBuf bigger;
+  cudaError_t e = bigger.reserve(n);
+  if (e == cudaSuccess && used) e = cudaMemcpyAsync(bigger.ptr, b.ptr, used, cudaMemcpyDeviceToDevice, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e != cudaSuccess) {
+    bigger.release();
+    return e;
+  }
+  b.release();
+  b = bigger;
+  return cudaSuccess;
+}
+
+// The BLASes of `meshes` (built on the GPU) into ctx->nodes from node tlas_room + *blas_nodes on, their
+// triangles and pdfs into ctx->tris and ctx->tri_pdf from host_tris on, and the parity of their
+// nodes' depths into ctx->bvh.scene_odd.
+int device_blases(bn_context* ctx, const bn_scene_desc* d, const std::vector<int>& meshes, int tlas_room, size_t n_tris,
+                  size_t host_tris, std::vector<MeshPrep>* mp, size_t* blas_nodes, std::vector<int32_t>* mesh_base) {
+  cudaStream_t st = ctx->stream;
+  bnc::BvhWork& k = ctx->bvh;
+  cudaError_t e;
+  size_t est = tlas_room + *blas_nodes;
+  for (int i : meshes) est += static_cast<size_t>(0.8 * d->meshes[i].n_triangles) + 200;  // leaves hold 2 to 3 boxes
+  if ((e = ctx->nodes.reserve(est * sizeof(bn_bvh_node))) != cudaSuccess ||
+      (e = ctx->tris.reserve(3 * n_tris * sizeof(float4))) != cudaSuccess ||
+      (e = ctx->tri_pdf.reserve(n_tris * sizeof(float))) != cudaSuccess)
+    return ctx->cuda_fail(e, "scene buffers");
+  const size_t first_node = *blas_nodes;
+  size_t tri_base = host_tris;
+  std::vector<std::vector<float>> areas(meshes.size());
+  for (size_t j = 0; j < meshes.size(); ++j) {
+    const int i = meshes[j], nt = d->meshes[i].n_triangles;
+    const bn_mesh_desc& m = d->meshes[i];
+    MeshPrep& p = (*mp)[i];
+    const size_t vb = 3 * static_cast<size_t>(m.n_vertices) * sizeof(float), ib = 3 * static_cast<size_t>(nt) * sizeof(int);
+    if ((e = k.vertices.reserve(vb)) != cudaSuccess || (e = k.indices.reserve(ib)) != cudaSuccess ||
+        (m.tri_material && (e = k.slots.reserve(nt * sizeof(int))) != cudaSuccess) ||
+        (e = k.bounds.reserve(6 * static_cast<size_t>(nt) * sizeof(float))) != cudaSuccess)
+      return ctx->cuda_fail(e, "mesh buffers");
+    cudaMemcpyAsync(k.vertices.ptr, m.vertices, vb, cudaMemcpyHostToDevice, st);
+    cudaMemcpyAsync(k.indices.ptr, m.indices, ib, cudaMemcpyHostToDevice, st);
+    if (m.tri_material) cudaMemcpyAsync(k.slots.ptr, m.tri_material, nt * sizeof(int), cudaMemcpyHostToDevice, st);
+    if ((e = bn::scene_launch_boxes(k.vertices.as<float>(), k.indices.as<int>(), nt, k.bounds.as<float>(), st)) != cudaSuccess)
+      return ctx->cuda_fail(e, "mesh boxes");
+    bool nan = false;
+    int n_nodes = 0;
+    const int rc = bnc::gpu_bvh_build_resident(ctx, k.bounds.as<float>(), nt, true, &nan, &n_nodes);
+    if (rc) return rc;
+    std::vector<unsigned char> odd;
+    if (nan) {
+      // the host builder's nodes and permutation, in the device's place
+      std::vector<float> boxes;
+      mesh_boxes(m, &boxes);
+      if (!bnh::bvh_build(boxes.data(), nt, &p.nodes, &p.perm))
+        return ctx->fail(BN_ERR_UNSUPPORTED, "mesh " + std::to_string(i) + ": BVH leaf larger than 127 triangles");
+      n_nodes = static_cast<int>(p.nodes.size());
+      odd.assign(n_nodes, 0);
+      for (int n = 0; n < n_nodes; ++n)
+        if (!p.nodes[n].is_leaf) odd[n + 1] = odd[p.nodes[n].right_or_offset] = !odd[n];
+    }
+    const size_t at = tlas_room + *blas_nodes;
+    if ((e = grow(ctx->nodes, at * sizeof(bn_bvh_node), (at + n_nodes) * sizeof(bn_bvh_node), st)) != cudaSuccess ||
+        (e = grow(k.scene_odd, *blas_nodes - first_node,
+                  std::max(*blas_nodes - first_node + n_nodes, est - tlas_room - first_node), st)) != cudaSuccess)
+      return ctx->cuda_fail(e, "scene nodes");
+    // bn_bvh_node is the walk's two float4 (put_node)
+    bn_bvh_node* dst = ctx->nodes.as<bn_bvh_node>() + at;
+    unsigned char* dst_odd = k.scene_odd.as<unsigned char>() + (*blas_nodes - first_node);
+    if (nan) {
+      cudaMemcpyAsync(dst, p.nodes.data(), n_nodes * sizeof(bn_bvh_node), cudaMemcpyHostToDevice, st);
+      cudaMemcpyAsync(dst_odd, odd.data(), n_nodes, cudaMemcpyHostToDevice, st);
+      if ((e = k.perm.reserve(nt * sizeof(int))) != cudaSuccess) return ctx->cuda_fail(e, "mesh permutation");
+      cudaMemcpyAsync(k.perm.ptr, p.perm.data(), nt * sizeof(int), cudaMemcpyHostToDevice, st);
+    } else {
+      cudaMemcpyAsync(dst, k.out.ptr, n_nodes * sizeof(bn_bvh_node), cudaMemcpyDeviceToDevice, st);
+      cudaMemcpyAsync(dst_odd, k.odd.ptr, n_nodes, cudaMemcpyDeviceToDevice, st);
+      p.nodes.resize(1);
+      cudaMemcpyAsync(p.nodes.data(), k.out.ptr, sizeof(bn_bvh_node), cudaMemcpyDeviceToHost, st);
+    }
+    float* pdf = ctx->tri_pdf.as<float>() + tri_base;
+    if ((e = bn::scene_launch_tris(k.vertices.as<float>(), k.indices.as<int>(), m.tri_material ? k.slots.as<int>() : nullptr,
+                                   k.perm.as<int>(), nt, ctx->tris.as<float4>() + 3 * tri_base, pdf, st)) != cudaSuccess)
+      return ctx->cuda_fail(e, "mesh triangles");
+    areas[j].resize(nt);
+    cudaMemcpyAsync(areas[j].data(), pdf, nt * sizeof(float), cudaMemcpyDeviceToHost, st);
+    // (also before the next mesh reuses the buffers)
+    if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return ctx->cuda_fail(e, "mesh triangles");
+    // the reference sums the areas in order, in 32 bits
+    float sum = 0.f;
+    for (float a : areas[j]) sum = sum + a;
+    if ((e = bn::scene_launch_pdf(pdf, nt, sum, st)) != cudaSuccess) return ctx->cuda_fail(e, "mesh pdfs");
+    p.on_device = true;
+    p.tri_base = static_cast<int>(tri_base);
+    p.node_base = static_cast<int>(*blas_nodes);
+    mesh_base->push_back(p.node_base);
+    tri_base += nt;
+    *blas_nodes += n_nodes;
+    if (*blas_nodes + tlas_room > 0x7fffffffu / 2) return ctx->fail(BN_ERR_UNSUPPORTED, "too many BVH nodes");
+  }
+  return BN_OK;
+}
+
+// The wide records of the device's BLASes behind the *n_records of the host, in ctx->nodes4.
+int device_records(bn_context* ctx, const std::vector<int>& meshes, const std::vector<int32_t>& mesh_base, int blas0,
+                   int host_nodes, int blas_nodes, std::vector<MeshPrep>* mp, size_t* n_records, bool* nested) {
+  cudaStream_t st = ctx->stream;
+  bnc::BvhWork& k = ctx->bvh;
+  const int nm = static_cast<int>(meshes.size());
+  bn::WideParams w{};
+  w.nodes = ctx->nodes.as<float4>();
+  w.base = blas0 + host_nodes;
+  w.n = blas_nodes - host_nodes;
+  w.odd = k.scene_odd.as<unsigned char>();
+  w.n_meshes = nm;
+  const int blocks = (w.n + 1023) / 1024;
+  cudaError_t e;
+  // rank | block sums | flag | roots | mesh bases
+  if ((e = k.wide.reserve((static_cast<size_t>(w.n) + blocks + 2 + 1 + 2 * nm) * sizeof(int))) != cudaSuccess)
+    return ctx->cuda_fail(e, "wide-record buffers");
+  w.rank = k.wide.as<int>();
+  w.sums = w.rank + w.n;
+  w.flags = w.sums + blocks + 2;
+  w.roots = w.flags + 1;
+  int* bases = w.roots + nm;
+  w.mesh_base = bases;
+  std::vector<int32_t> abs_base(mesh_base);
+  for (int32_t& b : abs_base) b += blas0;
+  cudaMemcpyAsync(bases, abs_base.data(), nm * sizeof(int), cudaMemcpyHostToDevice, st);
+  cudaMemsetAsync(w.flags, 0, sizeof(int), st);
+  int count = 0;
+  if ((e = bn::scene_launch_wide_count(w, st)) != cudaSuccess ||
+      (e = cudaMemcpyAsync(&count, w.sums + blocks, sizeof(int), cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
+      (e = cudaStreamSynchronize(st)) != cudaSuccess)
+    return ctx->cuda_fail(e, "wide records");
+  if ((e = ctx->nodes4.reserve((*n_records + count + 1) * 8 * sizeof(float4))) != cudaSuccess)
+    return ctx->cuda_fail(e, "wide records");
+  w.records = ctx->nodes4.as<float4>();
+  w.first_record = static_cast<int>(*n_records);
+  std::vector<int> back(1 + nm);
+  if ((e = bn::scene_launch_wide_fill(w, st)) != cudaSuccess ||
+      (e = cudaMemcpyAsync(back.data(), w.flags, back.size() * sizeof(int), cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
+      (e = cudaStreamSynchronize(st)) != cudaSuccess)
+    return ctx->cuda_fail(e, "wide records");
+  if (back[0]) *nested = false;
+  for (int j = 0; j < nm; ++j) (*mp)[meshes[j]].node4_root = back[1 + j];
+  *n_records += count;
+  return BN_OK;
+}
+
 }  // namespace
 
 extern "C" int bn_scene_upload(bn_context* ctx, const bn_scene_desc* d) {
@@ -195,9 +383,10 @@ extern "C" int bn_scene_upload(bn_context* ctx, const bn_scene_desc* d) {
     const bn_mesh_desc& m = d->meshes[i];
     if (m.n_triangles < 0 || m.n_vertices < 0 || (m.n_triangles > 0 && (!m.indices || !m.vertices)))
       return ctx->fail(BN_ERR_INVALID_ARG, "mesh " + std::to_string(i) + ": bad arrays");
-    for (long long k = 0; k < 3LL * m.n_triangles; ++k)
-      if (m.indices[k] < 0 || m.indices[k] >= m.n_vertices)
-        return ctx->fail(BN_ERR_INVALID_ARG, "mesh " + std::to_string(i) + ": vertex index out of range");
+    unsigned top = 0;  // the largest index; a negative one is larger than any other
+    for (long long k = 0; k < 3LL * m.n_triangles; ++k) top = std::max(top, static_cast<unsigned>(m.indices[k]));
+    if (m.n_triangles > 0 && top >= static_cast<unsigned>(m.n_vertices))
+      return ctx->fail(BN_ERR_INVALID_ARG, "mesh " + std::to_string(i) + ": vertex index out of range");
     if (m.tri_material)
       for (int k = 0; k < m.n_triangles; ++k)
         if (m.tri_material[k] < -1 || m.tri_material[k] >= d->n_materials)
@@ -229,50 +418,44 @@ extern "C" int bn_scene_upload(bn_context* ctx, const bn_scene_desc* d) {
   auto on_device = [&](int n) {
     return d->bvh_builder == BN_BUILDER_DEVICE || (d->bvh_builder == BN_BUILDER_AUTO && n >= 16384);
   };
+  const int ni = d->n_instances;
   std::vector<MeshPrep> mp(d->n_meshes);
   std::vector<float4> tris;
   std::vector<float> tri_pdf;
-  std::vector<bn_bvh_node> all_nodes;  // TLAS inserted in front later
   size_t blas_nodes = 0;
+  // meshes built on the host first (their nodes and triangles go up in one piece), then the others,
+  // whose buffers are filled on the device mesh by mesh
+  std::vector<int> device_meshes;
+  long long n_tris = 0;
   for (int i = 0; i < d->n_meshes; ++i) {
     const bn_mesh_desc& m = d->meshes[i];
-    std::vector<float> boxes(6 * static_cast<size_t>(m.n_triangles));
-    for (int t = 0; t < m.n_triangles; ++t) {
-      const V3 p0 = vtx(m, m.indices[3 * t]), p1 = vtx(m, m.indices[3 * t + 1]), p2 = vtx(m, m.indices[3 * t + 2]);
-      const V3 lo = bnh::min_native(bnh::min_native(p0, p1), p2), hi = bnh::max_native(bnh::max_native(p0, p1), p2);
-      float* b = &boxes[6 * static_cast<size_t>(t)];
-      b[0] = lo.x; b[1] = lo.y; b[2] = lo.z; b[3] = hi.x; b[4] = hi.y; b[5] = hi.z;
+    n_tris += m.n_triangles;
+    if (m.n_triangles > 0 && on_device(m.n_triangles)) {
+      device_meshes.push_back(i);
+      continue;
     }
-    if (on_device(m.n_triangles)) {
-      const int rc = bnc::gpu_bvh_build(ctx, boxes.data(), m.n_triangles, &mp[i].nodes, &mp[i].perm);
-      if (rc) return rc;
-    } else if (!bnh::bvh_build(boxes.data(), m.n_triangles, &mp[i].nodes, &mp[i].perm)) {
+    std::vector<float> boxes;
+    mesh_boxes(m, &boxes);
+    if (!bnh::bvh_build(boxes.data(), m.n_triangles, &mp[i].nodes, &mp[i].perm))
       return ctx->fail(BN_ERR_UNSUPPORTED, "mesh " + std::to_string(i) + ": BVH leaf larger than 127 triangles");
-    }
     mp[i].tri_base = static_cast<int>(tris.size() / 3);
     mp[i].node_base = static_cast<int>(blas_nodes);
     blas_nodes += mp[i].nodes.size();
-    std::vector<float> areas(m.n_triangles);
-    float sum = 0.f;
-    for (int k = 0; k < m.n_triangles; ++k) {
-      const int t = mp[i].perm[k];
-      const V3 p0 = vtx(m, m.indices[3 * t]), p1 = vtx(m, m.indices[3 * t + 1]), p2 = vtx(m, m.indices[3 * t + 2]);
-      const int slot = m.tri_material ? m.tri_material[t] : -1;
-      float slotf, tf;
-      std::memcpy(&slotf, &slot, 4);
-      std::memcpy(&tf, &t, 4);
-      tris.push_back(make_float4(p0.x, p0.y, p0.z, slotf));
-      tris.push_back(make_float4(p1.x, p1.y, p1.z, tf));
-      tris.push_back(make_float4(p2.x, p2.y, p2.z, 0.f));
-      areas[k] = 0.5f * bnh::length(bnh::cross(p1 - p0, p2 - p0));
-      sum = sum + areas[k];
-    }
-    for (int k = 0; k < m.n_triangles; ++k)
-      tri_pdf.push_back(sum == 0.f ? 1.f / static_cast<float>(m.n_triangles) : areas[k] / sum);
+    mesh_tris(m, mp[i].perm, &tris, &tri_pdf);
+  }
+  if (n_tris > 0x7fffffffLL / 3) return ctx->fail(BN_ERR_UNSUPPORTED, "too many triangles");
+  const size_t host_nodes = blas_nodes, host_tris = tris.size() / 3;
+  // The first BLAS node.  With meshes on the device the TLAS, whose size is not known yet, gets room
+  // for any tree over its instances (2 n nodes, or the 129 of a chain).
+  const int tlas_room = device_meshes.empty() ? 0 : std::max(2 * ni, 160);
+  std::vector<int32_t> mesh_base;  // first nodes of the device's meshes, relative to the first BLAS node
+  if (!device_meshes.empty()) {
+    const int rc = device_blases(ctx, d, device_meshes, tlas_room, static_cast<size_t>(n_tris), host_tris, &mp, &blas_nodes,
+                                 &mesh_base);
+    if (rc) return rc;
   }
 
   // ---- 3: instance world bounds
-  const int ni = d->n_instances;
   std::vector<float> ibox(6 * static_cast<size_t>(ni));
   for (int i = 0; i < ni; ++i) {
     const bn_instance_desc& in = d->instances[i];
@@ -310,15 +493,19 @@ extern "C" int bn_scene_upload(bn_context* ctx, const bn_scene_desc* d) {
     return ctx->fail(BN_ERR_UNSUPPORTED, "TLAS leaf larger than 127 instances");
   }
   const int n_tlas = static_cast<int>(tlas.size());
-  std::vector<float4> nodes(2 * (tlas.size() + blas_nodes));
+  const int blas0 = device_meshes.empty() ? n_tlas : tlas_room;
+  if (n_tlas > blas0) return ctx->fail(BN_ERR_UNSUPPORTED, "TLAS larger than two nodes per instance");
+  std::vector<float4> nodes(2 * (blas0 + host_nodes));
   for (size_t k = 0; k < tlas.size(); ++k) put_node(&nodes[2 * k], tlas[k]);
   for (int i = 0; i < d->n_meshes; ++i)
-    for (size_t k = 0; k < mp[i].nodes.size(); ++k) put_node(&nodes[2 * (n_tlas + mp[i].node_base + k)], mp[i].nodes[k]);
+    if (!mp[i].on_device)
+      for (size_t k = 0; k < mp[i].nodes.size(); ++k) put_node(&nodes[2 * (blas0 + mp[i].node_base + k)], mp[i].nodes[k]);
   // wide records for every BVH with an interior root (the TLAS's first, at record 0) when the
   // scene is walked wide: asked for, or automatically for scenes of 1,024+ nodes
   if (d->bvh_width != BN_BVH_AUTO && d->bvh_width != BN_BVH_BINARY && d->bvh_width != BN_BVH_WIDE)
     return ctx->fail(BN_ERR_INVALID_ARG, "bvh_width must be 0 (auto), 2 or 4");
-  const bool scene_wide = d->bvh_width == BN_BVH_WIDE || (d->bvh_width == BN_BVH_AUTO && nodes.size() / 2 >= 1024);
+  const bool scene_wide =
+      d->bvh_width == BN_BVH_WIDE || (d->bvh_width == BN_BVH_AUTO && n_tlas + blas_nodes >= 1024);
   std::vector<float4> nodes4;
   bool nested = true;
   if (scene_wide && !tlas[0].is_leaf) {
@@ -327,15 +514,21 @@ extern "C" int bn_scene_upload(bn_context* ctx, const bn_scene_desc* d) {
     nested = nested && c.nested;
   }
   for (int i = 0; i < d->n_meshes; ++i) {
-    if (!scene_wide || mp[i].nodes[0].is_leaf) continue;
+    if (!scene_wide || mp[i].on_device || mp[i].nodes[0].is_leaf) continue;
     Collapse c{mp[i].nodes, nodes4};
     mp[i].node4_root = c.emit(0);
     nested = nested && c.nested;
   }
+  size_t n_records = nodes4.size() / 8;
+  if (scene_wide && !device_meshes.empty() && nested) {
+    const int rc = device_records(ctx, device_meshes, mesh_base, blas0, static_cast<int>(host_nodes),
+                                  static_cast<int>(blas_nodes), &mp, &n_records, &nested);
+    if (rc) return rc;
+  }
   if (!nested) return ctx->fail(BN_ERR_INVALID_ARG, "non-finite triangle or instance bounds");
-  if (nodes4.size() / 8 >= (size_t{1} << 29))  // a stacked leaf slot is -1 - (4 * record + slot)
+  if (n_records >= (size_t{1} << 29))  // a stacked leaf slot is -1 - (4 * record + slot)
     return ctx->fail(BN_ERR_UNSUPPORTED, "scene too large for the wide BVH records");
-  if (nodes4.empty()) nodes4.resize(8);  // keep the buffer non-null
+  if (n_records == 0) nodes4.resize(8);  // keep the buffer non-null
 
   std::vector<bn::DevInstance> dinst(ni);
   std::vector<int32_t> inst_light(ni);
@@ -349,7 +542,7 @@ extern "C" int bn_scene_upload(bn_context* ctx, const bn_scene_desc* d) {
     columns(in.world_to_object, di.w2o);
     columns(in.object_to_world, di.o2w);
     di.prim_type = p.type == BN_PRIM_SPHERE ? bn::kPrimSphere : bn::kPrimMesh;
-    di.node_base = p.type == BN_PRIM_MESH ? n_tlas + mp[p.mesh].node_base : 0;
+    di.node_base = p.type == BN_PRIM_MESH ? blas0 + mp[p.mesh].node_base : 0;
     di.tri_base = p.type == BN_PRIM_MESH ? mp[p.mesh].tri_base : 0;
     di.n_tris = p.type == BN_PRIM_MESH ? d->meshes[p.mesh].n_triangles : 0;
     di.material = in.material;
@@ -372,6 +565,7 @@ extern "C" int bn_scene_upload(bn_context* ctx, const bn_scene_desc* d) {
   std::vector<bn::DevTriLight> tl;
   if (d->light_sampler == BN_LIGHTS_ALIAS_TRIANGLES) {
     std::vector<double> w;
+    std::map<int, std::vector<float4>> emitter_tris;
     for (int k : light_inst) {
       bn::DevInstance& di = dinst[k];
       if (di.prim_type != bn::kPrimMesh)
@@ -382,8 +576,24 @@ extern "C" int bn_scene_upload(bn_context* ctx, const bn_scene_desc* d) {
       const bn_light_desc& L = d->lights[in.light];
       const double lum = 0.2126 * L.emission[0] + 0.7152 * L.emission[1] + 0.0722 * L.emission[2];
       di.light_entry_base = static_cast<int>(tl.size());
+      // the triangles of an emitter built on the device come back once
+      const MeshPrep& em = mp[d->primitives[in.primitive].mesh];
+      const float4* mesh_tri = nullptr;
+      if (em.on_device) {
+        std::vector<float4>& back = emitter_tris[d->primitives[in.primitive].mesh];
+        if (back.empty() && di.n_tris > 0) {
+          back.resize(3 * static_cast<size_t>(di.n_tris));
+          cudaError_t e = cudaMemcpyAsync(back.data(), ctx->tris.as<float4>() + 3 * static_cast<size_t>(di.tri_base),
+                                          back.size() * sizeof(float4), cudaMemcpyDeviceToHost, ctx->stream);
+          if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+          if (e != cudaSuccess) return ctx->cuda_fail(e, "emitter triangles");
+        }
+        mesh_tri = back.data();
+      } else {
+        mesh_tri = tris.data() + 3 * static_cast<size_t>(di.tri_base);
+      }
       for (int j = 0; j < di.n_tris; ++j) {
-        const float4* t = &tris[3 * static_cast<size_t>(di.tri_base + j)];
+        const float4* t = mesh_tri + 3 * static_cast<size_t>(j);
         const V3 p0 = bnh::transform_point({t[0].x, t[0].y, t[0].z}, o2w);
         const V3 p1 = bnh::transform_point({t[1].x, t[1].y, t[1].z}, o2w);
         const V3 p2 = bnh::transform_point({t[2].x, t[2].y, t[2].z}, o2w);
@@ -432,6 +642,7 @@ extern "C" int bn_scene_upload(bn_context* ctx, const bn_scene_desc* d) {
   // ---- upload
   cudaStream_t st = ctx->stream;
   cudaError_t e;
+  // (with meshes on the device these buffers hold them already, behind the host's parts)
   if ((e = upload(ctx->nodes, nodes, st)) != cudaSuccess) return ctx->cuda_fail(e, "upload nodes");
   if ((e = upload(ctx->nodes4, nodes4, st)) != cudaSuccess) return ctx->cuda_fail(e, "upload wide nodes");
   if ((e = upload(ctx->tris, tris, st)) != cudaSuccess) return ctx->cuda_fail(e, "upload triangles");
@@ -442,6 +653,7 @@ extern "C" int bn_scene_upload(bn_context* ctx, const bn_scene_desc* d) {
   if ((e = upload(ctx->tri_pdf, tri_pdf, st)) != cudaSuccess) return ctx->cuda_fail(e, "upload triangle pdf");
   if ((e = upload(ctx->tri_lights, tl, st)) != cudaSuccess) return ctx->cuda_fail(e, "upload light table");
   if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return ctx->cuda_fail(e, "scene upload");
+  ctx->bvh.trim();
 
   bn::DevScene& s = ctx->scene;
   s.nodes = ctx->nodes.as<float4>();
@@ -455,10 +667,10 @@ extern "C" int bn_scene_upload(bn_context* ctx, const bn_scene_desc* d) {
   s.tri_lights = ctx->tri_lights.as<bn::DevTriLight>();
   s.n_inst = ni;
   s.n_tlas_nodes = n_tlas;
-  s.n_nodes = static_cast<int>(nodes.size() / 2);
-  s.n_nodes4 = static_cast<int>(nodes4.size() / 8);
+  s.n_nodes = static_cast<int>(blas0 + blas_nodes);
+  s.n_nodes4 = static_cast<int>(std::max<size_t>(n_records, 1));
   s.wide = scene_wide ? 1 : 0;
-  s.n_tris = static_cast<int>(tris.size() / 3);
+  s.n_tris = static_cast<int>(n_tris);
   s.n_light_inst = static_cast<int>(light_inst.size());
   s.n_tri_lights = static_cast<int>(tl.size());
   s.light_sampler = d->light_sampler;
