@@ -1,4 +1,5 @@
 // The C-ABI: contexts, queries, render dispatch and statistics.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <string>
@@ -73,11 +74,20 @@ bn::MegaParams mega_params(const bn_context* ctx, const bn_render_desc* d, const
   return p;
 }
 
+void queue_device_error(bn_context* ctx) {
+  cudaMemcpyAsync(ctx->pinned, ctx->error_word.ptr, sizeof(unsigned int), cudaMemcpyDeviceToHost, ctx->stream);
+}
+
 int check_device_error(bn_context* ctx) {
-  unsigned int w = 0;
-  cudaError_t e = cudaMemcpyAsync(&w, ctx->error_word.ptr, sizeof(w), cudaMemcpyDeviceToHost, ctx->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+  queue_device_error(ctx);
+  const cudaError_t e = cudaStreamSynchronize(ctx->stream);
   if (e != cudaSuccess) return ctx->cuda_fail(e, "kernel execution");
+  return queued_device_error(ctx);
+}
+
+int queued_device_error(bn_context* ctx) {
+  unsigned int w = 0;
+  std::memcpy(&w, ctx->pinned, sizeof(w));
   ctx->stats.device_error = w;
   if (w) {
     cudaMemsetAsync(ctx->error_word.ptr, 0, sizeof(unsigned int), ctx->stream);
@@ -166,7 +176,8 @@ int bn_create(int device, bn_context** out) {
       (e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking)) != cudaSuccess ||
       (e = cudaEventCreate(&ctx->ev0)) != cudaSuccess || (e = cudaEventCreate(&ctx->ev1)) != cudaSuccess ||
       (e = cudaEventCreate(&ctx->ev2)) != cudaSuccess || (e = ctx->error_word.reserve(256)) != cudaSuccess ||
-      (e = ctx->counters.reserve(sizeof(bn::DevCounters))) != cudaSuccess) {
+      (e = ctx->counters.reserve(sizeof(bn::DevCounters))) != cudaSuccess ||
+      (e = cudaHostAlloc(reinterpret_cast<void**>(&ctx->pinned), bnc::kPinnedBytes, cudaHostAllocDefault)) != cudaSuccess) {
     delete ctx;
     return BN_ERR_CUDA;
   }
@@ -187,6 +198,7 @@ int bn_destroy(bn_context* ctx) {
                     &ctx->adj_grad, &ctx->adj_aux, &ctx->adj_scene, &ctx->adj_rec};
   for (DevBuf* b : bufs) b->release();
   ctx->bvh.release();
+  cudaFreeHost(ctx->pinned);
   if (ctx->wf && ctx->wf_release) ctx->wf_release(ctx->wf);
   cudaEventDestroy(ctx->ev0);
   cudaEventDestroy(ctx->ev1);
@@ -222,15 +234,22 @@ int bn_trace(bn_context* ctx, const bn_ray* rays, int64_t n, uint32_t flags, bn_
   cudaError_t e;
   if ((e = ctx->q_in.reserve(n * sizeof(bn_ray))) != cudaSuccess) return ctx->cuda_fail(e, "alloc rays");
   if ((e = ctx->q_out.reserve(n * sizeof(bn_hit))) != cudaSuccess) return ctx->cuda_fail(e, "alloc hits");
-  cudaMemcpyAsync(ctx->q_in.ptr, rays, n * sizeof(bn_ray), cudaMemcpyHostToDevice, ctx->stream);
   if (flags & BN_TRACE_COUNT) cudaMemsetAsync(ctx->counters.ptr, 0, sizeof(bn::DevCounters), ctx->stream);
+  cudaMemcpyAsync(ctx->q_in.ptr, rays, n * sizeof(bn_ray), cudaMemcpyHostToDevice, ctx->stream);
   cudaEventRecord(ctx->ev0, ctx->stream);
   if ((e = bn::launch_trace(ctx->scene, ctx->q_in.as<bn_ray>(), ctx->q_out.as<bn_hit>(), n, flags,
+                            reinterpret_cast<unsigned long long*>(static_cast<char*>(ctx->error_word.ptr) + 64),
                             ctx->counters.as<bn::DevCounters>(), ctx->stream)) != cudaSuccess)
     return ctx->cuda_fail(e, "trace launch");
   cudaEventRecord(ctx->ev1, ctx->stream);
-  cudaMemcpyAsync(hits, ctx->q_out.ptr, n * sizeof(bn_hit), cudaMemcpyDeviceToHost, ctx->stream);
+  // short results come through pinned memory with the error word, so the call waits once
+  const size_t bytes = n * sizeof(bn_hit);
+  const bool staged = bytes <= bnc::kPinnedBytes - 64;
+  bnc::queue_device_error(ctx);
+  cudaMemcpyAsync(staged ? ctx->pinned + 64 : reinterpret_cast<char*>(hits), ctx->q_out.ptr, bytes, cudaMemcpyDeviceToHost,
+                  ctx->stream);
   if ((e = cudaStreamSynchronize(ctx->stream)) != cudaSuccess) return ctx->cuda_fail(e, "trace");
+  if (staged) std::memcpy(hits, ctx->pinned + 64, bytes);
   float ms = 0.f;
   cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
   ctx->stats.last_kernel_ms = ms;
@@ -247,7 +266,7 @@ int bn_trace(bn_context* ctx, const bn_ray* rays, int64_t n, uint32_t flags, bn_
   } else {
     ctx->stats.rays += static_cast<uint64_t>(n);
   }
-  return bnc::check_device_error(ctx);
+  return bnc::queued_device_error(ctx);
 }
 
 static int bsdf_common(bn_context* ctx, const bn_bsdf_query* q, int64_t n, bn_bsdf_result* out, bool sample) {

@@ -33,6 +33,7 @@ struct DevBuf {
 };
 
 namespace bnc {
+constexpr size_t kPinnedBytes = 65536;
 // the GPU BVH builder's buffers (bvh_gpu.cu)
 struct BvhWork {
   DevBuf bounds, items, ranges, level, nodes, out, perm, odd, counters;
@@ -48,11 +49,12 @@ struct bn_context {
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr;
   std::string err;
+  char* pinned = nullptr;  // bnc::kPinnedBytes of pinned host memory: the error word, then short results
 
   // scene
   bool has_scene = false;
   bn::DevScene scene{};
-  // error_word: 256 bytes, the BN_DEVERR_* word at 0 and the path machine's item counter at 64
+  // error_word: 256 bytes, the BN_DEVERR_* word at 0, the counter of claimed items at 64
   DevBuf nodes, nodes4, tris, inst, mats, lights, light_inst, tri_pdf, tri_lights, error_word, counters;
   std::vector<int32_t> inst_order;     // TLAS order -> descriptor index
   std::vector<bn::DevMaterial> host_mats;
@@ -95,7 +97,11 @@ struct bn_context {
 namespace bnc {
 // host-side view constants (Extensions/Camera/Pinhole.fs:16-22), shared by all render modes
 bn::DevView make_dev_view(const bn_view& v, long long pixel_offset, long long path_offset);
+// Waits for the stream and reports the device error word (BN_ERR_DEVICE, the word cleared); or the
+// same in two parts around a wait that the call makes anyway.
 int check_device_error(bn_context* ctx);
+void queue_device_error(bn_context* ctx);
+int queued_device_error(bn_context* ctx);
 // The plain megakernel's sample chunks: each work item runs spc consecutive samples of one pixel,
 // chunks = ceil(spp / spc) items per pixel.  max_items > 0 caps pixels * chunks (fixed scratch).
 struct MegaChunks {

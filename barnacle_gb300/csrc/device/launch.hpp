@@ -49,8 +49,9 @@ struct DevCounters {
   unsigned long long rays, nodes, tris, insts, paths, accepted, proposed, pad;
 };
 
+// next: the counter of claimed rays (scratch)
 cudaError_t launch_trace(const DevScene& s, const bn_ray* rays, bn_hit* hits, long long n, unsigned flags,
-                         DevCounters* counters, cudaStream_t st);
+                         unsigned long long* next, DevCounters* counters, cudaStream_t st);
 cudaError_t launch_bsdf(const DevScene& s, const bn_bsdf_query* q, bn_bsdf_result* out, long long n, bool sample,
                         cudaStream_t st);
 cudaError_t launch_sampler_stream(const uint32_t* seeds, long long n_streams, int n_draws, float* out, cudaStream_t st);
