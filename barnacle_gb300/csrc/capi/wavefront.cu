@@ -14,9 +14,9 @@ namespace {
 
 struct WfState {
   int pool = 0;
-  DevBuf params, ray, bl, hit, meta, q_active, q_bins, shadow, counters, work_next, film_acc;
+  DevBuf params, slot, q_active, q_bins, q_done, shadow, counters, work_next, film_acc;
   DevBuf mlt_smp, mlt_chain;  // PSSMLT chains: sampler state and chain records
-  DevBuf slot_key, q_key, q_ray, sh_key, q_shadow, hist, off;
+  DevBuf q_key, q_ray, sh_key, q_shadow, hist, off;
   DevBuf path_L;              // radiance per path of a batch (ordered renders)
   // captured graph (one per launch shape)
   cudaGraph_t graph = nullptr;
@@ -37,8 +37,8 @@ struct WfState {
   }
 
   void release() {
-    DevBuf* b[] = {&params, &ray, &bl, &hit, &meta, &q_active, &q_bins, &shadow, &counters,
-                   &work_next, &film_acc, &slot_key, &q_key, &q_ray, &sh_key, &q_shadow, &hist, &off,
+    DevBuf* b[] = {&params, &slot, &q_active, &q_bins, &q_done, &shadow, &counters,
+                   &work_next, &film_acc, &q_key, &q_ray, &sh_key, &q_shadow, &hist, &off,
                    &mlt_smp, &mlt_chain, &path_L};
     for (DevBuf* x : b) x->release();
     if (exec) cudaGraphExecDestroy(exec);
@@ -69,24 +69,21 @@ cudaError_t ensure_pool(WfState* w, int pool) {
   cudaError_t e;
   const size_t P = static_cast<size_t>(pool);
   if ((e = w->params.reserve(sizeof(bn::WfParams))) != cudaSuccess) return e;
-  if ((e = w->ray.reserve(2 * P * sizeof(float4))) != cudaSuccess) return e;
-  if ((e = w->bl.reserve(2 * P * sizeof(float4))) != cudaSuccess) return e;
-  if ((e = w->hit.reserve(2 * P * sizeof(float4))) != cudaSuccess) return e;
-  if ((e = w->meta.reserve(P * sizeof(int4))) != cudaSuccess) return e;
+  if ((e = w->slot.reserve(8 * P * sizeof(float4))) != cudaSuccess) return e;
   if ((e = w->q_active.reserve(P * sizeof(int))) != cudaSuccess) return e;
   if ((e = w->q_bins.reserve(P * bn::kNumBins * sizeof(int))) != cudaSuccess) return e;
   if ((e = w->shadow.reserve(P * 4 * sizeof(float4))) != cudaSuccess) return e;
   if ((e = w->counters.reserve(bn::kCntSize * sizeof(int))) != cudaSuccess) return e;
   if ((e = w->work_next.reserve(sizeof(unsigned long long))) != cudaSuccess) return e;
-  for (DevBuf* b : {&w->slot_key, &w->q_key, &w->q_ray, &w->sh_key, &w->q_shadow})
+  for (DevBuf* b : {&w->q_done, &w->q_key, &w->q_ray, &w->sh_key, &w->q_shadow})
     if ((e = b->reserve(P * sizeof(int))) != cudaSuccess) return e;
-  if ((e = w->hist.reserve(bn::kSortBins * sizeof(unsigned))) != cudaSuccess) return e;
+  if ((e = w->hist.reserve(2 * bn::kSortBins * sizeof(unsigned))) != cudaSuccess) return e;
   if ((e = w->off.reserve((bn::kSortBins + bn::kSortBins / 1024) * sizeof(unsigned))) != cudaSuccess) return e;
   w->pool = pool;
   return cudaSuccess;
 }
 
-// Path slots of a render that does not choose them: one per path, up to 64 M (15 GB).  Every path
+// Path slots of a render that does not choose them: one per path, up to 64 M (16 GB).  Every path
 // then starts at once, the queues are as long and the sorted rays as coherent as they can be, and
 // a bounce is one iteration; fewer slots cost more, short iterations, more slots only add rows to
 // scan.  Measured (kernel ms by log2 of the slots, the render's paths in brackets): Cornell box
@@ -178,11 +175,9 @@ int run(bn_context* ctx, WfState* w, const bn::DevScene& scene, const bn_render_
   p.max_iters = static_cast<int>(std::min<long long>(1LL << 30, ((end - first) / pool + 2) * (d->max_depth + 2) + 64));
   // bn_set_limits' cap is the wavefront mode's
   if (ctx->limit_iters > 0 && !ordered) p.max_iters = ctx->limit_iters;
-  p.ray = w->ray.as<float4>();
-  p.bl = w->bl.as<float4>();
-  p.hit = w->hit.as<float4>();
-  p.meta = w->meta.as<int4>();
+  p.slot = w->slot.as<float4>();
   p.q_active = w->q_active.as<int>();
+  p.q_done = w->q_done.as<int>();
   p.sort = sort ? 1 : 0;
   p.sort_shadow = sort_shadow ? 1 : 0;
   {
@@ -196,7 +191,6 @@ int run(bn_context* ctx, WfState* w, const bn::DevScene& scene, const bn_render_
     p.key_scale = make_float4(sc[0], sc[1], sc[2], 0.f);
     p.key_bits = key_bits;
   }
-  p.slot_key = w->slot_key.as<int>();
   p.q_key = w->q_key.as<int>();
   p.q_ray = sort ? w->q_ray.as<int>() : w->q_active.as<int>();
   p.sh_key = w->sh_key.as<int>();
@@ -226,13 +220,16 @@ int run(bn_context* ctx, WfState* w, const bn::DevScene& scene, const bn_render_
   cudaStream_t st = ctx->stream;
   cudaMemcpyAsync(w->params.ptr, &p, sizeof(p), cudaMemcpyHostToDevice, st);
   cudaMemsetAsync(w->counters.ptr, 0, bn::kCntSize * sizeof(int), st);
-  cudaMemsetAsync(w->hist.ptr, 0, bn::kSortBins * sizeof(unsigned), st);
+  for (int k = 0; k < 2; ++k)  // the bins in use of both queues' counts
+    cudaMemsetAsync(w->hist.as<unsigned>() + k * bn::kSortBins, 0, (sizeof(unsigned) << (2 * key_bits + 6)), st);
   cudaMemsetAsync(w->work_next.ptr, 0, sizeof(unsigned long long), st);
-  cudaMemsetAsync(w->meta.ptr, 0, static_cast<size_t>(pool) * sizeof(int4), st);
   if (!ordered) cudaMemsetAsync(w->film_acc.ptr, 0, static_cast<size_t>(n_pixels) * 3 * sizeof(double), st);
   cudaEventRecord(ctx->ev0, st);
   int launches = 0;
-  if (use_graph) {
+  if (p.max_depth <= 0 && p.integrator == BN_INTEGRATOR_PATH) {
+    // PathTracing: while (depth < maxDepth) never runs, every path's radiance is zero
+    // (Normal and Direct ignore maxDepth)
+  } else if (use_graph) {
     if ((e = cudaGraphLaunch(w->exec, st)) != cudaSuccess) return ctx->cuda_fail(e, "cudaGraphLaunch");
   } else {
     for (int it = 0; it < p.max_iters + 1; ++it) {
@@ -308,11 +305,9 @@ int run_mlt(bn_context* ctx, WfState* w, const bn_render_desc* d, const bn::MltP
   p.max_iters = static_cast<int>(std::min<long long>(
       1LL << 30, (static_cast<long long>(mp.mutations_per_chain) + 1) * (std::max(1, d->max_depth) + 1) + 64));
   if (ctx->limit_iters > 0) p.max_iters = ctx->limit_iters;
-  p.ray = w->ray.as<float4>();
-  p.bl = w->bl.as<float4>();
-  p.hit = w->hit.as<float4>();
-  p.meta = w->meta.as<int4>();
+  p.slot = w->slot.as<float4>();
   p.q_active = w->q_active.as<int>();
+  p.q_done = w->q_done.as<int>();
   p.sort = 0;
   p.sort_shadow = 0;
   p.key_bits = 5;
@@ -346,7 +341,7 @@ int run_mlt(bn_context* ctx, WfState* w, const bn_render_desc* d, const bn::MltP
   cudaStream_t st = ctx->stream;
   cudaMemcpyAsync(w->params.ptr, &p, sizeof(p), cudaMemcpyHostToDevice, st);
   cudaMemsetAsync(w->counters.ptr, 0, bn::kCntSize * sizeof(int), st);
-  cudaMemsetAsync(w->meta.ptr, 0, static_cast<size_t>(pool) * sizeof(int4), st);  // every chain unstarted
+  cudaMemsetAsync(w->slot.ptr, 0, static_cast<size_t>(pool) * 8 * sizeof(float4), st);  // every chain unstarted
   // (checking the loop condition every 4 or 16 iterations instead of every one measured slower:
   // 499 and 510 against 450 ms)
   for (int it = 0; it < p.max_iters + 1; ++it) {

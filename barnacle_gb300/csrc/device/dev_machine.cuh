@@ -5,7 +5,7 @@
 // per instruction, in PSSMLT's chains 4.  Here each lane is a small state machine that always
 // holds a walk (a closest hit or a shadow ray, of whatever bounce of whatever path), and the warp
 // alternates two things:
-//   * walk     the walking lanes vote on the kind of unit (trav_vote_full) and the winners take one
+//   * walk     the walking lanes vote on the kind of unit (TravVote) and the winners take one
 //              step of their walk;
 //   * service  once at most a quarter of the lanes still walk, every lane whose walk has ended is served
 //              together: a shadow ray's answer is added, a hit is shaded, an ended path is handed
@@ -29,15 +29,14 @@
 
 namespace bn {
 
-// the vote of trav_vote for whole warps (every lane calls it)
-__device__ __forceinline__ bool trav_vote_full(bool walking, int mode) {
-  const unsigned b0 = __ballot_sync(0xffffffffu, !walking || (mode & 1));
-  const unsigned b1 = __ballot_sync(0xffffffffu, !walking || (mode & 2));
-  const int cn = 2 * __popc(~(b0 | b1));
-  const int ct = 2 * __popc(b0 & ~b1);
-  const int ci = 3 * __popc(b1 & ~b0);
-  const int pick = (cn >= ct && cn >= ci) ? kTravNode : (ct >= ci ? kTravTri : kTravInst);
-  return walking && mode == pick;
+// a warp's walking lanes step until at most `stop` of them still walk (every lane calls it)
+template <int kAny, bool kWT, int kWalk, class Stack>
+__device__ __forceinline__ void walk_down_to(int stop, Trav& tr, const DevScene& s, Stack& stk, TraceCounters* tc) {
+  for (;;) {
+    const TravVote v(0xffffffffu, true, tr.mode);
+    if (v.walking() <= stop) break;
+    if (tr.mode == v.pick()) trav_step<kAny, kWT, kWalk, 4, true>(tr, s, stk, tc);
+  }
 }
 
 // Lanes of a warp that take paths: n paths spread over every warp of the grid when there are
@@ -149,9 +148,7 @@ __device__ __forceinline__ void path_machine(const DevScene& s, Task& task, Smp&
     // walk until few lanes still do
     const unsigned busy = __ballot_sync(0xffffffffu, phase != kLaneIdle);
     if (!busy) break;
-    const int stop = __popc(busy) * kMachineRefill / 32;
-    while (__popc(__ballot_sync(0xffffffffu, tr.mode != kTravDone)) > stop)
-      if (trav_vote_full(tr.mode != kTravDone, tr.mode)) trav_step<kAnyRuntime, kWT, kWalk, 4, true>(tr, s, stk, &tc);
+    walk_down_to<kAnyRuntime, kWT, kWalk>(__popc(busy) * kMachineRefill / 32, tr, s, stk, &tc);
   }
 }
 

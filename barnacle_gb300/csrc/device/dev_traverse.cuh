@@ -22,7 +22,7 @@
 //    into the step that needs them, so lanes at different levels run the same loop body and
 //    reconverge after every step instead of waiting out each other's nested BLAS loops.  A
 //    caller can refill a lane with a new ray as soon as its walk finishes, and let only the
-//    lanes at one kind of unit take a step (trav_vote).
+//    lanes at one kind of unit take a step (TravVote).
 
 namespace bn {
 
@@ -218,7 +218,9 @@ __device__ __forceinline__ int sel4(int a, int b, int c, int d, int i) {
 }
 
 // one wide step: the four slot boxes of record tr.cur; returns kStepPop when none is entered,
-// kStepOverflow when the stack is full
+// kStepOverflow when the stack is full.  The slots are put in visit order by three conditional swaps
+// (with the triangle test before a leaf's box test this took 6 instanced views of 4 spp from 95.3 to
+// 90.8 ms; selecting each slot by its number cost twice the instructions)
 enum : int { kStepOk = 0, kStepPop = 1, kStepOverflow = 2 };
 template <class Stack>
 __device__ __forceinline__ int trav_node4(Trav& tr, const DevScene& s, Stack& stk) {
@@ -234,39 +236,37 @@ __device__ __forceinline__ int trav_node4(Trav& tr, const DevScene& s, Stack& st
   const bool h1 = box_hit_t(mk(lx.y, ly.y, lz.y), mk(hx.y, hy.y, hz.y), r, inv, tr.t, &e1);
   const bool h2 = box_hit_t(mk(lx.z, ly.z, lz.z), mk(hx.z, hy.z, hz.z), r, inv, tr.t, &e2);
   const bool h3 = box_hit_t(mk(lx.w, ly.w, lz.w), mk(hx.w, hy.w, hz.w), r, inv, tr.t, &e3);
-  const int hm = int(h0) | (int(h1) << 1) | (int(h2) << 2) | (int(h3) << 3);
-  if (!hm) return kStepPop;
+  if (!(h0 | h1 | h2 | h3)) return kStepPop;
+  // what a stack entry says of each slot: a record, -1 - (4 * record + slot) for a leaf (records
+  // number less than 2^29), or nothing entered
+  constexpr int kNone = static_cast<int>(0x80000000u);
+  const int m = meta.y, nb = ~(4 * tr.cur);
+  const int c0 = !h0 ? kNone : ((m & 1) ? nb : ref.x), c1 = !h1 ? kNone : ((m & 2) ? nb - 1 : ref.y);
+  const int c2 = !h2 ? kNone : ((m & 4) ? nb - 2 : ref.z), c3 = !h3 ? kNone : ((m & 8) ? nb - 3 : ref.w);
   // the binary walk's order (the near child's slots, then the far child's, each pair ordered by
   // that child's own split axis: BVH.fs near-child rule at both levels) depends on the ray only
-  // through its octant; the upload stored the slot order of each octant, 8 bits per octant
-  const int m = meta.y;
+  // through its octant; the upload stored the slot order of each octant, 8 bits per octant: bit 1
+  // swaps the pairs, bits 0 and 4 the slots of the pair then first and second
   const int oct = tr.level ? tr.ooct : tr.woct;
-  const unsigned order = (static_cast<unsigned>(oct & 4 ? meta.w : meta.z) >> (8 * (oct & 3))) & 0xffu;
-  int v[4];
-  v[0] = order & 3;
-  v[1] = (order >> 2) & 3;
-  v[2] = (order >> 4) & 3;
-  v[3] = (order >> 6) & 3;
-  int first = 3;
-#pragma unroll
-  for (int k = 2; k >= 0; --k)
-    if ((hm >> v[k]) & 1) first = k;
-  const int extra = __popc(hm) - 1;
-  if (tr.sp + extra > s.stack_cap) return kStepOverflow;
-  // stack the later hits so that they pop in visit order
-#pragma unroll
-  for (int k = 3; k >= 1; --k) {
-    const int sl = v[k];
-    if (k > first && ((hm >> sl) & 1)) {
-      stk.put(tr.sp, ((m >> sl) & 1) ? -1 - (4 * tr.cur + sl) : sel4(ref.x, ref.y, ref.z, ref.w, sl),
-              sel4(e0, e1, e2, e3, sl));
-      ++tr.sp;
-    }
+  const unsigned order = static_cast<unsigned>(oct & 4 ? meta.w : meta.z) >> (8 * (oct & 3));
+  const bool sp = order & 2u, sa = order & 1u, sb = order & 16u;
+  const int a0 = sp ? c2 : c0, a1 = sp ? c3 : c1, b0 = sp ? c0 : c2, b1 = sp ? c1 : c3;
+  const float ea0 = sp ? e2 : e0, ea1 = sp ? e3 : e1, eb0 = sp ? e0 : e2, eb1 = sp ? e1 : e3;
+  const int v0 = sa ? a1 : a0, v1 = sa ? a0 : a1, v2 = sb ? b1 : b0, v3 = sb ? b0 : b1;
+  const float t1 = sa ? ea0 : ea1, t2 = sb ? eb1 : eb0, t3 = sb ? eb0 : eb1;
+  // the first slot entered comes next; the later ones are stacked to pop in order
+  const bool p0 = v0 != kNone, p1 = v1 != kNone, p2 = v2 != kNone, p3 = v3 != kNone;
+  if (tr.sp + 3 > s.stack_cap && tr.sp + int(p0) + int(p1) + int(p2) + int(p3) - 1 > s.stack_cap) return kStepOverflow;
+  if (p3 && (p0 | p1 | p2)) stk.put(tr.sp++, v3, t3);
+  if (p2 && (p0 | p1)) stk.put(tr.sp++, v2, t2);
+  if (p1 && p0) stk.put(tr.sp++, v1, t1);
+  const int next = p0 ? v0 : (p1 ? v1 : (p2 ? v2 : v3));
+  if (next >= 0) {
+    tr.cur = next;
+  } else {
+    const int sl = (-1 - next) & 3;
+    trav_enter_leaf(tr, sel4(ref.x, ref.y, ref.z, ref.w, sl), (meta.x >> (8 * sl)) & 0xff);
   }
-  const int sl = v[first];
-  const int rf = sel4(ref.x, ref.y, ref.z, ref.w, sl);
-  if ((m >> sl) & 1) trav_enter_leaf(tr, rf, (meta.x >> (8 * sl)) & 0xff);
-  else tr.cur = rf;
   return kStepOk;
 }
 
@@ -316,8 +316,9 @@ __device__ __forceinline__ bool trav_step(Trav& tr, const DevScene& s, Stack& st
       pop = true;
     }
   } else if (tr.mode == kTravTri) {
-    // kTris triangles of a BLAS leaf (0: the rest of the leaf): each its AABB pre-test
-    // (Mesh.fs:204,231), then the triangle test
+    // kTris triangles of a BLAS leaf (0: the rest of the leaf): each the triangle test, then its AABB
+    // test (Mesh.fs:204,231).  The reference tests the box first; a hit needs both, and the triangle
+    // test turns most triangles away earlier.
     int done = 0;
 #pragma unroll 1
     while (tr.ti < tr.ti_end) {
@@ -326,12 +327,12 @@ __device__ __forceinline__ bool trav_step(Trav& tr, const DevScene& s, Stack& st
       const float4 a = __ldg(tp), b = __ldg(tp + 1), c = __ldg(tp + 2);
       if (kCount) cnt->tris++;
       const V3 p0 = xyz(a), p1 = xyz(b), p2 = xyz(c);
-      const V3 lo = min_native(min_native(p0, p1), p2), hi = max_native(max_native(p0, p1), p2);
-      if (box_hit(lo, hi, tr.orr, tr.oinv, tr.t)) {
-        float tt, uu, vv;
-        const bool h = kWT ? tri_wt(p0, p1, p2, tr.orr, tr.wt, tr.t, &tt, &uu, &vv)
-                           : tri_mt(p0, p1, p2, tr.orr, tr.t, &tt, &uu, &vv);
-        if (h) {
+      float tt, uu, vv;
+      const bool h = kWT ? tri_wt(p0, p1, p2, tr.orr, tr.wt, tr.t, &tt, &uu, &vv)
+                         : tri_mt(p0, p1, p2, tr.orr, tr.t, &tt, &uu, &vv);
+      if (h) {
+        const V3 lo = min_native(min_native(p0, p1), p2), hi = max_native(max_native(p0, p1), p2);
+        if (box_hit(lo, hi, tr.orr, tr.oinv, tr.t)) {
           tr.found = true;
           if (any) {
             tr.mode = kTravDone;
@@ -419,21 +420,25 @@ __device__ __forceinline__ bool trav_step(Trav& tr, const DevScene& s, Stack& st
 
 // Lanes of a warp at different kinds of unit (a node record, a leaf's triangles, instances) run
 // different branches of a step one after the other, each with its own chain of dependent loads.
-// With this vote only the lanes in the mode with the largest weighted count take the step
-// (instances weigh 3, nodes and triangles 2); the others keep their state and wait.  Each lane's
-// sequence of units is unchanged, so its result is too.  Call it with every lane of the warp
-// that is in the loop; walking = the lane holds a walk that is not finished.
-__device__ __forceinline__ bool trav_vote(bool walking, int mode) {
-  static_assert(kTravNode == 0 && kTravTri == 1 && kTravInst == 2 && kTravDone == 3, "mode bits");
-  // two ballots on the mode's bits; a lane that is not walking counts as done (both bits)
-  const unsigned act = __activemask();
-  const unsigned b0 = __ballot_sync(act, !walking || (mode & 1)), b1 = __ballot_sync(act, !walking || (mode & 2));
-  const int cn = 2 * __popc(act & ~(b0 | b1));
-  const int ct = 2 * __popc(b0 & ~b1);
-  const int ci = 3 * __popc(b1 & ~b0);
-  const int pick = (cn >= ct && cn >= ci) ? kTravNode : (ct >= ci ? kTravTri : kTravInst);
-  return mode == pick || mode == kTravDone;
-}
+// With a vote only the lanes in the mode with the largest weighted count take the step (instances
+// weigh 3, nodes and triangles 2); the others keep their state and wait.  Each lane's sequence of
+// units is unchanged, so its result is too.  The vote is two ballots on the mode's bits, which also
+// tell how many lanes still walk; a lane that does not counts as done (both bits).
+struct TravVote {
+  unsigned act, b0, b1;
+  __device__ __forceinline__ TravVote(unsigned lanes, bool walking, int mode) : act(lanes) {
+    static_assert(kTravNode == 0 && kTravTri == 1 && kTravInst == 2 && kTravDone == 3, "mode bits");
+    b0 = __ballot_sync(act, !walking || (mode & 1));
+    b1 = __ballot_sync(act, !walking || (mode & 2));
+  }
+  __device__ __forceinline__ int walking() const { return __popc(act & ~(b0 & b1)); }
+  __device__ __forceinline__ int pick() const {
+    const int cn = 2 * __popc(act & ~(b0 | b1));
+    const int ct = 2 * __popc(b0 & ~b1);
+    const int ci = 3 * __popc(b1 & ~b0);
+    return (cn >= ct && cn >= ci) ? kTravNode : (ct >= ci ? kTravTri : kTravInst);
+  }
+};
 
 // A walk, inlined at its call site with the query fixed at compile time.
 template <int kAny, bool kWT, int kWalk>

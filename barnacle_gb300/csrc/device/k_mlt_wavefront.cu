@@ -73,7 +73,8 @@ __global__ void __launch_bounds__(256) k_mlt_regen(const WfParams* __restrict__ 
   // whole warps: the splats and the queue appends are warp-wide
   for (int chain = blockIdx.x * blockDim.x + threadIdx.x; chain < nw; chain += gridDim.x * blockDim.x) {
     const bool valid = chain < q.n_chains;
-    int4 st = valid ? p.meta[chain] : make_int4(0, 0, 0, kChainDone);
+    float4* rec = p.slot + 8LL * chain;
+    int4 st = valid ? *reinterpret_cast<const int4*>(rec + 6) : make_int4(0, 0, 0, kChainDone);
     bool queued = valid && st.w == kChainPath;
     Splat step{-1, mk(0.f, 0.f, 0.f)}, last{-1, mk(0.f, 0.f, 0.f)};
     if (valid && (st.w == kChainFree || st.w == kChainStep)) {
@@ -104,7 +105,7 @@ __global__ void __launch_bounds__(256) k_mlt_regen(const WfParams* __restrict__ 
         c0 = cr[0];
         c1 = cr[1];
         c2 = cr[2];
-        const float4 l4 = p.bl[2 * chain + 1];
+        const float4 l4 = rec[5];
         const V3 Ln = mk(l4.x, l4.y, l4.z);
         const float yn = luminance(Ln);
         const int it = __float_as_int(c2.y), npix = __float_as_int(c2.z);
@@ -154,10 +155,10 @@ __global__ void __launch_bounds__(256) k_mlt_regen(const WfParams* __restrict__ 
         int nx, ny;
         const Ray ray = mlt_camera(v, m, &nx, &ny);
         c2.z = __int_as_float((H - ny - 1) * W + nx);
-        p.ray[2 * chain] = make_float4(ray.o.x, ray.o.y, ray.o.z, 0.f);
-        p.ray[2 * chain + 1] = make_float4(ray.d.x, ray.d.y, ray.d.z, 0.f);
-        p.bl[2 * chain] = make_float4(1.f, 1.f, 1.f, 0.f);
-        p.bl[2 * chain + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
+        rec[0] = make_float4(ray.o.x, ray.o.y, ray.o.z, 0.f);
+        rec[1] = make_float4(ray.d.x, ray.d.y, ray.d.z, 0.f);
+        rec[4] = make_float4(1.f, 1.f, 1.f, 0.f);
+        rec[5] = make_float4(0.f, 0.f, 0.f, 0.f);
         st = make_int4(0, 0, 0, kChainPath);
         if (p.max_depth <= 0) st.w = kChainStep;  // while (depth < maxDepth) never runs
         else queued = true;
@@ -178,7 +179,7 @@ __global__ void __launch_bounds__(256) k_mlt_regen(const WfParams* __restrict__ 
     const int qi = append(&p.counters[kCntActiveNext], queued);
     if (queued && qi < p.pool) p.q_active[qi] = chain;
     else if (queued) flag_error(p.scene, BN_DEVERR_QUEUE_OVERFLOW);
-    if (valid) p.meta[chain] = st;
+    if (valid) *reinterpret_cast<int4*>(rec + 6) = st;
     // chains not finished keep the loop going (k_wf_control reads the count)
     const unsigned pending = __ballot_sync(0xffffffffu, valid && st.w != kChainDone);
     if ((threadIdx.x & 31) == 0 && pending) atomicAdd(&p.counters[kCntDone], __popc(pending));
@@ -200,23 +201,24 @@ __global__ void __launch_bounds__(128) k_mlt_shade(const WfParams* __restrict__ 
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nw; i += stride) {
     const bool valid = i < total;
     bool done = false, cont = false, shadow = false;
-    float4 sh_o, sh_d, sh_a, sh_b;
+    float4 sh_o, sh_d, sh_L;
     if (valid) {
       int b = 0, off = i;
       while (off >= cnt[b]) { off -= cnt[b]; ++b; }
       const int slot = p.q_bins[static_cast<long long>(b) * p.pool + off];
-      int4 st = p.meta[slot];
-      const float4 hf = p.hit[2 * slot];
+      float4* rec = p.slot + 8LL * slot;
+      int4 st = *reinterpret_cast<const int4*>(rec + 6);
+      const float4 hf = rec[2];
       const int hinst = __float_as_int(hf.w);
       if (b == kBinMiss || hinst < 0) {
         done = true;
       } else {
-        const float4 o = p.ray[2 * slot], d = p.ray[2 * slot + 1];
+        const float4 o = rec[0], d = rec[1];
         Ray ray;
         ray.o = mk(o.x, o.y, o.z);
         ray.d = mk(d.x, d.y, d.z);
         const float pdf_bsdf = d.w;
-        const int hprim = __float_as_int(p.hit[2 * slot + 1].x);
+        const int hprim = __float_as_int(rec[3].x);
         HitRec h;
         h.t = hf.x; h.u = hf.y; h.v = hf.z;
         h.inst = hinst;
@@ -224,9 +226,9 @@ __global__ void __launch_bounds__(128) k_mlt_shade(const WfParams* __restrict__ 
         h.tri = sphere ? 0 : hprim;
         h.sphere_root = sphere ? hprim : 0;
         const Interaction it = make_interaction(s, ray, h);
-        const float4 b4 = p.bl[2 * slot];
+        const float4 b4 = rec[4];
         V3 beta = mk(b4.x, b4.y, b4.z);
-        const float4 L4 = p.bl[2 * slot + 1];
+        const float4 L4 = rec[5];
         V3 L = mk(L4.x, L4.y, L4.z);
         const int depth = st.y;
         MltSampler m = chain_sampler<kKelemen>(q, slot);
@@ -257,8 +259,8 @@ __global__ void __launch_bounds__(128) k_mlt_shade(const WfParams* __restrict__ 
             const V3 bb = scale(__frcp_rn(__fadd_rn(be.pdf, ls.pdf)), ls.L);
             sh_o = make_float4(it.p.x, it.p.y, it.p.z, __fsub_rn(dist, 1e-3f));
             sh_d = make_float4(ls.wi.x, ls.wi.y, ls.wi.z, __int_as_float(slot));
-            sh_a = make_float4(a.x, a.y, a.z, 0.f);
-            sh_b = make_float4(bb.x, bb.y, bb.z, 0.f);
+            const V3 Lt = fma3(a, bb, L);
+            sh_L = make_float4(Lt.x, Lt.y, Lt.z, 0.f);
             shadow = shadow_contributes(a, bb, L);
           }
           const BsdfSample bs = bsdf_sample(mt, to_local(it.f, wo_w), u_lobe, ubx, uby);
@@ -275,20 +277,20 @@ __global__ void __launch_bounds__(128) k_mlt_shade(const WfParams* __restrict__ 
             }
             if (alive && depth + 1 < p.max_depth) {
               cont = true;
-              p.ray[2 * slot] = make_float4(it.p.x, it.p.y, it.p.z, 0.f);
-              p.ray[2 * slot + 1] = make_float4(nd.x, nd.y, nd.z, bs.pdf);
-              p.bl[2 * slot] = make_float4(beta.x, beta.y, beta.z, 0.f);
+              rec[0] = make_float4(it.p.x, it.p.y, it.p.z, 0.f);
+              rec[1] = make_float4(nd.x, nd.y, nd.z, bs.pdf);
+              rec[4] = make_float4(beta.x, beta.y, beta.z, 0.f);
               st.y = depth + 1;
             } else {
               done = true;
             }
           }
         }
-        p.bl[2 * slot + 1] = make_float4(L.x, L.y, L.z, 0.f);
+        rec[5] = make_float4(L.x, L.y, L.z, 0.f);
         q.smp[slot] = m.pack();
       }
       st.w = done ? (shadow ? kChainWait : kChainStep) : kChainPath;
-      p.meta[slot] = st;
+      *reinterpret_cast<int4*>(rec + 6) = st;
     }
     const int si = append(&p.counters[kCntShadowNext], shadow);
     if (shadow && si >= p.pool) {
@@ -297,7 +299,7 @@ __global__ void __launch_bounds__(128) k_mlt_shade(const WfParams* __restrict__ 
     }
     if (shadow) {
       float4* r = p.shadow + 4LL * si;
-      r[0] = sh_o; r[1] = sh_d; r[2] = sh_a; r[3] = sh_b;
+      r[0] = sh_o; r[1] = sh_d; r[2] = sh_L;
     }
   }
 }

@@ -112,10 +112,7 @@ __global__ void __launch_bounds__(kMachineThreads, kTraceBlocks)
     }
     const unsigned busy = __ballot_sync(0xffffffffu, phase != kLaneIdle);
     if (!busy) break;
-    const int stop = __popc(busy) / 2;
-    while (__popc(__ballot_sync(0xffffffffu, tr.mode != kTravDone)) > stop)
-      if (trav_vote_full(tr.mode != kTravDone, tr.mode))
-        trav_step<kAny ? kAnyHit : kClosest, kWT, kWalk, 4, true>(tr, s, stk, &tc);
+    walk_down_to<kAny ? kAnyHit : kClosest, kWT, kWalk>(__popc(busy) / 2, tr, s, stk, &tc);
   }
 }
 

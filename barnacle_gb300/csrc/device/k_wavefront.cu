@@ -1,18 +1,17 @@
 // The batched wavefront form of PathTracingIntegrator.Li (PathTracing.fs:14-81) over many views.
 //
-// A pool of P path slots lives in HBM, one array per kind of record (WfParams: each slot's ray,
-// throughput + radiance and hit are 32-byte records, one DRAM sector each).  One iteration of the
+// A pool of P path slots lives in HBM, a 128-byte record each (WfParams::slot).  One iteration of the
 // bounce loop is:
-//   regen    every slot (four 32-slot rows per warp): retire a finished path into the FP64 film,
-//            refill free slots with new camera paths (warp-aggregated claims on a global path
-//            counter), and append the active slots to the ray queue (ballot + popc compaction)
-//            with their sort keys
+//   regen    every slot whose path has ended (all of them at first; four rows of 32 per warp): retire
+//            the path into the FP64 film or path_L, claim a new camera path (warp-aggregated claims on
+//            a global path counter) and append it to the ray queue with its sort key
 //   sort     counting sort of the ray queue by key (octant, origin cell): scan + scatter
 //   extend   closest hit for the ray queue (persistent lanes that vote on the kind of traversal
-//            step, trav_vote); each hit is binned by the material type it shades
+//            step, TravVote); each hit is binned by the material type it shades
 //            with (__match_any_sync groups, one atomic per group) so shading runs type-sorted
 //   shade    emission with MIS, light sample + BSDF eval (a shadow-ray record), BSDF sample,
-//            Russian roulette; marks paths that end
+//            Russian roulette; paths that go on are appended to the next iteration's ray queue with
+//            their keys, the others to the queue of ended ones
 //   sort     the same counting sort of the shadow queue
 //   shadow   any hit for the shadow queue; unoccluded records add their NEE term to L
 //   control  one thread: decides whether another iteration is needed, resets the counters and
@@ -29,11 +28,10 @@
 namespace bn {
 namespace {
 
-constexpr int kStatusFree = 0, kStatusActive = 1, kStatusDone = 2;
 constexpr int kBinMiss = 4, kBinNoMaterial = 5;
 // the wavefront's traversal step: one wide record, up to 4 triangles of a BLAS leaf (a whole leaf
 // but for the builder's depth-capped ones), or a TLAS leaf's instances until one is entered; only
-// the lanes that win the mode vote (trav_vote) take it
+// the lanes that win the mode vote (TravVote) take it
 constexpr int kWfTris = 4;
 constexpr bool kWfInstRun = true;
 // blocks of 128 per SM the traversal kernels are compiled for (registers: 65,536 / (128 x blocks))
@@ -81,14 +79,25 @@ __device__ __forceinline__ int ray_key(const WfParams& p, V3 o, V3 d) {
   return static_cast<int>((oct << b) | m);
 }
 
-// histogram of the keys of the lanes with pred; lanes with equal keys share one atomic.  Called
-// by whole warps.
+// histogram of the keys of the lanes with pred; lanes with equal keys share one atomic (an atomic per
+// lane made a Cornell render 18 % longer, and the scatter's the same).  Called by whole warps.
 __device__ __forceinline__ void hist_add(unsigned* hist, int key, bool pred) {
   const unsigned peers = __match_any_sync(0xffffffffu, pred ? key : -1);
   if (pred && (threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(hist + key, static_cast<unsigned>(__popc(peers)));
 }
 
-// One warp takes kRegenRows rows of 32 slots at a time: their states are loaded together, so a
+// Appends of a whole warp: the lanes with pred get consecutive entries of the queue, one atomic per
+// warp.  Returns the entry; a queue holds at most one entry per slot, the check only guards the buffers.
+__device__ __forceinline__ int push(const WfParams& p, int* counter, bool* pred) {
+  const int i = warp_append(counter, *pred);
+  if (*pred && i >= p.pool) {
+    flag_error(p.scene, BN_DEVERR_QUEUE_OVERFLOW);
+    *pred = false;
+  }
+  return i;
+}
+
+// One warp takes kRegenRows rows of 32 ended paths at a time: their records are loaded together, so a
 // warp has that many independent loads in flight instead of one dependent chain per row, and the
 // path claims and queue appends of all its rows share one atomic each.
 constexpr int kRegenRows = 4;
@@ -99,109 +108,94 @@ __global__ void __launch_bounds__(256) k_wf_regen(const WfParams* __restrict__ p
   const int lane = threadIdx.x & 31;
   const unsigned below = (1u << lane) - 1u;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, n_warps = (gridDim.x * blockDim.x) >> 5;
-  const int rows = (p.pool + 31) >> 5;
+  const bool fresh = p.counters[kCntIter] == 0;  // every slot is free
+  const int n = fresh ? p.pool : min(p.counters[kCntRetire], p.pool);
+  const int rows = (n + 31) >> 5;
   // the loop runs in whole warps so the warp-wide claims and appends see all 32 lanes
   for (int r0 = warp * kRegenRows; r0 < rows; r0 += n_warps * kRegenRows) {
     int slot[kRegenRows];
     bool valid[kRegenRows];
-    int4 m[kRegenRows];
 #pragma unroll
     for (int k = 0; k < kRegenRows; ++k) {
-      slot[k] = (r0 + k) * 32 + lane;
-      valid[k] = slot[k] < p.pool;
-      m[k] = valid[k] ? p.meta[slot[k]] : make_int4(0, 0, 0, kStatusActive);
+      const int i = (r0 + k) * 32 + lane;
+      valid[k] = i < n;
+      slot[k] = valid[k] ? (fresh ? i : p.q_done[i]) : 0;
     }
-    // retire finished paths into the film
-    float4 L[kRegenRows];
+    if (!fresh) {
+      // retire the paths
+      float4 L[kRegenRows];
+      int at[kRegenRows];
 #pragma unroll
-    for (int k = 0; k < kRegenRows; ++k)
-      if (valid[k] && m[k].w == kStatusDone) L[k] = p.bl[2 * slot[k] + 1];
-    // (lanes retiring samples of the same pixel could first sum in a warp and share one set of
-    // atomics; measured 0.5% slower than one set per lane on the instanced workload)
-#pragma unroll
-    for (int k = 0; k < kRegenRows; ++k) {
-      if (valid[k] && m[k].w == kStatusDone) {
-        if (p.path_L) {  // kept path by path, summed in order afterwards (k_mega_chunks)
-          __stcs(p.path_L + m[k].x, L[k]);
-          m[k].w = kStatusFree;
-          continue;
+      for (int k = 0; k < kRegenRows; ++k)
+        if (valid[k]) {
+          const float4* r = p.slot + 8LL * slot[k];
+          L[k] = r[5];
+          at[k] = __float_as_int(r[6].x);
         }
-        double* f = p.film_acc + 3LL * m[k].x;
-        atomicAdd(f, static_cast<double>(__fmul_rn(L[k].x, inv_spp)));
-        atomicAdd(f + 1, static_cast<double>(__fmul_rn(L[k].y, inv_spp)));
-        atomicAdd(f + 2, static_cast<double>(__fmul_rn(L[k].z, inv_spp)));
-        m[k].w = kStatusFree;
-      }
-    }
-    // claim new paths for the free slots of all rows with one atomic
-    unsigned wmask[kRegenRows];
-    int nwant = 0;
-#pragma unroll
-    for (int k = 0; k < kRegenRows; ++k) {
-      wmask[k] = __ballot_sync(0xffffffffu, valid[k] && m[k].w == kStatusFree);
-      nwant += __popc(wmask[k]);
-    }
-    if (nwant) {
-      unsigned long long first = 0;
-      if (lane == 0) first = atomicAdd(p.work_next, static_cast<unsigned long long>(nwant));
-      first = __shfl_sync(0xffffffffu, first, 0);
+      // (lanes retiring samples of the same pixel could first sum in a warp and share one set of
+      // atomics; measured 0.5% slower than one set per lane on the instanced workload)
 #pragma unroll
       for (int k = 0; k < kRegenRows; ++k) {
-        const long long id = p.first_path + static_cast<long long>(first) + __popc(wmask[k] & below);
-        first += __popc(wmask[k]);
-        if (!((wmask[k] >> lane) & 1u) || id >= p.total_paths) continue;
+        if (!valid[k]) continue;
+        if (p.path_L) {  // kept path by path, summed in order afterwards (k_mega_chunks)
+          __stcs(p.path_L + at[k], L[k]);
+        } else {
+          double* f = p.film_acc + 3LL * at[k];
+          atomicAdd(f, static_cast<double>(__fmul_rn(L[k].x, inv_spp)));
+          atomicAdd(f + 1, static_cast<double>(__fmul_rn(L[k].y, inv_spp)));
+          atomicAdd(f + 2, static_cast<double>(__fmul_rn(L[k].z, inv_spp)));
+        }
+      }
+    }
+    // claim new paths for all rows with one atomic
+    const int nwant = min(n - r0 * 32, 32 * kRegenRows);
+    unsigned long long first = 0;
+    if (lane == 0) first = atomicAdd(p.work_next, static_cast<unsigned long long>(nwant));
+    first = __shfl_sync(0xffffffffu, first, 0);
+    const long long left = p.total_paths - p.first_path - static_cast<long long>(first);
+    if (left <= 0) continue;  // (the whole warp)
+    const int ngot = static_cast<int>(left < nwant ? left : nwant);
+    int qbase = 0;
+    if (lane == 0) qbase = atomicAdd(&p.counters[kCntActive], ngot);
+    qbase = __shfl_sync(0xffffffffu, qbase, 0);
+#pragma unroll
+    for (int k = 0; k < kRegenRows; ++k) {
+      const int j = k * 32 + lane;  // the rows are full but for the last
+      const bool got = j < ngot;
+      int key = 0;
+      if (got) {
+        const long long id = p.first_path + static_cast<long long>(first) + j;
         const int vi = find_view(p, id);
         const DevView& v = p.views[vi];
         // path ids run over the samples of a pixel first, so a warp's claims are mostly the
-        // samples of one pixel (their retirements share atomics, see above)
+        // samples of one pixel
         const long long local = id - v.path_offset;
         const long long pix = local / p.spp;
         const int sid = static_cast<int>(local - pix * p.spp);
-        const int x = static_cast<int>(pix % v.width), y = static_cast<int>(pix / v.width);
+        const int y = static_cast<int>(pix / v.width), x = static_cast<int>(pix - static_cast<long long>(y) * v.width);
         IndepSampler smp{xxhash32_three(static_cast<uint32_t>(x), static_cast<uint32_t>(y),
                                         static_cast<uint32_t>(p.frame_id * p.spp + sid))};
         const float upx = smp.next(), upy = smp.next();
         const float ulx = smp.next(), uly = smp.next();
         const Ray ray = camera_ray(v, x, y, upx, upy, ulx, uly);
-        float4* rr = p.ray + 2 * slot[k];
-        rr[0] = make_float4(ray.o.x, ray.o.y, ray.o.z, 0.f);
-        rr[1] = make_float4(ray.d.x, ray.d.y, ray.d.z, 0.f);  // .w: pdf of the last BSDF sample
-        if (p.sort) p.slot_key[slot[k]] = ray_key(p, ray.o, ray.d);
-        float4* bl = p.bl + 2 * slot[k];
-        bl[0] = make_float4(1.f, 1.f, 1.f, 0.f);
-        bl[1] = make_float4(0.f, 0.f, 0.f, 0.f);
         const long long film_pix = v.pixel_offset + static_cast<long long>(v.height - y - 1) * v.width + x;
-        m[k] = make_int4(static_cast<int>(p.path_L ? id - p.first_path : film_pix), 0, static_cast<int>(smp.state), kStatusActive);
-        // PathTracing: while (depth < maxDepth) never runs; Normal and Direct ignore maxDepth
-        if (p.max_depth <= 0 && p.integrator == BN_INTEGRATOR_PATH) m[k].w = kStatusDone;
+        float4* r = p.slot + 8LL * slot[k];
+        r[0] = make_float4(ray.o.x, ray.o.y, ray.o.z, 0.f);
+        r[1] = make_float4(ray.d.x, ray.d.y, ray.d.z, 0.f);  // .w: pdf of the last BSDF sample
+        r[4] = make_float4(1.f, 1.f, 1.f, 0.f);
+        r[5] = make_float4(0.f, 0.f, 0.f, 0.f);
+        r[6] = make_float4(__int_as_float(static_cast<int>(p.path_L ? id - p.first_path : film_pix)), __int_as_float(0),
+                           __uint_as_float(smp.state), 0.f);
+        key = ray_key(p, ray.o, ray.d);
+        const int qi = qbase + j;
+        if (qi < p.pool) {
+          p.q_active[qi] = slot[k];
+          p.q_key[qi] = key;
+        } else {
+          flag_error(p.scene, BN_DEVERR_QUEUE_OVERFLOW);
+        }
       }
-    }
-    // append the active slots of all rows to the ray queue with one atomic
-    unsigned amask[kRegenRows];
-    int nact = 0;
-#pragma unroll
-    for (int k = 0; k < kRegenRows; ++k) {
-      amask[k] = __ballot_sync(0xffffffffu, valid[k] && m[k].w == kStatusActive);
-      nact += __popc(amask[k]);
-    }
-    int qbase = 0;
-    if (nact && lane == 0) qbase = atomicAdd(&p.counters[kCntActive], nact);
-    qbase = __shfl_sync(0xffffffffu, qbase, 0);
-#pragma unroll
-    for (int k = 0; k < kRegenRows; ++k) {
-      const bool active = (amask[k] >> lane) & 1u;
-      const int qi = qbase + __popc(amask[k] & below);
-      qbase += __popc(amask[k]);
-      // a queue holds at most one entry per slot; the checks only guard the buffers
-      const bool fits = qi < p.pool;
-      if (active && !fits) flag_error(p.scene, BN_DEVERR_QUEUE_OVERFLOW);
-      if (active && fits) p.q_active[qi] = slot[k];
-      if (p.sort) {
-        const int key = active ? p.slot_key[slot[k]] : 0;
-        if (active && fits) p.q_key[qi] = key;
-        hist_add(p.hist, key, active && fits);
-      }
-      if (valid[k]) p.meta[slot[k]] = m[k];
+      hist_add(p.hist, key, got);
     }
   }
 }
@@ -267,15 +261,17 @@ __global__ void __launch_bounds__(128, kExtendBlocks) k_wf_extend(const WfParams
   TraceCounters tc{0, 0, 0};
   unsigned long long nrays = 0;  // rays this lane walked (counting walks)
   int slot = -1;
-  bool have = false, pending = false;
+  bool have = false;
   for (;;) {
-    if (__popc(__ballot_sync(__activemask(), have)) <= refill_below) {
-      if (pending) {
-        pending = false;
+    // (a walk can end at init, its root box missed)
+    TravVote vote(__activemask(), have, tr.mode);
+    if (vote.walking() <= refill_below) {
+      if (have && tr.mode == kTravDone) {
+        have = false;
         int bin = kBinMiss;
+        float4* hr = p.slot + 8LL * slot + 2;
         if (tr.found) {
           const HitRec& h = tr.hit;
-          float4* hr = p.hit + 2 * slot;
           hr[0] = make_float4(h.t, h.u, h.v, __int_as_float(h.inst));
           hr[1] = make_float4(__int_as_float(h.sphere_root ? h.sphere_root : h.tri), 0.f, 0.f, 0.f);
           const DevInstance* I = s.inst + h.inst;
@@ -286,7 +282,7 @@ __global__ void __launch_bounds__(128, kExtendBlocks) k_wf_extend(const WfParams
           }
           bin = m < 0 ? kBinNoMaterial : s.mats[m].type;
         } else {
-          p.hit[2 * slot] = make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
+          hr[0] = make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
         }
         // material binning among the lanes finishing together: equal keys share one atomic
         const unsigned act = __activemask();
@@ -304,7 +300,7 @@ __global__ void __launch_bounds__(128, kExtendBlocks) k_wf_extend(const WfParams
       if (!have) {
         if (qi >= n) break;
         slot = p.q_ray[qi];
-        const float4 o = p.ray[2 * slot], d = p.ray[2 * slot + 1];
+        const float4 o = p.slot[8LL * slot], d = p.slot[8LL * slot + 1];
         Ray ray;
         ray.o = mk(o.x, o.y, o.z);
         ray.d = mk(d.x, d.y, d.z);
@@ -312,26 +308,21 @@ __global__ void __launch_bounds__(128, kExtendBlocks) k_wf_extend(const WfParams
         have = true;
         ++nrays;
       }
+      vote = TravVote(__activemask(), have, tr.mode);
     }
-    // a walk can end at init (root box missed)
-    const bool go = trav_vote(have, tr.mode);
-    if (have && go && (tr.mode == kTravDone || trav_step<kClosest, kWT, kWalk, kWfTris, kWfInstRun>(tr, s, stk, &tc))) {
-      have = false;
-      pending = true;
-    }
+    if (have && tr.mode == vote.pick()) trav_step<kClosest, kWT, kWalk, kWfTris, kWfInstRun>(tr, s, stk, &tc);
   }
   if (kWalk == kWalkCount) add_trace_counts(p.trace_counters, nrays, tc);
 }
 
 // DirectIntegrator.Li (Extensions/Integrator/Direct.fs:10-40) as two wavefront vertices.  At the
-// camera hit: emission seen directly (EvalEmit(-d)), a shadow record for one light sample (a = f,
-// b = L_light / pdf_light; the shadow kernel adds fma(a, b, L) if unoccluded, as the reference's
-// FusedMultiplyAdd), and a BSDF sample that always continues with beta = f.  At the second hit:
+// camera hit: emission seen directly (EvalEmit(-d)), a shadow record for one light sample (L with f * L_light / pdf_light
+// added, as the reference's FusedMultiplyAdd, if the shadow ray gets through), and a BSDF sample that always continues with beta = f.  At the second hit:
 // a light scores fma(beta, Le / pdf_light, L); the path ends either way.
 __device__ __forceinline__ void shade_direct(const WfParams& p, const DevScene& s, int slot, const Ray& ray,
                                              const Interaction& it, int depth, IndepSampler& smp, V3* beta, V3* L,
-                                             bool* done, bool* cont, bool* shadow, float4* sh_o, float4* sh_d,
-                                             float4* sh_a, float4* sh_b) {
+                                             V3* next_d, float* next_pdf, bool* done, bool* cont, bool* shadow,
+                                             float4* sh_o, float4* sh_d, float4* sh_L) {
   const int light = __ldg(&s.inst[it.inst].light);
   if (depth > 0) {
     if (light >= 0) {
@@ -358,22 +349,24 @@ __device__ __forceinline__ void shade_direct(const WfParams& p, const DevScene& 
   const V3 bb = scale(__frcp_rn(ls.pdf), ls.L);
   *sh_o = make_float4(it.p.x, it.p.y, it.p.z, __fsub_rn(dist, 1e-3f));
   *sh_d = make_float4(ls.wi.x, ls.wi.y, ls.wi.z, __int_as_float(slot));
-  *sh_a = make_float4(be.f.x, be.f.y, be.f.z, 0.f);
-  *sh_b = make_float4(bb.x, bb.y, bb.z, 0.f);
+  const V3 Ln = fma3(be.f, bb, *L);
+  *sh_L = make_float4(Ln.x, Ln.y, Ln.z, 0.f);
   *shadow = shadow_contributes(be.f, bb, *L);
   const float u_lobe = smp.next(), ubx = smp.next(), uby = smp.next();
   const BsdfSample bs = bsdf_sample(mt, to_local(it.f, wo_w), u_lobe, ubx, uby);
-  const V3 nd = to_world(it.f, bs.wi);
+  *next_d = to_world(it.f, bs.wi);
+  *next_pdf = bs.pdf;
   *beta = bs.f;
-  p.ray[2 * slot] = make_float4(it.p.x, it.p.y, it.p.z, 0.f);
-  p.ray[2 * slot + 1] = make_float4(nd.x, nd.y, nd.z, bs.pdf);
-  p.bl[2 * slot] = make_float4(bs.f.x, bs.f.y, bs.f.z, 0.f);
-  if (p.sort) p.slot_key[slot] = ray_key(p, it.p, nd);
   *cont = true;
 }
 
+// Bound by its loads' latency (20 warps per SM at 96 registers, 36 % of the issue slots used; a Cornell
+// bounce of 3.7 M paths takes 415 us and moves 1.04 GB of DRAM, 1.63 GB when a slot's fields lay in
+// separate 32-byte records).  6 and 8 blocks per SM, prefetching the next record into L2 or L1, and
+// fetching a warp's 32 records as whole lines through shared memory were each 0 to 5 % slower on it
+// (the last 1.3 % faster on the instanced scene, 2.5 % slower on all-PBR materials).
 template <bool kWT>
-__global__ void __launch_bounds__(128) k_wf_shade(const WfParams* __restrict__ pp) {
+__global__ void __launch_bounds__(128, 5) k_wf_shade(const WfParams* __restrict__ pp) {
   const WfParams& p = *pp;
   const DevScene& s = p.scene;
   int cnt[kNumBins], total = 0;
@@ -383,26 +376,28 @@ __global__ void __launch_bounds__(128) k_wf_shade(const WfParams* __restrict__ p
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nw; i += stride) {
     const bool valid = i < total;
     bool done = false, cont = false, shadow = false;
-    int slot = 0;
-    float4 sh_o, sh_d, sh_a, sh_b;
+    int slot = 0, key = 0;
+    float4 sh_o, sh_d, sh_L;
     if (valid) {
       int b = 0, off = i;
       while (off >= cnt[b]) { off -= cnt[b]; ++b; }
       slot = p.q_bins[static_cast<long long>(b) * p.pool + off];
-      int4 m = p.meta[slot];
-      const float4 hf = p.hit[2 * slot];
+      float4* rec = p.slot + 8LL * slot;
+      const float4 m = rec[6];
+      const float4 hf = rec[2];
       const int hinst = __float_as_int(hf.w);
-      const long long vertex = static_cast<long long>(m.y) * (p.total_paths - p.first_path) + m.x;
+      const int depth = __float_as_int(m.y);
+      const long long vertex = static_cast<long long>(depth) * (p.total_paths - p.first_path) + __float_as_int(m.x);
       if (hinst < 0) {
         if (p.rec) p.rec[vertex] = make_float4(0.f, __int_as_float(-1), 0.f, 0.f);
         done = true;
       } else {
-        const float4 o = p.ray[2 * slot], d = p.ray[2 * slot + 1];
+        const float4 o = rec[0], d = rec[1];
         Ray ray;
         ray.o = mk(o.x, o.y, o.z);
         ray.d = mk(d.x, d.y, d.z);
         const float pdf_bsdf = d.w;
-        const int hprim = __float_as_int(p.hit[2 * slot + 1].x);
+        const int hprim = __float_as_int(rec[3].x);
         if (p.rec) p.rec[vertex] = make_float4(hf.x, hf.w, __int_as_float(hprim), 0.f);
         HitRec h;
         h.t = hf.x; h.u = hf.y; h.v = hf.z;
@@ -411,19 +406,19 @@ __global__ void __launch_bounds__(128) k_wf_shade(const WfParams* __restrict__ p
         h.tri = sphere ? 0 : hprim;
         h.sphere_root = sphere ? hprim : 0;
         const Interaction it = make_interaction(s, ray, h);
-        const float4 b4 = p.bl[2 * slot];
+        const float4 b4 = rec[4], L4 = rec[5];
         V3 beta = mk(b4.x, b4.y, b4.z);
-        float4 L4 = p.bl[2 * slot + 1];
         V3 L = mk(L4.x, L4.y, L4.z);
-        const int depth = m.y;
+        V3 nd = L;
+        float pdf_next = 0.f;
         const DevInstance* I = s.inst + it.inst;
-        IndepSampler smp{static_cast<uint32_t>(m.z)};
+        IndepSampler smp{__float_as_uint(m.z)};
         if (p.integrator == BN_INTEGRATOR_NORMAL) {
           L = normal_color(it.f.n);
           done = true;
         } else if (p.integrator == BN_INTEGRATOR_DIRECT) {
-          shade_direct(p, s, slot, ray, it, depth, smp, &beta, &L, &done, &cont, &shadow, &sh_o, &sh_d, &sh_a, &sh_b);
-          if (cont) m.y = 1;
+          shade_direct(p, s, slot, ray, it, depth, smp, &beta, &L, &nd, &pdf_next, &done, &cont, &shadow, &sh_o, &sh_d,
+                       &sh_L);
         } else {
         if (__ldg(&I->light) >= 0) {
           V3 le;
@@ -447,8 +442,8 @@ __global__ void __launch_bounds__(128) k_wf_shade(const WfParams* __restrict__ p
             const V3 bb = scale(__frcp_rn(__fadd_rn(be.pdf, ls.pdf)), ls.L);
             sh_o = make_float4(it.p.x, it.p.y, it.p.z, __fsub_rn(dist, 1e-3f));
             sh_d = make_float4(ls.wi.x, ls.wi.y, ls.wi.z, __int_as_float(slot));
-            sh_a = make_float4(a.x, a.y, a.z, __int_as_float(static_cast<int>(vertex)));
-            sh_b = make_float4(bb.x, bb.y, bb.z, __int_as_float(static_cast<int>(vertex >> 32)));
+            const V3 Ln = fma3(a, bb, L);
+            sh_L = make_float4(Ln.x, Ln.y, Ln.z, __int_as_float(static_cast<int>(vertex)));
             shadow = shadow_contributes(a, bb, L) || (p.rec && (bb.x != 0.f || bb.y != 0.f || bb.z != 0.f));
           }
           const float u_lobe = smp.next(), ubx = smp.next(), uby = smp.next();
@@ -456,7 +451,8 @@ __global__ void __launch_bounds__(128) k_wf_shade(const WfParams* __restrict__ p
           if (bs.pdf == 0.f) {
             done = true;
           } else {
-            const V3 nd = to_world(it.f, bs.wi);
+            nd = to_world(it.f, bs.wi);
+            pdf_next = bs.pdf;
             beta = scale(__frcp_rn(bs.pdf), mul(beta, bs.f));
             bool alive = true;
             if (depth >= p.rr_depth) {
@@ -466,42 +462,40 @@ __global__ void __launch_bounds__(128) k_wf_shade(const WfParams* __restrict__ p
             }
             if (alive && depth + 1 < p.max_depth) {
               cont = true;
-              p.ray[2 * slot] = make_float4(it.p.x, it.p.y, it.p.z, 0.f);
-              p.ray[2 * slot + 1] = make_float4(nd.x, nd.y, nd.z, bs.pdf);
-              if (p.sort) p.slot_key[slot] = ray_key(p, it.p, nd);
-              p.bl[2 * slot] = make_float4(beta.x, beta.y, beta.z, 0.f);
-              m.y = depth + 1;
             } else {
               done = true;
             }
           }
         }
         }
-        p.bl[2 * slot + 1] = make_float4(L.x, L.y, L.z, 0.f);
-        m.z = static_cast<int>(smp.state);
+        rec[5] = make_float4(L.x, L.y, L.z, 0.f);
+        if (cont) {
+          rec[0] = make_float4(it.p.x, it.p.y, it.p.z, 0.f);
+          rec[1] = make_float4(nd.x, nd.y, nd.z, pdf_next);
+          rec[4] = make_float4(beta.x, beta.y, beta.z, 0.f);
+          rec[6] = make_float4(m.x, __int_as_float(depth + 1), __uint_as_float(smp.state), 0.f);
+          key = ray_key(p, it.p, nd);
+        }
       }
-      if (done) m.w = kStatusDone;
-      p.meta[slot] = m;
     }
-    int si = warp_append(&p.counters[kCntShadow], shadow);
-    if (shadow && si >= p.pool) {
-      flag_error(s, BN_DEVERR_QUEUE_OVERFLOW);
-      shadow = false;
-    }
+    const int si = push(p, &p.counters[kCntShadow], &shadow);
+    int shadow_key = 0;
     if (shadow) {
       float4* r = p.shadow + 4LL * si;
-      r[0] = sh_o; r[1] = sh_d; r[2] = sh_a; r[3] = sh_b;
+      r[0] = sh_o; r[1] = sh_d; r[2] = sh_L;
+      shadow_key = ray_key(p, mk(sh_o.x, sh_o.y, sh_o.z), mk(sh_d.x, sh_d.y, sh_d.z));
+      p.sh_key[si] = shadow_key;
     }
-    if (p.sort_shadow) {
-      const int key = shadow ? ray_key(p, mk(sh_o.x, sh_o.y, sh_o.z), mk(sh_d.x, sh_d.y, sh_d.z)) : 0;
-      if (shadow) p.sh_key[si] = key;
-      hist_add(p.hist, key, shadow);
+    hist_add(p.hist + kSortBins, shadow_key, shadow);
+    // the paths that go on are the next iteration's ray queue
+    const int qi = push(p, &p.counters[kCntActiveNext], &cont);
+    if (cont) {
+      p.q_active[qi] = slot;
+      p.q_key[qi] = key;
     }
-    const unsigned cm = __ballot_sync(0xffffffffu, cont), dm = __ballot_sync(0xffffffffu, done);
-    if ((threadIdx.x & 31) == 0) {
-      if (cm) atomicAdd(&p.counters[kCntCont], __popc(cm));
-      if (dm) atomicAdd(&p.counters[kCntDone], __popc(dm));
-    }
+    hist_add(p.hist, key, cont);
+    const int di = push(p, &p.counters[kCntDone], &done);
+    if (done) p.q_done[di] = slot;
   }
 }
 
@@ -517,22 +511,19 @@ __global__ void __launch_bounds__(128, kShadowBlocks) k_wf_shadow(const WfParams
   TraceCounters tc{0, 0, 0};
   unsigned long long nrays = 0;  // rays this lane walked (counting walks)
   int rec = -1;
-  bool have = false, pending = false;
+  bool have = false;
   for (;;) {
-    if (__popc(__ballot_sync(__activemask(), have)) <= refill_below) {
-      if (pending) {
-        pending = false;
+    // (a walk can end at init, its root box missed)
+    TravVote vote(__activemask(), have, tr.mode);
+    if (vote.walking() <= refill_below) {
+      if (have && tr.mode == kTravDone) {
+        have = false;
         if (!tr.found) {
           const float4* r = p.shadow + 4LL * rec;
           const int slot = __float_as_int(r[1].w);
-          const float4 a = r[2], b = r[3];
-          float4 L = p.bl[2 * slot + 1];
-          L.x = fmaf(a.x, b.x, L.x);
-          L.y = fmaf(a.y, b.y, L.y);
-          L.z = fmaf(a.z, b.z, L.z);
-          p.bl[2 * slot + 1] = L;
-          if (p.lit)
-            p.lit[static_cast<long long>(__float_as_uint(a.w)) | (static_cast<long long>(__float_as_int(b.w)) << 32)] = 1;
+          const float4 Ln = r[2];
+          p.slot[8LL * slot + 5] = make_float4(Ln.x, Ln.y, Ln.z, 0.f);
+          if (p.lit) p.lit[__float_as_int(Ln.w)] = 1;
         }
       }
       const int qi = fetch_next(&p.counters[kCntFetchShadow], !have);
@@ -548,12 +539,9 @@ __global__ void __launch_bounds__(128, kShadowBlocks) k_wf_shadow(const WfParams
         have = true;
         ++nrays;
       }
+      vote = TravVote(__activemask(), have, tr.mode);
     }
-    const bool go = trav_vote(have, tr.mode);
-    if (have && go && (tr.mode == kTravDone || trav_step<kAnyHit, kWT, kWalk, kWfTris, kWfInstRun>(tr, p.scene, stk, &tc))) {
-      have = false;
-      pending = true;
-    }
+    if (have && tr.mode == vote.pick()) trav_step<kAnyHit, kWT, kWalk, kWfTris, kWfInstRun>(tr, p.scene, stk, &tc);
   }
   if (kWalk == kWalkCount) add_trace_counts(p.trace_counters, nrays, tc);
 }
@@ -586,15 +574,16 @@ __device__ __forceinline__ unsigned block_exclusive_scan(unsigned v, unsigned* t
   return x - v + (wid ? warp_sum[wid - 1] : 0u);
 }
 
-__global__ void __launch_bounds__(1024) k_wf_sort_tiles(const WfParams* __restrict__ pp) {
+__global__ void __launch_bounds__(1024) k_wf_sort_tiles(const WfParams* __restrict__ pp, int shadow_queue) {
   const WfParams& p = *pp;
   unsigned total;
-  block_exclusive_scan(p.hist[blockIdx.x * 1024 + threadIdx.x], &total);
+  block_exclusive_scan(p.hist[shadow_queue * kSortBins + blockIdx.x * 1024 + threadIdx.x], &total);
   if (threadIdx.x == 0) p.off[kSortBins + blockIdx.x] = total;  // tile sums after the offsets
 }
 
-__global__ void __launch_bounds__(1024) k_wf_sort_scan(const WfParams* __restrict__ pp) {
+__global__ void __launch_bounds__(1024) k_wf_sort_scan(const WfParams* __restrict__ pp, int shadow_queue) {
   const WfParams& p = *pp;
+  unsigned* hist = p.hist + shadow_queue * kSortBins;
   __shared__ unsigned tile_base;
   if (threadIdx.x < 32) {
     unsigned b = 0;
@@ -603,11 +592,11 @@ __global__ void __launch_bounds__(1024) k_wf_sort_scan(const WfParams* __restric
     if (threadIdx.x == 0) tile_base = b;
   }
   const int i = blockIdx.x * 1024 + threadIdx.x;
-  const unsigned c = p.hist[i];
+  const unsigned c = hist[i];
   unsigned total;
   const unsigned x = block_exclusive_scan(c, &total);  // its barriers also publish tile_base
   p.off[i] = tile_base + x;
-  p.hist[i] = 0u;
+  hist[i] = 0u;
 }
 
 // counting sort, step 2: every queue entry to its bucket (order within a bucket is arbitrary;
@@ -637,25 +626,20 @@ __global__ void k_wf_control(WfParams* pp, int use_graph) {
   int* c = p.counters;
   const bool more_work = *p.work_next < static_cast<unsigned long long>(p.total_paths - p.first_path);
   // PSSMLT chains: the chain regen counted the chains that are not finished into kCntDone
-  bool again = p.mlt ? c[kCntDone] > 0 : (c[kCntCont] > 0 || c[kCntDone] > 0 || more_work);
+  bool again = p.mlt ? c[kCntDone] > 0 : (c[kCntActiveNext] > 0 || c[kCntDone] > 0 || more_work);
   const int iter = ++c[kCntIter];
   if (again && iter >= p.max_iters) {
     atomicOr(p.scene.error_word, BN_DEVERR_WATCHDOG);
     again = false;
   }
-  if (p.mlt) {
-    // the chains' queues were filled this iteration for the next one
-    c[kCntActive] = c[kCntActiveNext];
-    c[kCntShadow] = c[kCntShadowNext];
-    c[kCntActiveNext] = 0;
-    c[kCntShadowNext] = 0;
-  } else {
-    c[kCntActive] = 0;
-    c[kCntShadow] = 0;
-  }
+  // the queues filled this iteration for the next one
+  c[kCntActive] = c[kCntActiveNext];
+  c[kCntActiveNext] = 0;
+  c[kCntShadow] = p.mlt ? c[kCntShadowNext] : 0;
+  c[kCntShadowNext] = 0;
+  c[kCntRetire] = c[kCntDone];
   c[kCntFetchRay] = 0;
   c[kCntFetchShadow] = 0;
-  c[kCntCont] = 0;
   c[kCntDone] = 0;
   for (int b = 0; b < kNumBins; ++b) c[kCntBin0 + b] = 0;
   c[kCntAgain] = again ? 1 : 0;
@@ -677,8 +661,8 @@ cudaError_t wf_launch_iteration(WfParams* dparams, const WfLaunch& l, bool use_g
                                 const WfFork* fk) {
   auto sort = [&](int shadow_queue) {
     if (!l.sort || (shadow_queue && !l.sort_shadow)) return;
-    k_wf_sort_tiles<<<l.sort_tiles, 1024, 0, st>>>(dparams);
-    k_wf_sort_scan<<<l.sort_tiles, 1024, 0, st>>>(dparams);
+    k_wf_sort_tiles<<<l.sort_tiles, 1024, 0, st>>>(dparams, shadow_queue);
+    k_wf_sort_scan<<<l.sort_tiles, 1024, 0, st>>>(dparams, shadow_queue);
     k_wf_sort_scatter<<<l.grid_scatter, 256, 0, st>>>(dparams, shadow_queue);
   };
   cudaError_t e = cudaSuccess;

@@ -25,15 +25,15 @@ inline int sort_key_bits(long long pool) {
 enum : int {
   kCntActive = 0,   // ray-queue length
   kCntShadow = 1,   // shadow-queue length
-  kCntCont = 2,     // paths continuing after shade
-  kCntDone = 3,     // paths that ended this iteration (retired by the next regen)
+  kCntRetire = 2,   // paths that ended in the last iteration: this regen retires them
+  kCntDone = 3,     // paths that ended this iteration; PSSMLT: chains not finished
   kCntIter = 4,     // iterations run
   kCntAgain = 5,    // last control decision (host-driven loop)
   kCntFetchRay = 6, // dynamic-fetch cursors of the extend and shadow kernels
   kCntFetchShadow = 7,
   kCntBin0 = 8,     // 8..13: per-bin hit counts
-  // PSSMLT chains: the queues filled in one iteration and traced in the next (k_wf_control moves
-  // them into kCntActive / kCntShadow)
+  // queues filled in one iteration and traced in the next (k_wf_control moves them into kCntActive /
+  // kCntShadow; the shadow one only of PSSMLT chains)
   kCntShadowNext = 14,
   kCntActiveNext = 15,
   kCntSize = 16
@@ -69,28 +69,29 @@ struct WfParams {
   long long first_path;         // path ids [first_path, total_paths)
   long long total_paths;
   long long n_pixels;
-  // per slot
-  // per slot, 32-byte records so that a slot's part of each is one DRAM sector
-  float4* ray;                  // 2 per slot: (o, -), (d, pdf of the last BSDF sample)
-  float4* bl;                   // 2 per slot: (beta, -), (L, -)
-  float4* hit;                  // 2 per slot: (t, u, v, instance | -1 as int bits),
-                                //             (triangle or sphere root as int bits, -, -, -)
-  int4* meta;                   // (film pixel, or path - first_path with path_L; depth, sampler state, status)
+  // Per slot one 128-byte record of 8 float4: (o, -), (d, pdf of the last BSDF sample), (t, u, v,
+  // instance | -1), (triangle or sphere root, -, -, -), (beta, -), (L, -), (film pixel, or path -
+  // first_path with path_L; depth, sampler state, -), unused.  The queues visit slots in no order of
+  // theirs, and DRAM reads 64 bytes at a time: the ray and its hit share one such half, what shading
+  // updates the other.
+  float4* slot;
   // queues
   int* q_active;                // pool entries
   int* q_bins;                  // kNumBins x pool entries
+  int* q_done;                  // slots whose path has ended
   // spatial sort of both ray queues (counting sort by key, when sort != 0)
   int sort, sort_shadow;
   float4 key_lo, key_scale;     // origin cell = (o - key_lo) * key_scale, in [0, 2^b) x [0, 8) x [0, 2^b)
   int key_bits;                 // b (sort_key_bits): the keys span 2^(2b + 6) bins
-  int* slot_key;                // per slot: key of the ray the slot holds (written by shade)
   int* q_key;                   // per ray-queue entry: its key
   int* q_ray;                   // the ray queue in key order (read by extend)
   int* sh_key;                  // per shadow record: its key
   int* q_shadow;                // shadow-record indices in key order (read by shadow)
-  unsigned* hist;               // kSortBins counts; zero between uses (the scan clears it)
+  unsigned* hist;               // kSortBins counts of the ray queue's keys, then as many of the shadow
+                                // queue's; zero between uses (the scan clears them)
   unsigned* off;                // kSortBins bucket offsets, then kSortBins / 1024 tile sums
-  float4* shadow;               // 4 float4 per record: (o, tmax), (d, owner), a, b
+  float4* shadow;               // 4 float4 per record: (o, tmax), (d, slot), (L if the ray gets through,
+                                // vertex in lit), -
   int* counters;                // kCntSize ints
   void* trace_counters;         // DevCounters (rays, nodes, triangles, instances) of counting walks
   unsigned long long* work_next;
@@ -98,7 +99,7 @@ struct WfParams {
   float4* path_L;               // or, if not null, the radiance of path first_path + i at i
   // records of an ordered render's vertices, or null: (t, instance | -1, triangle or sphere root, -)
   // of path first_path + i's hit at depth k at k * n + i, n = total_paths - first_path, and 1 in lit
-  // where the vertex's shadow ray got through.  With them a shadow ray is also traced when only
+  // where the vertex's shadow ray got through (fewer than 2^31 vertices).  With them a shadow ray is also traced when only
   // the derivative of its term can be other than zero.
   float4* rec;
   unsigned char* lit;

@@ -178,7 +178,7 @@ enum bn_render_mode {
   BN_MODE_MEGAKERNEL = 0, /* each pixel's samples summed in order (the film is the     */
                           /* same on every run); one kernel of lanes that run whole   */
                           /* paths, from 1 M paths on the wavefront's queues (2 GB    */
-                          /* and 224 B per slot of device memory at most; without it, */
+                          /* and 240 B per slot of device memory at most; without it, */
                           /* the one kernel).  PSSMLT: a lane per chain               */
   BN_MODE_WAVEFRONT = 1   /* persistent queues compacted every bounce, many views per */
                           /* launch (PSSMLT: one path slot per chain, same decisions) */
@@ -219,7 +219,7 @@ typedef struct bn_render_desc {
   float eps_min, eps_max;    /* Kelemen s1, s2                                       */
   /* wavefront launch shape (0 = default) */
   int32_t block_size;        /* traversal blocks per SM cap                           */
-  int32_t queue_capacity;    /* path slots, 224 B of device memory each; by default   */
+  int32_t queue_capacity;    /* path slots, 240 B of device memory each; by default   */
                              /* one per path of the render, at most 64 M               */
   int32_t pad_;
 } bn_render_desc;
