@@ -84,6 +84,20 @@ def test_wavefront_sort_key_widths(ctx, pool):
         assert_same_image(w, m)
 
 
+@pytest.mark.parametrize("w,h,spp,pool", [(1, 1, 1, 0), (31, 1, 1, 0), (33, 1, 1, 0), (127, 3, 1, 0), (129, 5, 3, 1024),
+                                          (513, 151, 4, 0)])
+def test_wavefront_ragged_record_tiles(ctx, w, h, spp, pool):
+    """Shading moves 32 path records of a warp at a time, two tiles in turn: path counts below, at and
+    past a tile, tiles whose bins leave a remainder, and queues longer than one pass of the grid."""
+    b = Bundle.generate("materials", 1)
+    ctx.upload(b)
+    v = b.views[0]
+    v.width, v.height = w, h
+    mega = render(ctx, b, [v], spp, capi.BN_MODE_MEGAKERNEL)[0]
+    wave = render(ctx, b, [v], spp, capi.BN_MODE_WAVEFRONT, pool=pool)[0]
+    assert_same_image(wave, mega)
+
+
 def test_wavefront_many_views_one_launch(ctx):
     b = Bundle.generate("instances", 1)
     ctx.upload(b)
