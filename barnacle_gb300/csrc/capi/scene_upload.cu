@@ -69,7 +69,9 @@ struct MeshPrep {
 struct Collapse {
   const std::vector<bn_bvh_node>& b;
   std::vector<float4>& out;
+  const int leaf_bits;
   bool nested = true;
+  bool codes = true;  // every leaf's items fit its code
 
   static bool inside(const bn_bvh_node& in, const bn_bvh_node& outer) {
     for (int a = 0; a < 3; ++a)
@@ -97,7 +99,6 @@ struct Collapse {
     const float nan = std::numeric_limits<float>::quiet_NaN();
     float box[6][4];
     int ref[4] = {0, 0, 0, 0};
-    unsigned counts = 0, leaf_mask = 0;
     for (int s = 0; s < 4; ++s) {
       if (slot[s] < 0) {
         for (int r = 0; r < 6; ++r) box[r][s] = nan;
@@ -109,9 +110,9 @@ struct Collapse {
         box[3 + a][s] = n.bounds_max[a];
       }
       if (n.is_leaf) {
-        ref[s] = n.right_or_offset;
-        counts |= static_cast<unsigned>(static_cast<uint8_t>(n.count)) << (8 * s);
-        leaf_mask |= 1u << s;
+        const int last = static_cast<uint8_t>(n.count) - 1;
+        codes = codes && last >= 0 && last < (1 << leaf_bits);
+        ref[s] = static_cast<int>(~((static_cast<unsigned>(n.right_or_offset) << leaf_bits) | static_cast<unsigned>(last)));
       } else {
         ref[s] = emit(slot[s]);  // grows out: the record is written by index below
       }
@@ -131,11 +132,7 @@ struct Collapse {
       const unsigned v0 = pa + (fa ? 0 : 1), v1 = pa + (fa ? 1 : 0), v2 = pb + (fb ? 0 : 1), v3 = pb + (fb ? 1 : 0);
       orders[oct >> 2] |= (v0 | (v1 << 2) | (v2 << 4) | (v3 << 6)) << (8 * (oct & 3));
     }
-    const int meta[4] = {static_cast<int>(counts),
-                         static_cast<int>(leaf_mask | (static_cast<unsigned>(axis[0] & 3) << 4) |
-                                          (static_cast<unsigned>(axis[1] & 3) << 6) |
-                                          (static_cast<unsigned>(axis[2] & 3) << 8)),
-                         static_cast<int>(orders[0]), static_cast<int>(orders[1])};
+    const int meta[4] = {static_cast<int>(orders[0]), static_cast<int>(orders[1]), 0, 0};
     std::memcpy(&mt, meta, 16);
     r[6] = rf;
     r[7] = mt;
@@ -321,7 +318,8 @@ int device_blases(bn_context* ctx, const bn_scene_desc* d, const std::vector<int
 
 // The wide records of the device's BLASes behind the *n_records of the host, in ctx->nodes4.
 int device_records(bn_context* ctx, const std::vector<int>& meshes, const std::vector<int32_t>& mesh_base, int blas0,
-                   int host_nodes, int blas_nodes, std::vector<MeshPrep>* mp, size_t* n_records, bool* nested) {
+                   int host_nodes, int blas_nodes, int leaf_bits, std::vector<MeshPrep>* mp, size_t* n_records,
+                   bool* nested, bool* codes) {
   cudaStream_t st = ctx->stream;
   bnc::BvhWork& k = ctx->bvh;
   const int nm = static_cast<int>(meshes.size());
@@ -331,6 +329,7 @@ int device_records(bn_context* ctx, const std::vector<int>& meshes, const std::v
   w.n = blas_nodes - host_nodes;
   w.odd = k.scene_odd.as<unsigned char>();
   w.n_meshes = nm;
+  w.leaf_bits = leaf_bits;
   const int blocks = (w.n + 1023) / 1024;
   cudaError_t e;
   // rank | block sums | flag | roots | mesh bases
@@ -360,7 +359,8 @@ int device_records(bn_context* ctx, const std::vector<int>& meshes, const std::v
       (e = cudaMemcpyAsync(back.data(), w.flags, back.size() * sizeof(int), cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
       (e = cudaStreamSynchronize(st)) != cudaSuccess)
     return ctx->cuda_fail(e, "wide records");
-  if (back[0]) *nested = false;
+  if (back[0] & 1) *nested = false;
+  if (back[0] & 2) *codes = false;
   for (int j = 0; j < nm; ++j) (*mp)[meshes[j]].node4_root = back[1 + j];
   *n_records += count;
   return BN_OK;
@@ -504,30 +504,42 @@ extern "C" int bn_scene_upload(bn_context* ctx, const bn_scene_desc* d) {
   // scene is walked wide: asked for, or automatically for scenes of 1,024+ nodes
   if (d->bvh_width != BN_BVH_AUTO && d->bvh_width != BN_BVH_BINARY && d->bvh_width != BN_BVH_WIDE)
     return ctx->fail(BN_ERR_INVALID_ARG, "bvh_width must be 0 (auto), 2 or 4");
-  const bool scene_wide =
+  bool scene_wide =
       d->bvh_width == BN_BVH_WIDE || (d->bvh_width == BN_BVH_AUTO && n_tlas + blas_nodes >= 1024);
   std::vector<float4> nodes4;
-  bool nested = true;
+  bool nested = true, codes = true;
+  int most = ni;  // items of the largest BVH
+  for (int i = 0; i < d->n_meshes; ++i) most = std::max(most, d->meshes[i].n_triangles);
+  const int leaf_bits = bn::leaf_count_bits(most);
   if (scene_wide && !tlas[0].is_leaf) {
-    Collapse c{tlas, nodes4};
+    Collapse c{tlas, nodes4, leaf_bits};
     c.emit(0);
     nested = nested && c.nested;
+    codes = codes && c.codes;
   }
   for (int i = 0; i < d->n_meshes; ++i) {
     if (!scene_wide || mp[i].on_device || mp[i].nodes[0].is_leaf) continue;
-    Collapse c{mp[i].nodes, nodes4};
+    Collapse c{mp[i].nodes, nodes4, leaf_bits};
     mp[i].node4_root = c.emit(0);
     nested = nested && c.nested;
+    codes = codes && c.codes;
   }
   size_t n_records = nodes4.size() / 8;
   if (scene_wide && !device_meshes.empty() && nested) {
     const int rc = device_records(ctx, device_meshes, mesh_base, blas0, static_cast<int>(host_nodes),
-                                  static_cast<int>(blas_nodes), &mp, &n_records, &nested);
+                                  static_cast<int>(blas_nodes), leaf_bits, &mp, &n_records, &nested, &codes);
     if (rc) return rc;
   }
   if (!nested) return ctx->fail(BN_ERR_INVALID_ARG, "non-finite triangle or instance bounds");
-  if (n_records >= (size_t{1} << 29))  // a stacked leaf slot is -1 - (4 * record + slot)
+  if (n_records >= (size_t{1} << 29))
     return ctx->fail(BN_ERR_UNSUPPORTED, "scene too large for the wide BVH records");
+  if (!codes) {
+    // a BVH of over 16 M items with a leaf, at the depth limit, of more items than its code can say
+    scene_wide = false;
+    for (MeshPrep& m : mp) m.node4_root = -1;
+    nodes4.clear();
+    n_records = 0;
+  }
   if (n_records == 0) nodes4.resize(8);  // keep the buffer non-null
 
   std::vector<bn::DevInstance> dinst(ni);
@@ -670,6 +682,7 @@ extern "C" int bn_scene_upload(bn_context* ctx, const bn_scene_desc* d) {
   s.n_nodes = static_cast<int>(blas0 + blas_nodes);
   s.n_nodes4 = static_cast<int>(std::max<size_t>(n_records, 1));
   s.wide = scene_wide ? 1 : 0;
+  s.leaf_bits = leaf_bits;
   s.n_tris = static_cast<int>(n_tris);
   s.n_light_inst = static_cast<int>(light_inst.size());
   s.n_tri_lights = static_cast<int>(tl.size());

@@ -136,13 +136,19 @@ struct SharedStack {
   }
 };
 
+// a leaf slot's code in a wide record (dev_types.cuh): its items without reading the record again
+__device__ __forceinline__ void trav_enter_code(Trav& tr, const DevScene& s, int code) {
+  const int v = ~code;
+  trav_enter_leaf(tr, v >> s.leaf_bits, (v & ((1 << s.leaf_bits) - 1)) + 1);
+}
+
 __device__ __forceinline__ const float4* node4_at(const DevScene& s, int i) {
   return s.nodes4 + 8 * static_cast<size_t>(i);
 }
 
 // the next stacked node still within reach; an exhausted BLAS returns to the instances of its
 // TLAS leaf, an exhausted TLAS ends the walk.  Binary entries are node indices within the level;
-// wide entries are record indices (>= 0) or -1 - (4 * record + slot) for a leaf slot.
+// wide entries are a record's slots: record indices (>= 0) or a leaf's code (< 0).
 template <bool kWide, class Stack>
 __device__ __forceinline__ void trav_pop(Trav& tr, const DevScene& s, const Stack& stk) {
   for (;;) {
@@ -159,9 +165,7 @@ __device__ __forceinline__ void trav_pop(Trav& tr, const DevScene& s, const Stac
           tr.cur = c;
           tr.mode = kTravNode;
         } else {
-          const int k = -1 - c, sl = k & 3;
-          const int* rec = reinterpret_cast<const int*>(node4_at(s, k >> 2) + 6);
-          trav_enter_leaf(tr, __ldg(rec + sl), (__ldg(rec + 4) >> (8 * sl)) & 0xff);
+          trav_enter_code(tr, s, c);
         }
         return;
       }
@@ -210,17 +214,12 @@ __device__ __forceinline__ void trav_init(Trav& tr, const DevScene& s, const Ray
   }
 }
 
-__device__ __forceinline__ float sel4(float a, float b, float c, float d, int i) {
-  return (i & 2) ? ((i & 1) ? d : c) : ((i & 1) ? b : a);
-}
-__device__ __forceinline__ int sel4(int a, int b, int c, int d, int i) {
-  return (i & 2) ? ((i & 1) ? d : c) : ((i & 1) ? b : a);
-}
-
 // one wide step: the four slot boxes of record tr.cur; returns kStepPop when none is entered,
 // kStepOverflow when the stack is full.  The slots are put in visit order by three conditional swaps
 // (with the triangle test before a leaf's box test this took 6 instanced views of 4 spp from 95.3 to
 // 90.8 ms; selecting each slot by its number cost twice the instructions)
+// A slot is stacked as the record says it (a record's index or a leaf's code): with leaves stacked as
+// (record, slot), whose items the pop had to read, six instanced views took 89.2 ms, now 87.0.
 enum : int { kStepOk = 0, kStepPop = 1, kStepOverflow = 2 };
 template <class Stack>
 __device__ __forceinline__ int trav_node4(Trav& tr, const DevScene& s, Stack& stk) {
@@ -230,25 +229,23 @@ __device__ __forceinline__ int trav_node4(Trav& tr, const DevScene& s, Stack& st
   const float4 lx = __ldg(q), ly = __ldg(q + 1), lz = __ldg(q + 2);
   const float4 hx = __ldg(q + 3), hy = __ldg(q + 4), hz = __ldg(q + 5);
   const int4 ref = __ldg(reinterpret_cast<const int4*>(q + 6));
-  const int4 meta = __ldg(reinterpret_cast<const int4*>(q + 7));
+  const int2 orders = __ldg(reinterpret_cast<const int2*>(q + 7));
   float e0, e1, e2, e3;
   const bool h0 = box_hit_t(mk(lx.x, ly.x, lz.x), mk(hx.x, hy.x, hz.x), r, inv, tr.t, &e0);
   const bool h1 = box_hit_t(mk(lx.y, ly.y, lz.y), mk(hx.y, hy.y, hz.y), r, inv, tr.t, &e1);
   const bool h2 = box_hit_t(mk(lx.z, ly.z, lz.z), mk(hx.z, hy.z, hz.z), r, inv, tr.t, &e2);
   const bool h3 = box_hit_t(mk(lx.w, ly.w, lz.w), mk(hx.w, hy.w, hz.w), r, inv, tr.t, &e3);
   if (!(h0 | h1 | h2 | h3)) return kStepPop;
-  // what a stack entry says of each slot: a record, -1 - (4 * record + slot) for a leaf (records
-  // number less than 2^29), or nothing entered
+  // what a stack entry says of each slot: a record, a leaf's code, or nothing entered (no leaf has
+  // that code)
   constexpr int kNone = static_cast<int>(0x80000000u);
-  const int m = meta.y, nb = ~(4 * tr.cur);
-  const int c0 = !h0 ? kNone : ((m & 1) ? nb : ref.x), c1 = !h1 ? kNone : ((m & 2) ? nb - 1 : ref.y);
-  const int c2 = !h2 ? kNone : ((m & 4) ? nb - 2 : ref.z), c3 = !h3 ? kNone : ((m & 8) ? nb - 3 : ref.w);
+  const int c0 = h0 ? ref.x : kNone, c1 = h1 ? ref.y : kNone, c2 = h2 ? ref.z : kNone, c3 = h3 ? ref.w : kNone;
   // the binary walk's order (the near child's slots, then the far child's, each pair ordered by
   // that child's own split axis: BVH.fs near-child rule at both levels) depends on the ray only
   // through its octant; the upload stored the slot order of each octant, 8 bits per octant: bit 1
   // swaps the pairs, bits 0 and 4 the slots of the pair then first and second
   const int oct = tr.level ? tr.ooct : tr.woct;
-  const unsigned order = static_cast<unsigned>(oct & 4 ? meta.w : meta.z) >> (8 * (oct & 3));
+  const unsigned order = static_cast<unsigned>(oct & 4 ? orders.y : orders.x) >> (8 * (oct & 3));
   const bool sp = order & 2u, sa = order & 1u, sb = order & 16u;
   const int a0 = sp ? c2 : c0, a1 = sp ? c3 : c1, b0 = sp ? c0 : c2, b1 = sp ? c1 : c3;
   const float ea0 = sp ? e2 : e0, ea1 = sp ? e3 : e1, eb0 = sp ? e0 : e2, eb1 = sp ? e1 : e3;
@@ -261,12 +258,8 @@ __device__ __forceinline__ int trav_node4(Trav& tr, const DevScene& s, Stack& st
   if (p2 && (p0 | p1)) stk.put(tr.sp++, v2, t2);
   if (p1 && p0) stk.put(tr.sp++, v1, t1);
   const int next = p0 ? v0 : (p1 ? v1 : (p2 ? v2 : v3));
-  if (next >= 0) {
-    tr.cur = next;
-  } else {
-    const int sl = (-1 - next) & 3;
-    trav_enter_leaf(tr, sel4(ref.x, ref.y, ref.z, ref.w, sl), (meta.x >> (8 * sl)) & 0xff);
-  }
+  if (next >= 0) tr.cur = next;
+  else trav_enter_code(tr, s, next);
   return kStepOk;
 }
 

@@ -9,11 +9,11 @@
 //             the two binary levels below it in one record.  Slots 0-1 hold the left child's
 //             children (or the left child itself, slot 1 unused, when it is a leaf), slots 2-3
 //             the right child's.  (lo.x[4], lo.y[4], lo.z[4], hi.x[4], hi.y[4], hi.z[4]) slot
-//             boxes, int4 ref (node4 index of an interior slot, first item of a leaf slot),
-//             int4 meta (x: leaf item count, 8 bits per slot; y: leaf mask bits 0-3, split axis
-//             of the node << 4, of its left child << 6, of its right child << 8; z, w: the slot
-//             visit order for each of the 8 ray octants, 8 bits = 4 x 2-bit slots per octant,
-//             octants 0-3 in z, 4-7 in w).  Unused slots
+//             boxes, int4 ref (node4 index of an interior slot, or a leaf's code
+//             ~(first item << leaf_bits | items - 1)), int2 orders (the slot visit order for each
+//             of the 8 ray octants, 8 bits = 4 x 2-bit slots per octant, octants 0-3 in x, 4-7 in
+//             y), 8 bytes of nothing.  A leaf's code is what the walk stacks, so a leaf taken from
+//             the stack is entered without reading its record again.  Unused slots
 //             have NaN boxes, which no ray enters.  TLAS records first (root at 0 when the TLAS
 //             root is interior), then every BLAS at DevInstance::node4_root.  Built when the
 //             scene is walked wide (DevScene::wide).
@@ -109,6 +109,7 @@ struct DevScene {
   int n_nodes;
   int n_nodes4;
   int wide;                               // walked through nodes4 (kWalkWide kernels)
+  int leaf_bits;                          // bits of a leaf's item count in nodes4 (leaf_count_bits)
   int n_tris;
   int n_light_inst;
   int n_tri_lights;
@@ -117,5 +118,13 @@ struct DevScene {
   int stack_cap;                          // usable stack entries (kStackSize; lower for tests)
   unsigned int* error_word;               // BN_DEVERR_* bits
 };
+
+// The bits that a leaf's code leaves for its items - 1 when items are numbered below n: 7 (leaves of
+// 128; a node's count ends at 127) up to 16 M items in a mesh or the TLAS, fewer beyond.
+__host__ __device__ inline int leaf_count_bits(long long n) {
+  int bits = 7;
+  while (bits > 0 && n >= (1LL << (31 - bits))) --bits;
+  return bits;
+}
 
 }  // namespace bn

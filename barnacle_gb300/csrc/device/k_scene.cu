@@ -161,7 +161,6 @@ __global__ void __launch_bounds__(128) k_wide_fill(WideParams p) {
   if (!nested) atomicOr(p.flags, 1);
   float box[6][4];
   int ref[4] = {0, 0, 0, 0};
-  unsigned counts = 0, leaf_mask = 0;
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     if (slot[k] < 0) {
@@ -175,9 +174,9 @@ __global__ void __launch_bounds__(128) k_wide_fill(WideParams p) {
       box[3 + a][k] = s[k].hi[a];
     }
     if (s[k].leaf()) {
-      ref[k] = s[k].link;
-      counts |= ((s[k].bytes >> 16) & 0xffu) << (8 * k);
-      leaf_mask |= 1u << k;
+      const int last = static_cast<int>((s[k].bytes >> 16) & 0xffu) - 1;
+      if (last < 0 || last >= (1 << p.leaf_bits)) atomicOr(p.flags, 2);
+      ref[k] = static_cast<int>(~((static_cast<unsigned>(s[k].link) << p.leaf_bits) | static_cast<unsigned>(last)));
     } else {
       ref[k] = record_of(p, slot[k] - p.base);
     }
@@ -197,10 +196,7 @@ __global__ void __launch_bounds__(128) k_wide_fill(WideParams p) {
 #pragma unroll
   for (int k = 0; k < 6; ++k) o[k] = make_float4(box[k][0], box[k][1], box[k][2], box[k][3]);
   o[6] = make_float4(__int_as_float(ref[0]), __int_as_float(ref[1]), __int_as_float(ref[2]), __int_as_float(ref[3]));
-  const unsigned axes = leaf_mask | (static_cast<unsigned>(axis[0] & 3) << 4) | (static_cast<unsigned>(axis[1] & 3) << 6) |
-                        (static_cast<unsigned>(axis[2] & 3) << 8);
-  o[7] = make_float4(__uint_as_float(counts), __uint_as_float(axes), __uint_as_float(orders[0]),
-                     __uint_as_float(orders[1]));
+  o[7] = make_float4(__uint_as_float(orders[0]), __uint_as_float(orders[1]), 0.f, 0.f);
 }
 
 unsigned blocks_for(long long n, int bs) { return static_cast<unsigned>((n + bs - 1) / bs); }

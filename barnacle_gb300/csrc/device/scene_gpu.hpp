@@ -23,9 +23,10 @@ struct WideParams {
   const unsigned char* odd;
   const int* mesh_base;
   int n_meshes;
+  int leaf_bits;    // leaf_count_bits of the largest BVH
   int* rank;        // n: records before the node in its block of 1,024 nodes
   int* sums;        // n / 1,024 + 2: records before each block, then their number
-  int* flags;       // 0: every box contains its children's; 1: some does not
+  int* flags;       // bit 0: some box does not contain its children's; bit 1: some leaf does not fit its code
   int* roots;       // n_meshes: record of the mesh's root, -1 where it is a leaf
   float4* records;  // 8 per record
   int first_record; // index of the first of them
