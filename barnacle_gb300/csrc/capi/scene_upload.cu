@@ -518,7 +518,10 @@ extern "C" int bn_scene_upload(bn_context* ctx, const bn_scene_desc* d) {
     codes = codes && c.codes;
   }
   for (int i = 0; i < d->n_meshes; ++i) {
-    if (!scene_wide || mp[i].on_device || mp[i].nodes[0].is_leaf) continue;
+    if (!scene_wide) continue;
+    const bn_bvh_node& root = mp[i].nodes[0];
+    if (root.is_leaf) codes = codes && root.count <= (1 << leaf_bits);  // entered by its code too
+    if (mp[i].on_device || root.is_leaf) continue;
     Collapse c{mp[i].nodes, nodes4, leaf_bits};
     mp[i].node4_root = c.emit(0);
     nested = nested && c.nested;

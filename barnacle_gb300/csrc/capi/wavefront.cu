@@ -155,6 +155,14 @@ int run(bn_context* ctx, WfState* w, const bn::DevScene& scene, const bn_render_
       w->exec = nullptr;
     }
   }
+  const bn::DevScene walk = bn::walk_scene(scene);
+  if (std::memcmp(&w->shape.walk, &walk, sizeof(walk)) != 0) {  // part of the captured launches
+    w->shape.walk = walk;
+    if (w->exec) {
+      cudaGraphExecDestroy(w->exec);
+      w->exec = nullptr;
+    }
+  }
   bn::WfParams p{};
   p.scene = scene;
   p.views = ctx->views.as<bn::DevView>();
@@ -165,10 +173,6 @@ int run(bn_context* ctx, WfState* w, const bn::DevScene& scene, const bn_render_
   p.frame_id = d->frame_id;
   p.integrator = d->integrator;
   p.pool = pool;
-  // lanes of 32 still walking when a traversal warp refills (12 / 16 / 20 / 24 measured 192.9 /
-  // 193.7 / 191.6 / 187.8 M paths/s on the instanced workload, when the mode vote came in)
-  p.refill_extend = 16;
-  p.refill_shadow = 16;
   p.first_path = first;
   p.total_paths = end;
   p.n_pixels = n_pixels;
@@ -286,6 +290,7 @@ int run_mlt(bn_context* ctx, WfState* w, const bn_render_desc* d, const bn::MltP
       w->exec = nullptr;
     }
   }
+  w->shape.walk = bn::walk_scene(ctx->scene);
   bn::WfParams p{};
   p.scene = ctx->scene;
   p.views = mp.view;
@@ -296,8 +301,6 @@ int run_mlt(bn_context* ctx, WfState* w, const bn_render_desc* d, const bn::MltP
   p.frame_id = d->frame_id;
   p.integrator = BN_INTEGRATOR_PSSMLT;
   p.pool = pool;
-  p.refill_extend = 16;
-  p.refill_shadow = 16;
   p.total_paths = 0;
   p.n_pixels = 0;
   // a mutation's path takes at most max_depth iterations (at least one), and one more when its

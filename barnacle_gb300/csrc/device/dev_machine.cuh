@@ -81,8 +81,8 @@ __device__ __forceinline__ void path_machine(const DevScene& s, Task& task, Smp&
       V3 org = mk(0.f, 0.f, 0.f), dir = org;  // the next walk
       float tmax = CUDART_INF_F;
       if (phase == kLaneClosest) {
-        if constexpr (kRecord) task.hit(depth, tr.found, tr.hit);
-        if (!tr.found) {
+        if constexpr (kRecord) task.hit(depth, tr.found(), tr.hit());
+        if (!tr.found()) {
           over = true;
         } else {
           Bounce b;
@@ -93,7 +93,7 @@ __device__ __forceinline__ void path_machine(const DevScene& s, Task& task, Smp&
           ps.pdf_bsdf = pdf;
           ps.depth = depth;
           const int vertex = depth;
-          bounce_shade<kFixed7, kSimple>(s, ps, tr.hit, smp, max_depth, rr_depth, &b);
+          bounce_shade<kFixed7, kSimple>(s, ps, tr.hit(), smp, max_depth, rr_depth, &b);
           L = ps.L;
           beta = ps.beta;
           pdf = ps.pdf_bsdf;
@@ -113,7 +113,7 @@ __device__ __forceinline__ void path_machine(const DevScene& s, Task& task, Smp&
           }
         }
       } else if (phase == kLaneShadow) {
-        if (!tr.found) {
+        if (!tr.found()) {
           L = Ln;
           if constexpr (kRecord) task.lit();
         }

@@ -47,26 +47,47 @@ enum : int { kTravNode = 0, kTravTri = 1, kTravInst = 2, kTravDone = 3 };
 // is not > 0, as in BVH.fs)
 __device__ __forceinline__ int octant(V3 d) { return int(d.x > 0.f) | (int(d.y > 0.f) << 1) | (int(d.z > 0.f) << 2); }
 
+// A walk's state.  The traversal kernels hold it in 64 to 80 registers with everything else, so what
+// can be had from another field is not kept.
 struct Trav {
   Ray wr;            // world ray
   V3 winv;
-  int woct;          // octant of the world direction: bit a set when d[a] > 0
-  Ray orr;           // object-space ray of the instance being walked
+  Ray orr;           // the ray of the level: the object-space ray of the instance being walked, or wr
   V3 oinv;
-  int ooct;          // the same for the object-space direction
+  int ooct;          // octant of orr's direction: bit a set when d[a] > 0
   WtRay wt;
   float t;
-  NodeRec n;         // current interior node (kTravNode), its box already passed
-  int mode, level;   // level 0 = TLAS, 1 = BLAS
-  int cur, base;     // node index within the level, the level's base in nodes[]
-  int tri_base, inst;
-  int sp, blas_sp0;
-  int ii, ii_end;    // instances of the TLAS leaf being processed
-  int ti, ti_end;    // triangles of the BLAS leaf being processed
-  bool found;
+  NodeRec n;         // current interior node of the binary walk (kTravNode), its box already passed
+  int mode;
+  int cur, base;     // node or record index, in the wide walk also the code of the BLAS leaf being
+                     // processed; the level's base in nodes[] (binary walk)
+  int tri_base;
+  int sp, blas_sp0;  // blas_sp0: the stack below the BLAS being walked, -1 in the TLAS
+  int ii, ii_end;    // instances of the TLAS leaf being processed; the BLAS walked is ii - 1's
+  int ti, ti_end;    // triangles of the BLAS leaf being processed (binary walk)
   bool any;          // any-hit query (runtime choice, kAnyRuntime walks)
-  HitRec hit;
+  // the hit at t: barycentrics, instance (-1: none), triangle or ~root of a sphere
+  float hu, hv;
+  int hinst, hprim;
+
+  __device__ __forceinline__ bool found() const { return hinst >= 0; }
+  __device__ __forceinline__ HitRec hit() const {
+    HitRec h;
+    h.t = t; h.u = hu; h.v = hv;
+    h.inst = hinst;
+    h.tri = hprim < 0 ? 0 : hprim;
+    h.sphere_root = hprim < 0 ? ~hprim : 0;
+    return h;
+  }
 };
+
+// back to the TLAS with the world ray
+__device__ __forceinline__ void trav_world(Trav& tr) {
+  tr.orr = tr.wr;
+  tr.oinv = tr.winv;
+  tr.ooct = octant(tr.wr.d);
+  tr.blas_sp0 = -1;
+}
 
 // enter a node whose box passed: an interior node is walked, a leaf's items are iterated
 __device__ __forceinline__ void trav_enter(Trav& tr, int cur, const NodeRec& n) {
@@ -74,26 +95,13 @@ __device__ __forceinline__ void trav_enter(Trav& tr, int cur, const NodeRec& n) 
   if (!n.leaf) {
     tr.n = n;
     tr.mode = kTravNode;
-  } else if (tr.level == 0) {
+  } else if (tr.blas_sp0 < 0) {
     tr.ii = n.link;
     tr.ii_end = n.link + n.count;
     tr.mode = kTravInst;
   } else {
     tr.ti = n.link;
     tr.ti_end = n.link + n.count;
-    tr.mode = kTravTri;
-  }
-}
-
-// a leaf's item range: instances at the TLAS level, triangles at the BLAS level
-__device__ __forceinline__ void trav_enter_leaf(Trav& tr, int first, int count) {
-  if (tr.level == 0) {
-    tr.ii = first;
-    tr.ii_end = first + count;
-    tr.mode = kTravInst;
-  } else {
-    tr.ti = first;
-    tr.ti_end = first + count;
     tr.mode = kTravTri;
   }
 }
@@ -136,10 +144,22 @@ struct SharedStack {
   }
 };
 
-// a leaf slot's code in a wide record (dev_types.cuh): its items without reading the record again
+// a leaf by its code in a wide record (dev_types.cuh): instances in the TLAS, triangles in a BLAS
+__device__ __forceinline__ int leaf_code(const DevScene& s, int first, int count) {
+  return ~((first << s.leaf_bits) | (count - 1));
+}
+__device__ __forceinline__ void leaf_items(const DevScene& s, int code, int* first, int* end) {
+  *first = ~code >> s.leaf_bits;
+  *end = *first + (~code & ((1 << s.leaf_bits) - 1)) + 1;
+}
 __device__ __forceinline__ void trav_enter_code(Trav& tr, const DevScene& s, int code) {
-  const int v = ~code;
-  trav_enter_leaf(tr, v >> s.leaf_bits, (v & ((1 << s.leaf_bits) - 1)) + 1);
+  if (tr.blas_sp0 < 0) {
+    leaf_items(s, code, &tr.ii, &tr.ii_end);
+    tr.mode = kTravInst;
+  } else {
+    tr.cur = code;
+    tr.mode = kTravTri;
+  }
 }
 
 __device__ __forceinline__ const float4* node4_at(const DevScene& s, int i) {
@@ -152,7 +172,7 @@ __device__ __forceinline__ const float4* node4_at(const DevScene& s, int i) {
 template <bool kWide, class Stack>
 __device__ __forceinline__ void trav_pop(Trav& tr, const DevScene& s, const Stack& stk) {
   for (;;) {
-    const int bottom = tr.level ? tr.blas_sp0 : 0;
+    const int bottom = max(tr.blas_sp0, 0);
     while (tr.sp > bottom) {
       --tr.sp;
       int c;
@@ -170,9 +190,9 @@ __device__ __forceinline__ void trav_pop(Trav& tr, const DevScene& s, const Stac
         return;
       }
     }
-    if (tr.level == 1) {
-      tr.level = 0;
+    if (tr.blas_sp0 >= 0) {
       tr.base = 0;
+      trav_world(tr);
       if (tr.ii < tr.ii_end) {
         tr.mode = kTravInst;
         return;
@@ -191,16 +211,13 @@ template <int kWalk>
 __device__ __forceinline__ void trav_init(Trav& tr, const DevScene& s, const Ray& ray, float tmax, TraceCounters* cnt) {
   tr.wr = ray;
   tr.winv = inv_dir(ray.d);
-  tr.woct = octant(ray.d);
   tr.t = tmax;
-  tr.found = false;
-  tr.hit.inst = -1;
+  tr.hinst = -1;
   tr.sp = 0;
-  tr.blas_sp0 = 0;
-  tr.level = 0;
   tr.base = 0;
   tr.ii = tr.ii_end = 0;
   tr.ti = tr.ti_end = 0;
+  trav_world(tr);
   const NodeRec root = load_node(s.nodes, 0);
   if (kWalk == kWalkCount) cnt->nodes++;
   float te;
@@ -218,13 +235,11 @@ __device__ __forceinline__ void trav_init(Trav& tr, const DevScene& s, const Ray
 // kStepOverflow when the stack is full.  The slots are put in visit order by three conditional swaps
 // (with the triangle test before a leaf's box test this took 6 instanced views of 4 spp from 95.3 to
 // 90.8 ms; selecting each slot by its number cost twice the instructions)
-// A slot is stacked as the record says it (a record's index or a leaf's code): with leaves stacked as
-// (record, slot), whose items the pop had to read, six instanced views took 89.2 ms, now 87.0.
 enum : int { kStepOk = 0, kStepPop = 1, kStepOverflow = 2 };
 template <class Stack>
 __device__ __forceinline__ int trav_node4(Trav& tr, const DevScene& s, Stack& stk) {
-  const Ray& r = tr.level ? tr.orr : tr.wr;
-  const V3 inv = tr.level ? tr.oinv : tr.winv;
+  const Ray& r = tr.orr;
+  const V3 inv = tr.oinv;
   const float4* q = node4_at(s, tr.cur);
   const float4 lx = __ldg(q), ly = __ldg(q + 1), lz = __ldg(q + 2);
   const float4 hx = __ldg(q + 3), hy = __ldg(q + 4), hz = __ldg(q + 5);
@@ -244,7 +259,7 @@ __device__ __forceinline__ int trav_node4(Trav& tr, const DevScene& s, Stack& st
   // that child's own split axis: BVH.fs near-child rule at both levels) depends on the ray only
   // through its octant; the upload stored the slot order of each octant, 8 bits per octant: bit 1
   // swaps the pairs, bits 0 and 4 the slots of the pair then first and second
-  const int oct = tr.level ? tr.ooct : tr.woct;
+  const int oct = tr.ooct;
   const unsigned order = static_cast<unsigned>(oct & 4 ? orders.y : orders.x) >> (8 * (oct & 3));
   const bool sp = order & 2u, sa = order & 1u, sb = order & 16u;
   const int a0 = sp ? c2 : c0, a1 = sp ? c3 : c1, b0 = sp ? c0 : c2, b1 = sp ? c1 : c3;
@@ -265,7 +280,7 @@ __device__ __forceinline__ int trav_node4(Trav& tr, const DevScene& s, Stack& st
 
 // one step: a wide record or a node pair, one instance (kInstRun: the leaf's instances until one
 // is entered), or kTris triangles of a leaf (0 = the rest of it); returns true once the walk is
-// finished (tr.found / tr.hit hold the answer).
+// finished (tr.found() and tr.hit() give the answer).
 // kAny: kClosest, kAnyHit, or kAnyRuntime (tr.any decides).  Every branch that exhausts its unit
 // asks for a pop, which runs once at the end of the step.
 enum : int { kClosest = 0, kAnyHit = 1, kAnyRuntime = 2 };
@@ -283,8 +298,8 @@ __device__ __forceinline__ bool trav_step(Trav& tr, const DevScene& s, Stack& st
     }
     pop = r == kStepPop;
   } else if (tr.mode == kTravNode) {
-    const Ray& r = tr.level ? tr.orr : tr.wr;
-    const V3 inv = tr.level ? tr.oinv : tr.winv;
+    const Ray& r = tr.orr;
+    const V3 inv = tr.oinv;
     const int li = tr.cur + 1, ri = tr.n.link;
     const NodeRec a = load_node(s.nodes, tr.base + li);
     const NodeRec b = load_node(s.nodes, tr.base + ri);
@@ -312,10 +327,11 @@ __device__ __forceinline__ bool trav_step(Trav& tr, const DevScene& s, Stack& st
     // kTris triangles of a BLAS leaf (0: the rest of the leaf): each the triangle test, then its AABB
     // test (Mesh.fs:204,231).  The reference tests the box first; a hit needs both, and the triangle
     // test turns most triangles away earlier.
-    int done = 0;
+    int done = 0, ti = tr.ti, ti_end = tr.ti_end;
+    if (kWide) leaf_items(s, tr.cur, &ti, &ti_end);
 #pragma unroll 1
-    while (tr.ti < tr.ti_end) {
-      const int j = tr.ti++;
+    while (ti < ti_end) {
+      const int j = ti++;
       const float4* tp = s.tris + 3 * (tr.tri_base + j);
       const float4 a = __ldg(tp), b = __ldg(tp + 1), c = __ldg(tp + 2);
       if (kCount) cnt->tris++;
@@ -326,18 +342,20 @@ __device__ __forceinline__ bool trav_step(Trav& tr, const DevScene& s, Stack& st
       if (h) {
         const V3 lo = min_native(min_native(p0, p1), p2), hi = max_native(max_native(p0, p1), p2);
         if (box_hit(lo, hi, tr.orr, tr.oinv, tr.t)) {
-          tr.found = true;
+          tr.hinst = tr.ii - 1;
           if (any) {
             tr.mode = kTravDone;
             return true;
           }
           tr.t = tt;
-          tr.hit.inst = tr.inst; tr.hit.tri = j; tr.hit.t = tt; tr.hit.u = uu; tr.hit.v = vv; tr.hit.sphere_root = 0;
+          tr.hprim = j; tr.hu = uu; tr.hv = vv;
         }
       }
       if (kTris > 0 && ++done >= kTris) break;
     }
-    pop = tr.ti >= tr.ti_end;
+    pop = ti >= ti_end;
+    if (!kWide) tr.ti = ti;
+    else if (!pop) tr.cur = leaf_code(s, ti, ti_end - ti);
   } else if (tr.mode == kTravInst) {
     // the next instance of a TLAS leaf, or with kInstRun the leaf's instances until one is
     // entered (PrimitiveInstance.Intersect, Primitive.fs:111-129)
@@ -356,33 +374,37 @@ __device__ __forceinline__ bool trav_step(Trav& tr, const DevScene& s, Stack& st
       const float4 rlo = __ldg(line + 5), rhi = __ldg(line + 6);
       const int4 ids = __ldg(reinterpret_cast<const int4*>(line + 7));  // prim_type, node_base, tri_base, node4_root
       if (box_hit(xyz(bmin), xyz(bmax), tr.wr, tr.winv, tr.t)) {
-        tr.orr.o = xf_point(w2o, tr.wr.o);
-        tr.orr.d = xf_dir(w2o, tr.wr.d);
+        Ray orr;
+        orr.o = xf_point(w2o, tr.wr.o);
+        orr.d = xf_dir(w2o, tr.wr.d);
         if (ids.x == kPrimSphere) {
           float ts;
-          const int root = sphere_hit(bmax.w, tr.orr, tr.t, &ts);
+          const int root = sphere_hit(bmax.w, orr, tr.t, &ts);
           if (root) {
-            tr.found = true;
+            tr.hinst = k;
             if (any) {
               tr.mode = kTravDone;
               return true;
             }
             tr.t = ts;
-            tr.hit.inst = k; tr.hit.tri = 0; tr.hit.sphere_root = root; tr.hit.t = ts; tr.hit.u = 0.f; tr.hit.v = 0.f;
+            tr.hprim = ~root; tr.hu = 0.f; tr.hv = 0.f;
           }
         } else {
-          tr.oinv = inv_dir(tr.orr.d);
-          tr.ooct = octant(tr.orr.d);
-          if (kWT) tr.wt = wt_setup(tr.orr.d);
+          const V3 oinv = inv_dir(orr.d);
+          auto enter = [&]() {
+            tr.orr = orr;
+            tr.oinv = oinv;
+            tr.ooct = octant(orr.d);
+            if (kWT) tr.wt = wt_setup(orr.d);
+          };
           const int base = ids.y;
           float te;
           if (kWide && ids.w >= 0) {
             // the root's box from the instance line, its record next (the root is interior)
-            if (box_hit_t(xyz(rlo), xyz(rhi), tr.orr, tr.oinv, tr.t, &te)) {
-              tr.level = 1;
+            if (box_hit_t(xyz(rlo), xyz(rhi), orr, oinv, tr.t, &te)) {
+              enter();
               tr.base = base;
               tr.tri_base = ids.z;
-              tr.inst = k;
               tr.blas_sp0 = tr.sp;
               tr.cur = ids.w;
               tr.mode = kTravNode;
@@ -391,13 +413,13 @@ __device__ __forceinline__ bool trav_step(Trav& tr, const DevScene& s, Stack& st
           } else {
             const NodeRec root = load_node(s.nodes, base);
             if (kCount) cnt->nodes++;
-            if (box_hit_t(root.bmin, root.bmax, tr.orr, tr.oinv, tr.t, &te)) {
-              tr.level = 1;
+            if (box_hit_t(root.bmin, root.bmax, orr, oinv, tr.t, &te)) {
+              enter();
               tr.base = base;
               tr.tri_base = ids.z;
-              tr.inst = k;
               tr.blas_sp0 = tr.sp;
-              trav_enter(tr, 0, root);
+              if (kWide) trav_enter_code(tr, s, leaf_code(s, root.link, root.count));  // (a leaf)
+              else trav_enter(tr, 0, root);
               entered = true;
             }
           }
@@ -442,8 +464,8 @@ __device__ __forceinline__ bool trace_walk_inline(const DevScene& s, const Ray& 
   trav_init<kWalk>(tr, s, ray, tmax, cnt);
   while (!trav_step<kAny, kWT, kWalk, 0>(tr, s, stk, cnt)) {
   }
-  if (kAny == kClosest) *hit = tr.hit;
-  return tr.found;
+  if (kAny == kClosest) *hit = tr.hit();
+  return tr.found();
 }
 
 // One walk for both queries, kept out of line: a path loop that traces closest and any hits
@@ -459,8 +481,8 @@ __device__ __noinline__ bool trace_walk_outline(const DevScene& s, const Ray& ra
   trav_init<kWalk>(tr, s, ray, tmax, cnt);
   while (!trav_step<kAnyRuntime, kWT, kWalk, 0>(tr, s, stk, cnt)) {
   }
-  if (!any) *hit = tr.hit;
-  return tr.found;
+  if (!any) *hit = tr.hit();
+  return tr.found();
 }
 
 template <bool kWT, int kWalk, bool kOutline = false>

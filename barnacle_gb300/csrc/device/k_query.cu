@@ -65,13 +65,13 @@ __global__ void __launch_bounds__(128) k_trace_plain(DevScene s, const bn_ray* _
 
 // Persistent lanes: a lane whose walk has ended writes its hit and claims the next ray, together
 // with its neighbours once half of the lanes still walk; the walking lanes vote on the kind of step
-// (dev_machine.cuh).  1,000,003 closest hits in the instanced scene take 1.13 ms against 1.61 with a
-// thread per ray, any hits 0.71 against 0.99, Cornell with objects 0.45 against 0.60.  6 blocks per SM (80
-// registers); 7 blocks 1.12 ms, 5 blocks 1.19; service when 20, 12 or 8 of 32 lanes still walk 1.13,
-// 1.16, 1.19 ms.  Few rays are spread over the warps, so none waits for a neighbour (64 rays of
+// (dev_machine.cuh).  1,000,003 closest hits in the instanced scene took 1.13 ms against 1.61 with a
+// thread per ray, any hits 0.71 against 0.99, Cornell with objects 0.45 against 0.60; with the walk's
+// later changes 0.97 and 0.64.  7 blocks per SM (72 registers); 8 blocks 0.99 ms, 6 blocks 1.00, 5 blocks
+// 1.09; service when 20, 12 or 8 of 32 lanes still walk 1.13, 1.16, 1.19 ms where 16 took 1.13.  Few rays are spread over the warps, so none waits for a neighbour (64 rays of
 // the Cornell box: 18 us against 27).  Between the two, at about one ray per lane, the votes buy
 // nothing (30,001 instanced / 131,071 Cornell-with-objects rays: 0.205 / 0.125 against 0.199 / 0.114 ms).
-constexpr int kTraceBlocks = 6;
+constexpr int kTraceBlocks = 7;
 constexpr long long kTraceFew = 4096, kTraceMany = 196608;
 template <bool kAny, bool kWT, int kWalk>
 __global__ void __launch_bounds__(kMachineThreads, kTraceBlocks)
@@ -92,9 +92,9 @@ __global__ void __launch_bounds__(kMachineThreads, kTraceBlocks)
         out.t = tmax;
         out.instance = out.primitive = -1;
         if (kAny) {
-          if (tr.found) out.instance = 0;
-        } else if (tr.found) {
-          put_closest(&out, s, tr.wr, tr.hit);
+          if (tr.found()) out.instance = 0;
+        } else if (tr.found()) {
+          put_closest(&out, s, tr.wr, tr.hit());
         }
         hits[at] = out;
       }

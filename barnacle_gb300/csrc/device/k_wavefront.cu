@@ -35,7 +35,12 @@ constexpr int kBinMiss = 4, kBinNoMaterial = 5;
 constexpr int kWfTris = 4;
 constexpr bool kWfInstRun = true;
 // blocks of 128 per SM the traversal kernels are compiled for (registers: 65,536 / (128 x blocks))
+// Six instanced views of 4 spp took 82.2 ms; extend at 8 or 6 blocks with shadow at 8: 83.2 and 83.5, shadow
+// at 7 or 9 with extend at 7: 82.4 and 83.2.
 constexpr int kExtendBlocks = 7, kShadowBlocks = 8;
+// a traversal warp refills once at most this many of its lanes still walk (12 / 16 / 20 / 24 measured
+// 192.9 / 193.7 / 191.6 / 187.8 M paths/s on the instanced workload, when the mode vote came in)
+constexpr int kWfRefill = 16;
 // stack entries per lane kept in shared memory (8 bytes each, x 128 lanes per block)
 constexpr int kWfSharedStack = 16;
 using WfStack = SharedStack<kWfSharedStack, 128>;
@@ -248,30 +253,30 @@ __device__ __forceinline__ int lanes_taking_rays(int n) {
   return min(32, max(1, (n + warps - 1) / warps));
 }
 
+// The scene comes as a parameter beside WfParams: its pointers are then constants, not loads or
+// registers (walk_scene).  With the walk's state as small as Trav has it, nothing is spilled under these
+// bounds: a quarter of the L1 requests were spills (six instanced views of 4 spp 87.0 -> 80.6 ms, Cornell
+// with objects 19.7 -> 18.7, Cornell 5.68 -> 5.54).
 template <bool kWT, int kWalk>
-__global__ void __launch_bounds__(128, kExtendBlocks) k_wf_extend(const WfParams* __restrict__ pp) {
+__global__ void __launch_bounds__(128, kExtendBlocks) k_wf_extend(const WfParams* __restrict__ pp, const DevScene s) {
   const WfParams& p = *pp;
-  const DevScene& s = p.scene;
   const int n = min(p.counters[kCntActive], p.pool);
-  const int refill_below = p.refill_extend;
   if ((threadIdx.x & 31) >= lanes_taking_rays<kWalk>(n)) return;
   __shared__ int2 stack_block[kWfSharedStack * 128];
   WfStack stk(stack_block);
   Trav tr;
   TraceCounters tc{0, 0, 0};
   unsigned long long nrays = 0;  // rays this lane walked (counting walks)
-  int slot = -1;
-  bool have = false;
+  int slot = -1;  // the lane's ray, -1: none
   for (;;) {
     // (a walk can end at init, its root box missed)
-    TravVote vote(__activemask(), have, tr.mode);
-    if (vote.walking() <= refill_below) {
-      if (have && tr.mode == kTravDone) {
-        have = false;
+    TravVote vote(__activemask(), slot >= 0, tr.mode);
+    if (vote.walking() <= kWfRefill) {
+      if (slot >= 0 && tr.mode == kTravDone) {
         int bin = kBinMiss;
         float4* hr = p.slot + 8LL * slot + 2;
-        if (tr.found) {
-          const HitRec& h = tr.hit;
+        if (tr.found()) {
+          const HitRec h = tr.hit();
           hr[0] = make_float4(h.t, h.u, h.v, __int_as_float(h.inst));
           hr[1] = make_float4(__int_as_float(h.sphere_root ? h.sphere_root : h.tri), 0.f, 0.f, 0.f);
           const DevInstance* I = s.inst + h.inst;
@@ -280,7 +285,7 @@ __global__ void __launch_bounds__(128, kExtendBlocks) k_wf_extend(const WfParams
             const int slot_m = __float_as_int(__ldg(&s.tris[3 * (__ldg(&I->tri_base) + h.tri)].w));
             if (slot_m >= 0) m = slot_m;
           }
-          bin = m < 0 ? kBinNoMaterial : s.mats[m].type;
+          bin = m < 0 ? kBinNoMaterial : p.scene.mats[m].type;
         } else {
           hr[0] = make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
         }
@@ -295,9 +300,10 @@ __global__ void __launch_bounds__(128, kExtendBlocks) k_wf_extend(const WfParams
         const int qb = base + __popc(peers & ((1u << lane) - 1u));
         if (qb < p.pool) p.q_bins[static_cast<long long>(bin) * p.pool + qb] = slot;
         else flag_error(s, BN_DEVERR_QUEUE_OVERFLOW);
+        slot = -1;
       }
-      const int qi = fetch_next(&p.counters[kCntFetchRay], !have);
-      if (!have) {
+      const int qi = fetch_next(&p.counters[kCntFetchRay], slot < 0);
+      if (slot < 0) {
         if (qi >= n) break;
         slot = p.q_ray[qi];
         const float4 o = p.slot[8LL * slot], d = p.slot[8LL * slot + 1];
@@ -305,12 +311,11 @@ __global__ void __launch_bounds__(128, kExtendBlocks) k_wf_extend(const WfParams
         ray.o = mk(o.x, o.y, o.z);
         ray.d = mk(d.x, d.y, d.z);
         trav_init<kWalk>(tr, s, ray, CUDART_INF_F, &tc);
-        have = true;
         ++nrays;
       }
-      vote = TravVote(__activemask(), have, tr.mode);
+      vote = TravVote(__activemask(), slot >= 0, tr.mode);
     }
-    if (have && tr.mode == vote.pick()) trav_step<kClosest, kWT, kWalk, kWfTris, kWfInstRun>(tr, s, stk, &tc);
+    if (slot >= 0 && tr.mode == vote.pick()) trav_step<kClosest, kWT, kWalk, kWfTris, kWfInstRun>(tr, s, stk, &tc);
   }
   if (kWalk == kWalkCount) add_trace_counts(p.trace_counters, nrays, tc);
 }
@@ -554,34 +559,32 @@ __global__ void __launch_bounds__(128, 5) k_wf_shade(const WfParams* __restrict_
 }
 
 template <bool kWT, int kWalk>
-__global__ void __launch_bounds__(128, kShadowBlocks) k_wf_shadow(const WfParams* __restrict__ pp) {
+__global__ void __launch_bounds__(128, kShadowBlocks) k_wf_shadow(const WfParams* __restrict__ pp, const DevScene s) {
   const WfParams& p = *pp;
   const int n = min(p.counters[kCntShadow], p.pool);
-  const int refill_below = p.refill_shadow;
   if ((threadIdx.x & 31) >= lanes_taking_rays<kWalk>(n)) return;
   __shared__ int2 stack_block[kWfSharedStack * 128];
   WfStack stk(stack_block);
   Trav tr;
   TraceCounters tc{0, 0, 0};
   unsigned long long nrays = 0;  // rays this lane walked (counting walks)
-  int rec = -1;
-  bool have = false;
+  int rec = -1;  // the lane's shadow record, -1: none
   for (;;) {
     // (a walk can end at init, its root box missed)
-    TravVote vote(__activemask(), have, tr.mode);
-    if (vote.walking() <= refill_below) {
-      if (have && tr.mode == kTravDone) {
-        have = false;
-        if (!tr.found) {
+    TravVote vote(__activemask(), rec >= 0, tr.mode);
+    if (vote.walking() <= kWfRefill) {
+      if (rec >= 0 && tr.mode == kTravDone) {
+        if (!tr.found()) {
           const float4* r = p.shadow + 4LL * rec;
           const int slot = __float_as_int(r[1].w);
           const float4 Ln = r[2];
           p.slot[8LL * slot + 5] = make_float4(Ln.x, Ln.y, Ln.z, 0.f);
           if (p.lit) p.lit[__float_as_int(Ln.w)] = 1;
         }
+        rec = -1;
       }
-      const int qi = fetch_next(&p.counters[kCntFetchShadow], !have);
-      if (!have) {
+      const int qi = fetch_next(&p.counters[kCntFetchShadow], rec < 0);
+      if (rec < 0) {
         if (qi >= n) break;
         rec = p.sort_shadow ? p.q_shadow[qi] : qi;
         const float4* r = p.shadow + 4LL * rec;
@@ -589,13 +592,12 @@ __global__ void __launch_bounds__(128, kShadowBlocks) k_wf_shadow(const WfParams
         Ray ray;
         ray.o = mk(o.x, o.y, o.z);
         ray.d = mk(d.x, d.y, d.z);
-        trav_init<kWalk>(tr, p.scene, ray, o.w, &tc);
-        have = true;
+        trav_init<kWalk>(tr, s, ray, o.w, &tc);
         ++nrays;
       }
-      vote = TravVote(__activemask(), have, tr.mode);
+      vote = TravVote(__activemask(), rec >= 0, tr.mode);
     }
-    if (have && tr.mode == vote.pick()) trav_step<kAnyHit, kWT, kWalk, kWfTris, kWfInstRun>(tr, p.scene, stk, &tc);
+    if (rec >= 0 && tr.mode == vote.pick()) trav_step<kAnyHit, kWT, kWalk, kWfTris, kWfInstRun>(tr, s, stk, &tc);
   }
   if (kWalk == kWalkCount) add_trace_counts(p.trace_counters, nrays, tc);
 }
@@ -731,8 +733,8 @@ cudaError_t wf_launch_iteration(WfParams* dparams, const WfLaunch& l, bool use_g
         if ((e = cudaEventRecord(fk->fork, st)) != cudaSuccess) return;
         if ((e = cudaStreamWaitEvent(fk->side, fk->fork, 0)) != cudaSuccess) return;
       }
-      k_wf_shadow<kWT, kWalk><<<l.grid_shadow, 128, 0, fk ? fk->side : st>>>(dparams);
-      k_wf_extend<kWT, kWalk><<<l.grid_extend, 128, 0, st>>>(dparams);
+      k_wf_shadow<kWT, kWalk><<<l.grid_shadow, 128, 0, fk ? fk->side : st>>>(dparams, l.walk);
+      k_wf_extend<kWT, kWalk><<<l.grid_extend, 128, 0, st>>>(dparams, l.walk);
       if (fk) {
         if ((e = cudaEventRecord(fk->join, fk->side)) != cudaSuccess) return;
         if ((e = cudaStreamWaitEvent(st, fk->join, 0)) != cudaSuccess) return;
@@ -743,10 +745,10 @@ cudaError_t wf_launch_iteration(WfParams* dparams, const WfLaunch& l, bool use_g
     }
     k_wf_regen<<<l.grid_regen, 256, 0, st>>>(dparams);
     sort(0);
-    k_wf_extend<kWT, kWalk><<<l.grid_extend, 128, 0, st>>>(dparams);
+    k_wf_extend<kWT, kWalk><<<l.grid_extend, 128, 0, st>>>(dparams, l.walk);
     k_wf_shade<kWT><<<l.grid_shade, 128, 0, st>>>(dparams);
     sort(1);
-    k_wf_shadow<kWT, kWalk><<<l.grid_shadow, 128, 0, st>>>(dparams);
+    k_wf_shadow<kWT, kWalk><<<l.grid_shadow, 128, 0, st>>>(dparams, l.walk);
   };
   using WT = std::integral_constant<bool, true>;
   using MT = std::integral_constant<bool, false>;

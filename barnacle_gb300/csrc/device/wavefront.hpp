@@ -64,8 +64,6 @@ struct WfParams {
   int integrator;               // BN_INTEGRATOR_PATH, _NORMAL or _DIRECT
   int pool;                     // path slots
   int max_iters;                // watchdog
-  int refill_extend;            // extend lanes refill when at most this many of a warp still walk
-  int refill_shadow;            // the same for the shadow kernel
   long long first_path;         // path ids [first_path, total_paths)
   long long total_paths;
   long long n_pixels;
@@ -118,7 +116,21 @@ struct WfLaunch {
   bool count;                   // binary walks that count their visits (BN_RENDER_COUNT)
   bool mlt;                     // PSSMLT chains: mlt regen and shade kernels instead of regen / shade
   bool mlt_kelemen;             // their mutation strategy (Kelemen, else Gaussian)
+  DevScene walk;                // what the walks read of the scene (walk_scene)
 };
+
+// The fields that a walk reads, as a parameter of the traversal kernels: there they are constants.
+inline DevScene walk_scene(const DevScene& s) {
+  DevScene w{};
+  w.nodes = s.nodes;
+  w.nodes4 = s.nodes4;
+  w.tris = s.tris;
+  w.inst = s.inst;
+  w.leaf_bits = s.leaf_bits;
+  w.stack_cap = s.stack_cap;
+  w.error_word = s.error_word;
+  return w;
+}
 
 // mlt_chains: PSSMLT chains (one slot each); sizes the traversal grids so both fit side by side
 WfLaunch wf_launch_shape(bool watertight, bool wide, bool sort, bool sort_shadow, bool count, int blocks_per_sm_cap,

@@ -98,6 +98,24 @@ def test_wavefront_ragged_record_tiles(ctx, w, h, spp, pool):
     assert_same_image(wave, mega)
 
 
+@pytest.mark.parametrize("bvh", [capi.BN_BVH_BINARY, capi.BN_BVH_WIDE])
+def test_wavefront_follows_the_uploaded_scene(bvh):
+    """The captured bounce loop holds the scene's buffers: another upload, whose buffers lie elsewhere or
+    hold another scene, is followed by the next render, with the graph and without."""
+    from barnacle_gb300 import Context
+
+    with Context() as c:
+        for name in ("cornell", "instances", "materials", "cornell"):
+            b = Bundle.generate(name, 1)
+            b.scene.contents.bvh_width = bvh
+            c.upload(b)
+            v = b.views[0]
+            v.width, v.height = 97, 61
+            mega = render(c, b, [v], 2, capi.BN_MODE_MEGAKERNEL)[0]
+            for flags in (0, capi.BN_RENDER_NO_GRAPH):
+                assert_same_image(render(c, b, [v], 2, capi.BN_MODE_WAVEFRONT, flags=flags)[0], mega)
+
+
 def test_wavefront_many_views_one_launch(ctx):
     b = Bundle.generate("instances", 1)
     ctx.upload(b)
