@@ -12,7 +12,7 @@
 //   shade    emission with MIS, light sample + BSDF eval (a shadow-ray record), BSDF sample,
 //            Russian roulette; paths that go on are appended to the next iteration's ray queue with
 //            their keys, the others to the queue of ended ones
-//   sort     the same counting sort of the shadow queue
+//   sort     the same counting sort of the shadow queue, in scenes of many instances
 //   shadow   any hit for the shadow queue; unoccluded records add their NEE term to L
 //   control  one thread: decides whether another iteration is needed, resets the counters and
 //            sets the CUDA-graph while-condition (or a flag for host-driven loops); an iteration
@@ -72,16 +72,18 @@ __device__ __forceinline__ int ray_key(const WfParams& p, V3 o, V3 d) {
   const unsigned x = static_cast<unsigned>(fminf(fmaxf((o.x - p.key_lo.x) * p.key_scale.x, 0.f), top));
   const unsigned y = static_cast<unsigned>(fminf(fmaxf((o.y - p.key_lo.y) * p.key_scale.y, 0.f), 7.f));
   const unsigned z = static_cast<unsigned>(fminf(fmaxf((o.z - p.key_lo.z) * p.key_scale.z, 0.f), top));
-  // interleave x(b-1) z(b-1) y2 x(b-2) z(b-2) y1 x(b-3) z(b-3) y0 ... x0 z0 (2b + 3 bits)
-  unsigned m = 0;
-  int b = 0;
-  for (int k = 0; k < nb; ++k) {
-    m |= ((z >> k) & 1u) << b++;
-    m |= ((x >> k) & 1u) << b++;
-    if (k >= nb - 3) m |= ((y >> (k - (nb - 3))) & 1u) << b++;
-  }
+  // interleave x(b-1) z(b-1) y2 x(b-2) z(b-2) y1 x(b-3) z(b-3) y0 ... x0 z0 (2b + 3 bits): x and z, of
+  // at most 8 bits, spread over even bits side by side, then y's bits put behind the top three pairs
+  unsigned v = z | (x << 16);
+  v = (v | (v << 4)) & 0x0f0f0f0fu;
+  v = (v | (v << 2)) & 0x33333333u;
+  v = (v | (v << 1)) & 0x55555555u;
+  v = (v & 0xffffu) | (v >> 15);
+  const int low = 2 * (nb - 3);
+  const unsigned t = v >> low;
+  const unsigned top3 = (t & 3u) | ((t & 12u) << 1) | ((t & 48u) << 2) | ((y & 1u) << 2) | ((y & 2u) << 4) | ((y & 4u) << 6);
   const unsigned oct = (d.x < 0.f ? 1u : 0u) | (d.y < 0.f ? 2u : 0u) | (d.z < 0.f ? 4u : 0u);
-  return static_cast<int>((oct << b) | m);
+  return static_cast<int>((((oct << 9) | top3) << low) | (v & ((1u << low) - 1u)));
 }
 
 // histogram of the keys of the lanes with pred; lanes with equal keys share one atomic (an atomic per
@@ -538,10 +540,12 @@ __global__ void __launch_bounds__(128, 5) k_wf_shade(const WfParams* __restrict_
     if (shadow) {
       float4* r = p.shadow + 4LL * si;
       r[0] = sh_o; r[1] = sh_d; r[2] = sh_L;
-      shadow_key = ray_key(p, mk(sh_o.x, sh_o.y, sh_o.z), mk(sh_d.x, sh_d.y, sh_d.z));
-      p.sh_key[si] = shadow_key;
+      if (p.sort_shadow) {
+        shadow_key = ray_key(p, mk(sh_o.x, sh_o.y, sh_o.z), mk(sh_d.x, sh_d.y, sh_d.z));
+        p.sh_key[si] = shadow_key;
+      }
     }
-    hist_add(p.hist + kSortBins, shadow_key, shadow);
+    if (p.sort_shadow) hist_add(p.hist + kSortBins, shadow_key, shadow);
     // the paths that go on are the next iteration's ray queue
     const int qi = push(p, &p.counters[kCntActiveNext], &cont);
     if (cont) {
