@@ -140,9 +140,14 @@ int run(bn_context* ctx, WfState* w, const bn::DevScene& scene, const bn_render_
     return ctx->cuda_fail(e, "wavefront film allocation");
   const bool wt = d->flags & BN_RENDER_WATERTIGHT;
   const bool wide = scene.wide != 0;
-  // both queues sorted by ray key: on the 1,024-instance workload 111.5 M paths/s against 110.0
-  // (ray queue only) and 107.9 (neither)
-  const bool sort = true, sort_shadow = true;
+  // The ray queue is sorted by ray key: without it 8 to 10 % more.  Shadow rays are sorted in scenes of
+  // many instances.  They are written in the order in which the sorted extension rays ended, and in a
+  // scene of few instances that is order enough: kernel ms sorted / not, 16 instanced views of 4 spp (1,089
+  // instances) 225.9 / 229.7, one view 16.92 / 16.95; Cornell box at 64 and 256 spp (8 instances) 5.44 / 5.28
+  // and 20.4 / 19.6, Cornell with objects at 8, 32 and 128 spp (11) 7.45 / 7.31, 18.45 / 18.22 and 62.3 /
+  // 61.4, materials at 32, 128 and 512 spp (14) 4.54 / 4.47, 12.15 / 12.18 and 43.1 / 43.6.  The line lies
+  // between the measured 14 and 1,089.
+  const bool sort = true, sort_shadow = scene.n_inst >= 128;
   const bool count = d->flags & BN_RENDER_COUNT;
   const int key_bits = bn::sort_key_bits(pool);
   if (w->shape_cap != cap || w->shape.watertight != wt || w->shape.wide != wide || w->shape.sort != sort ||
