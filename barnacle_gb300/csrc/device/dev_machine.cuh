@@ -7,7 +7,7 @@
 // alternates two things:
 //   * walk     the walking lanes vote on the kind of unit (TravVote) and the winners take one
 //              step of their walk;
-//   * service  once at most a quarter of the lanes still walk, every lane whose walk has ended is served
+//   * service  once at most an eighth of the lanes still walk, every lane whose walk has ended is served
 //              together: a shadow ray's answer is added, a hit is shaded, an ended path is handed
 //              to the task and the lane's next path is begun, and the lane's next walk is set up.
 // So a lane with a short path goes on to its next one instead of waiting, and both the walk and
@@ -49,11 +49,12 @@ __host__ __device__ __forceinline__ int machine_lanes(long long n, long long war
 
 // Launch shape.  Blocks of 128, 4 per SM (128 registers): 64 spp of the Cornell box / 32 spp of
 // Cornell with objects / two instanced views of 4 spp took 10.0 / 45.7 / 35.8 ms, at 5 blocks 10.4 /
-// 48.4 / 35.5, at 6 blocks 11.6 / 50.1 / 36.1 (spills), at 3 up to 15 % more than at 4.  Service when 20, 16,
-// 12, 8 or 4 of the 32 lanes still walk: 12.4 10.6 10.2 10.1 9.9 / 60.2 56.1 53.2 51.1 51 / 47.6
-// 42.6 39.8 38.6 40 (before the inner walk loop): a quarter of the lanes.
+// 48.4 / 35.5, at 6 blocks 11.6 / 50.1 / 36.1 (spills), at 3 up to 15 % more than at 4.  Service when 8, 4, 3
+// or 2 of the 32 lanes still walk: Cornell with objects at 3 spp 4.90 4.74 4.66 4.73 ms, one instanced
+// view at 1 spp 6.33 6.34 6.49 6.76, 65,536 PSSMLT chains 55.1 53.0 52.5 52.9 (when 12 still walk 57): an
+// eighth of the lanes.
 constexpr int kMachineThreads = 128, kMachineBlocks = 4;
-constexpr int kMachineRefill = 8;
+constexpr int kMachineRefill = 4;
 constexpr int kMachineStack = 16;  // stack entries per lane in shared memory
 
 enum : int { kLaneNew = 0, kLaneClosest = 1, kLaneShadow = 2, kLaneIdle = 3 };

@@ -169,9 +169,11 @@ struct MltTask {
 // 65,536 chains of a 512^2 render (Cornell with objects, Kelemen) took 94.5 ms as a plain loop per
 // chain in lockstep (4.1 lanes active, 205 KB of code, no instruction to issue 12 cycles out of
 // 16); on the path machine 91, with one copy of the draws (113 KB) 60, with the
-// normalisations called 54.9; 4,096 chains 383 -> 203 ms.  3 blocks per SM (153 registers, no spills): the
-// lanes are as many as the chains, about 27 per warp at 4 blocks, which took 57.4 ms.
-constexpr int kChainBlocks = 3;
+// normalisations called 54.9; 4,096 chains 383 -> 203 ms.  4 blocks per SM (128 registers, no spills since
+// the walk's state is small enough) against 3 (141), both with service at an eighth: 65,536 chains 53.0 and 52.7
+// ms, 262,144 chains 44.0 and 45.3, 4,096 chains 193 and 200; in the Cornell box 34.5 and 35.9; with the
+// Gaussian strategy 62.2 and 60.9, 262,144 chains 51.8 and 52.7.
+constexpr int kChainBlocks = 4;
 
 // kKelemen: the mutation strategy fixed at compile time (1 Kelemen, 0 Gaussian), so the kernel
 // holds one strategy's code
