@@ -77,8 +77,10 @@ template <bool kAny, bool kWT, int kWalk>
 __global__ void __launch_bounds__(kMachineThreads, kTraceBlocks)
     k_trace(DevScene s, const bn_ray* __restrict__ rays, bn_hit* __restrict__ hits, long long n, unsigned long long* next,
             int lanes) {
-  __shared__ int2 stack_block[kMachineStack * kMachineThreads];
-  SharedStack<kMachineStack, kMachineThreads> stk(stack_block);
+  using Stack = std::conditional_t<kAny, SharedCodes<kMachineStack, kMachineThreads>,
+                                   SharedStack<kMachineStack, kMachineThreads>>;
+  __shared__ typename Stack::Entry stack_block[kMachineStack * kMachineThreads];
+  Stack stk(stack_block);
   TraceCounters tc{0, 0, 0};
   Trav tr;
   tr.mode = kTravDone;

@@ -44,6 +44,7 @@ constexpr int kWfRefill = 16;
 // stack entries per lane kept in shared memory (8 bytes each, x 128 lanes per block)
 constexpr int kWfSharedStack = 16;
 using WfStack = SharedStack<kWfSharedStack, 128>;
+using WfShadowStack = SharedCodes<kWfSharedStack, 128>;
 
 __device__ __forceinline__ int warp_append(int* counter, bool pred) {
   // ballot + popc compaction: one atomic per warp
@@ -601,8 +602,8 @@ __global__ void __launch_bounds__(128, kShadowBlocks) k_wf_shadow(const WfParams
   const WfParams& p = *pp;
   const int n = min(p.counters[kCntShadow], p.pool);
   if ((threadIdx.x & 31) >= lanes_taking_rays<kWalk>(n)) return;
-  __shared__ int2 stack_block[kWfSharedStack * 128];
-  WfStack stk(stack_block);
+  __shared__ WfShadowStack::Entry stack_block[kWfSharedStack * 128];
+  WfShadowStack stk(stack_block);
   Trav tr;
   TraceCounters tc{0, 0, 0};
   unsigned long long nrays = 0;  // rays this lane walked (counting walks)
