@@ -105,7 +105,7 @@ int follow_paths(bn_context* ctx, const bn_adjoint_desc* d, const bn::AdjParams&
                                 ctx->n_lights, st)) != cudaSuccess)
     return ctx->cuda_fail(e, "adjoint scene launch");
   bool ran = false;
-  if (n >= (1 << 20)) {
+  if (n >= bnc::kQueuePaths) {
     bn_render_desc r{};
     r.integrator = BN_INTEGRATOR_PATH;
     r.spp = d->spp;

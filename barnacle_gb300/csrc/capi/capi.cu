@@ -131,13 +131,10 @@ int render_megakernel(bn_context* ctx, const bn_render_desc* d, const std::vecto
   p.count = count;
   p.partial = ctx->partial.as<float4>();
   p.film = ctx->film.as<float>();
-  // The path tracer's long renders run their paths through the wavefront's queues, whose sorted
-  // rays keep 15 to 26 of a warp's 32 lanes walking where one kernel's lanes keep 9 to 11; their
-  // radiances are summed in this mode's order.  The line is where the two take as long
-  // (262,144 / 1.23 M / 2.10 M paths, kernel ms: Cornell box 0.67 2.8 4.8 against 0.91 2.2 3.4, Cornell with objects
-  // 2.0 6.9 12.3 against 4.0 6.5 8.6, an instanced view 3.0 9.7 17.3 against 6.4 11.4 15.4).
+  // The path tracer's long renders run their paths through the wavefront's queues; their radiances
+  // are summed in this mode's order.
   if (d->integrator == BN_INTEGRATOR_PATH && !count && !(d->flags & BN_RENDER_CULL_SHADOW) && d->max_depth > 0 &&
-      p.n_paths >= (1 << 20) && d->spp <= 65536) {
+      p.n_paths >= bnc::kQueuePaths && d->spp <= 65536) {
     bool ran = false;
     const int rc = bnc::render_ordered(ctx, d, p, &ran);
     if (rc || ran) return rc;

@@ -112,6 +112,12 @@ MegaChunks mega_chunks(long long pixels, int spp, long long max_items);
 // offsets, partial sums, film and counting are filled in by the caller).
 bn::MegaParams mega_params(const bn_context* ctx, const bn_render_desc* d, const std::vector<bn::DevView>& views,
                            const MegaChunks& ck, long long items, long long pixels);
+// Paths from which on a render's paths run in the wavefront's queues, whose sorted rays keep 15 to 26 of
+// a warp's 32 lanes walking where the path machine's lanes keep 9 to 11.  Kernel ms on the machine / in
+// the queues: Cornell box at 393,216 and 786,432 paths 1.03 / 0.95 and 1.95 / 1.40 (196,608: 0.56 / 0.77),
+// Cornell with objects at 524,288 and 786,432 3.23 / 4.04 and 4.72 / 4.65, material forward 2.07 / 2.45 and 2.97 /
+// 2.74, material gradient 2.62 / 2.92 and 3.74 / 3.46, an instanced view at 2 and 3 spp 10.76 / 10.74 and 13.5 / 13.6.
+constexpr long long kQueuePaths = 3 << 18;
 // A megakernel-mode render (p: its launch parameters) whose paths run in the wavefront's queues and
 // are summed in the mode's order.  *ran stays false, with nothing rendered, when the path state
 // does not fit the GPU's free memory.

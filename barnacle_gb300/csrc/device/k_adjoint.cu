@@ -15,7 +15,7 @@
 //
 // When the sampling follows the values (sparams == params, every step of a fit), the paths are an
 // ordinary render of a scene with the slots' materials and the scaled lights (launch_adj_patch): they
-// run on the path machine or, from 1 M on, through the wavefront's queues, which leave each vertex's
+// run on the path machine or, from 0.8 M on, through the wavefront's queues, which leave each vertex's
 // hit (16 bytes) and whether its light sample was lit (a byte).  The adjoint then replays the paths
 // from those records without tracing a ray (k_adj_replay).  256^2, 16 spp, 32 slots, depth 8:
 // the gradient call 15.6 -> 4.7 ms (the adjoint's kernel 9.7 -> 0.85, the paths 5.9 -> 3.6), a forward

@@ -67,10 +67,12 @@ __global__ void __launch_bounds__(128) k_trace_plain(DevScene s, const bn_ray* _
 // with its neighbours once half of the lanes still walk; the walking lanes vote on the kind of step
 // (dev_machine.cuh).  1,000,003 closest hits in the instanced scene took 1.13 ms against 1.61 with a
 // thread per ray, any hits 0.71 against 0.99, Cornell with objects 0.45 against 0.60; with the walk's
-// later changes 0.97 and 0.64.  7 blocks per SM (72 registers); 8 blocks 0.99 ms, 6 blocks 1.00, 5 blocks
-// 1.09; service when 20, 12 or 8 of 32 lanes still walk 1.13, 1.16, 1.19 ms where 16 took 1.13.  Few rays are spread over the warps, so none waits for a neighbour (64 rays of
-// the Cornell box: 18 us against 27).  Between the two, at about one ray per lane, the votes buy
-// nothing (30,001 instanced / 131,071 Cornell-with-objects rays: 0.205 / 0.125 against 0.199 / 0.114 ms).
+// later changes 0.97 and 0.62.  7 blocks per SM (72 registers); 8 blocks 0.99 ms, 6 blocks 1.00, 5 blocks
+// 1.09; service when 20, 12 or 8 of 32 lanes still walk 1.13, 1.16, 1.19 ms where 16 took 1.13.  Few rays
+// are spread over the warps, so none waits for a neighbour (64 rays of the Cornell box: 18 us against 27).
+// Between the two, at about one ray per lane, the votes buy nothing (131,071 any hits in Cornell with
+// objects, 131,071 and 65,537 closest hits among instances: 0.124, 0.276 and 0.258 ms against 0.101, 0.262
+// and 0.240).
 constexpr int kTraceBlocks = 7;
 constexpr long long kTraceFew = 4096, kTraceMany = 196608;
 template <bool kAny, bool kWT, int kWalk>

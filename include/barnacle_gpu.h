@@ -177,7 +177,7 @@ enum bn_integrator_type {
 enum bn_render_mode {
   BN_MODE_MEGAKERNEL = 0, /* each pixel's samples summed in order (the film is the     */
                           /* same on every run); one kernel of lanes that run whole   */
-                          /* paths, from 1 M paths on the wavefront's queues (2 GB    */
+                          /* paths, from 0.8 M paths on the wavefront's queues (2 GB  */
                           /* and 240 B per slot of device memory at most; without it, */
                           /* the one kernel).  PSSMLT: a lane per chain               */
   BN_MODE_WAVEFRONT = 1   /* persistent queues compacted every bounce, many views per */

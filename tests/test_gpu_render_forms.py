@@ -62,6 +62,17 @@ def test_forms_agree_on_depths_and_walks(ctx, width, bvh):
         both(ctx, b, [v], 10, max_depth=depth, rr_depth=rr)
 
 
+@pytest.mark.parametrize("name", ["cornell", "materials"])
+@pytest.mark.parametrize("w,h,spp", [(4369, 6, 30), (512, 512, 3), (617, 425, 3)])
+def test_forms_agree_at_the_queues_line(ctx, name, w, h, spp):
+    """786,420, 786,432 and 786,675 paths: the last on the path machine, the first in the queues."""
+    b = Bundle.generate(name, 1)
+    ctx.upload(b)
+    v = b.views[0]
+    v.width, v.height = w, h
+    both(ctx, b, [v], spp)
+
+
 def test_wavefront_limits_leave_megakernel_renders_alone(ctx):
     """bn_set_limits' iteration cap is the wavefront mode's; the stack cap is every walk's."""
     b = Bundle.generate("cornell", 1)
