@@ -9,6 +9,7 @@ from __future__ import annotations
 import collections
 import ctypes as C
 import math
+import time
 import weakref
 
 import numpy as np
@@ -104,6 +105,12 @@ class Bundle:
         return [s.materials[i] for i in range(s.n_materials)]
 
 
+class _Block(np.ndarray):
+    """Bytes of a _ResultMemory; `taken`: when they were last handed out to be written."""
+
+    taken = 0.0
+
+
 class _Lease:
     """One block of a _ResultMemory for as long as an array lies in it."""
 
@@ -126,9 +133,14 @@ class _ResultMemory:
     The driver copies into memory that is mapped already at 170 GB/s, into fresh pages at a tenth of
     that (the hits of a million rays: 0.26 against 2 ms).  At most LIMIT bytes wait here unused; they go
     with the context.  Blocks come back in whatever thread drops the last array: the deque's appends
-    and pops are atomic."""
+    and pops are atomic.
+
+    A block handed out longer than STALE seconds ago is let go instead: on some hosts the device's
+    copy into memory that has lain mapped for a while is slower than into fresh pages (16 films, 176 MB
+    together, each written every 0.65 s: 1 ms on some hosts, 24 on average on others, fresh pages 7)."""
 
     LIMIT = 512 << 20
+    STALE = 0.1
     SMALL = 1 << 16  # below this the C allocator reuses mapped memory itself
 
     def __init__(self):
@@ -139,19 +151,22 @@ class _ResultMemory:
         nbytes = (shape if isinstance(shape, int) else math.prod(shape)) * dtype.itemsize
         if nbytes < self.SMALL:
             return np.zeros(shape, dtype)
-        block, others = None, []
+        block, others, now = None, [], time.monotonic()
         while block is None:
             try:
                 b = self._free.pop()  # the latest first
             except IndexError:
                 break
+            if now - b.taken > self.STALE:
+                continue
             if nbytes <= b.nbytes <= 2 * nbytes:
                 block = b
             else:
                 others.append(b)
         self._free.extendleft(others)
         if block is None:
-            block = np.empty(nbytes, np.uint8)
+            block = np.empty(nbytes, np.uint8).view(_Block)
+        block.taken = now
         return np.asarray(_Lease(block, nbytes, self)).view(dtype).reshape(shape)
 
     def give(self, block: np.ndarray) -> None:
