@@ -135,18 +135,19 @@ class _ResultMemory:
     with the context.  Blocks come back in whatever thread drops the last array: the deque's appends
     and pops are atomic.
 
-    A block handed out longer than STALE seconds ago is let go instead: on some hosts the device's
+    A block handed out longer than `stale` seconds ago is let go instead: on some hosts the device's
     copy into memory that has lain mapped for a while is slower than into fresh pages (16 films, 176 MB
-    together, each written every 0.65 s: 1 ms on some hosts, 24 on average on others, fresh pages 7)."""
+    together, each written every 0.65 s: 1 ms on some hosts, 24 on average on others, fresh pages 7).  Films, whose
+    calls may be that far apart, ask for it (FILM_STALE)."""
 
     LIMIT = 512 << 20
-    STALE = 0.1
+    FILM_STALE = 0.1
     SMALL = 1 << 16  # below this the C allocator reuses mapped memory itself
 
     def __init__(self):
         self._free = collections.deque()
 
-    def array(self, shape, dtype) -> np.ndarray:
+    def array(self, shape, dtype, stale: float = math.inf) -> np.ndarray:
         dtype = np.dtype(dtype)
         nbytes = (shape if isinstance(shape, int) else math.prod(shape)) * dtype.itemsize
         if nbytes < self.SMALL:
@@ -157,7 +158,7 @@ class _ResultMemory:
                 b = self._free.pop()  # the latest first
             except IndexError:
                 break
-            if now - b.taken > self.STALE:
+            if now - b.taken > stale:
                 continue
             if nbytes <= b.nbytes <= 2 * nbytes:
                 block = b
@@ -247,7 +248,7 @@ class Context:
             views = [views]
         arr = (capi.bn_view * len(views))(*views)
         total = sum(v.width * v.height * 3 for v in views)
-        out = self._results.array(total, np.float32) if to_host else None
+        out = self._results.array(total, np.float32, self._results.FILM_STALE) if to_host else None
         self._check(self.lib.bn_render(self._h, C.byref(desc), arr, len(views), ptr(out)))
         if not to_host:
             return None

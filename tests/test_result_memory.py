@@ -83,15 +83,13 @@ def test_threads_never_share_a_block():
 
 def test_blocks_written_long_ago_are_let_go():
     m = _ResultMemory()
-    m.STALE = 1e9
     a, b = m.array(1 << 20, np.uint8), m.array(1 << 20, np.uint8)
     at = {address(a), address(b)}
     del a, b
-    c = m.array(1 << 20, np.uint8)
+    c = m.array(1 << 20, np.uint8, stale=1e9)
     assert address(c) in at and len(m._free) == 1
     del c
-    m.STALE = -1  # now both are older than that
-    d = m.array(1 << 20, np.uint8)
+    d = m.array(1 << 20, np.uint8, stale=-1)  # both are older than that
     assert not m._free
     del d
     assert len(m._free) == 1
