@@ -168,6 +168,7 @@ SIGNATURES = {
     "bn_image_write_png": (C.c_int, [C.c_char_p, P, C.c_int32, C.c_int32]),
     "bn_render_noalloc": (C.c_int, [P, C.POINTER(bn_render_desc), C.POINTER(bn_view), C.c_int32, P]),
     "bn_set_limits": (C.c_int, [P, C.c_int32, C.c_int32]),
+    "bn_set_memory_limit": (C.c_int, [P, C.c_int64]),
     "bn_get_stats": (C.c_int, [P, C.POINTER(bn_stats)]),
     "bn_reset_stats": (C.c_int, [P]),
     "bn_forward": (C.c_int, [P, C.POINTER(bn_adjoint_desc), P, P, P]),

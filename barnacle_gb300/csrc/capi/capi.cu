@@ -399,6 +399,14 @@ int bn_set_limits(bn_context* ctx, int32_t stack_entries, int32_t max_bounce_ite
   return BN_OK;
 }
 
+int bn_set_memory_limit(bn_context* ctx, int64_t path_state_bytes) {
+  if (!ctx) return BN_ERR_INVALID_ARG;
+  if (path_state_bytes < 0) return ctx->fail(BN_ERR_INVALID_ARG, "bn_set_memory_limit: bytes >= 0 (0 = no limit)");
+  cudaSetDevice(ctx->device);
+  bnc::set_path_memory_limit(ctx, static_cast<size_t>(path_state_bytes));
+  return BN_OK;
+}
+
 int bn_get_stats(const bn_context* ctx, bn_stats* out) {
   if (!ctx || !out) return BN_ERR_INVALID_ARG;
   *out = ctx->stats;

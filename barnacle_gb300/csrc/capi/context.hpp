@@ -9,28 +9,7 @@
 #include "../device/dev_types.cuh"
 #include "../device/launch.hpp"
 #include "../device/pssmlt.hpp"
-
-// growable device buffer
-struct DevBuf {
-  void* ptr = nullptr;
-  size_t bytes = 0;
-  cudaError_t reserve(size_t n) {
-    if (n <= bytes) return cudaSuccess;
-    if (ptr) cudaFree(ptr);
-    ptr = nullptr;
-    bytes = 0;
-    cudaError_t e = cudaMalloc(&ptr, n);
-    if (e == cudaSuccess) bytes = n;
-    return e;
-  }
-  void release() {
-    if (ptr) cudaFree(ptr);
-    ptr = nullptr;
-    bytes = 0;
-  }
-  template <class T>
-  T* as() const { return static_cast<T*>(ptr); }
-};
+#include "dev_buf.hpp"
 
 namespace bnc {
 constexpr size_t kPinnedBytes = 65536;
@@ -132,6 +111,8 @@ struct PathRecords {
 // false when the path state does not fit the GPU's free memory.
 int wavefront_paths(bn_context* ctx, const bn::DevScene& scene, const bn_render_desc* d, long long n_paths,
                     const PathRecords& out, bool* ran);
+// bn_set_memory_limit: bytes of path state that a call may ask for (0: what the GPU has)
+void set_path_memory_limit(bn_context* ctx, size_t bytes);
 int render_wavefront(bn_context* ctx, const bn_render_desc* d, const std::vector<bn::DevView>& views);
 // BVHNode.Build on the GPU (bvh_gpu.cu): the host builder's nodes and permutation
 int gpu_bvh_build(bn_context* ctx, const float* bounds, int32_t n, std::vector<bn_bvh_node>* nodes,

@@ -9,15 +9,15 @@
 #include "../device/pssmlt.hpp"
 #include "../device/wavefront.hpp"
 #include "context.hpp"
+#include "path_state.hpp"
 
 namespace {
 
 struct WfState {
-  int pool = 0;
-  DevBuf params, slot, q_active, q_bins, q_done, shadow, counters, work_next, film_acc;
+  bnc::PathState paths;
+  DevBuf params, counters, work_next, hist, off;  // of one size, whatever the pool
+  DevBuf film_acc;
   DevBuf mlt_smp, mlt_chain;  // PSSMLT chains: sampler state and chain records
-  DevBuf q_key, q_ray, sh_key, q_shadow, hist, off;
-  DevBuf path_L;              // radiance per path of a batch (ordered renders)
   // captured graph (one per launch shape)
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
@@ -37,10 +37,8 @@ struct WfState {
   }
 
   void release() {
-    DevBuf* b[] = {&params, &slot, &q_active, &q_bins, &q_done, &shadow, &counters,
-                   &work_next, &film_acc, &q_key, &q_ray, &sh_key, &q_shadow, &hist, &off,
-                   &mlt_smp, &mlt_chain, &path_L};
-    for (DevBuf* x : b) x->release();
+    paths.release();
+    for (DevBuf* x : {&params, &counters, &work_next, &hist, &off, &film_acc, &mlt_smp, &mlt_chain}) x->release();
     if (exec) cudaGraphExecDestroy(exec);
     if (graph) cudaGraphDestroy(graph);
     exec = nullptr;
@@ -64,23 +62,16 @@ WfState* state(bn_context* ctx) {
   return static_cast<WfState*>(ctx->wf);
 }
 
-cudaError_t ensure_pool(WfState* w, int pool) {
-  if (w->pool == pool) return cudaSuccess;
-  cudaError_t e;
-  const size_t P = static_cast<size_t>(pool);
-  if ((e = w->params.reserve(sizeof(bn::WfParams))) != cudaSuccess) return e;
-  if ((e = w->slot.reserve(8 * P * sizeof(float4))) != cudaSuccess) return e;
-  if ((e = w->q_active.reserve(P * sizeof(int))) != cudaSuccess) return e;
-  if ((e = w->q_bins.reserve(P * bn::kNumBins * sizeof(int))) != cudaSuccess) return e;
-  if ((e = w->shadow.reserve(P * 4 * sizeof(float4))) != cudaSuccess) return e;
-  if ((e = w->counters.reserve(bn::kCntSize * sizeof(int))) != cudaSuccess) return e;
-  if ((e = w->work_next.reserve(sizeof(unsigned long long))) != cudaSuccess) return e;
-  for (DevBuf* b : {&w->q_done, &w->q_key, &w->q_ray, &w->sh_key, &w->q_shadow})
-    if ((e = b->reserve(P * sizeof(int))) != cudaSuccess) return e;
-  if ((e = w->hist.reserve(2 * bn::kSortBins * sizeof(unsigned))) != cudaSuccess) return e;
-  if ((e = w->off.reserve((bn::kSortBins + bn::kSortBins / 1024) * sizeof(unsigned))) != cudaSuccess) return e;
-  w->pool = pool;
-  return cudaSuccess;
+// what a run of `pool` slots works in, and `paths` radiances of an ordered one
+cudaError_t ensure_pool(WfState* w, int pool, long long paths = 0) {
+  cudaError_t e = w->paths.reserve(static_cast<size_t>(pool), static_cast<size_t>(paths));
+  if (e == cudaSuccess) e = w->params.reserve(sizeof(bn::WfParams));
+  if (e == cudaSuccess) e = w->counters.reserve(bn::kCntSize * sizeof(int));
+  if (e == cudaSuccess) e = w->work_next.reserve(sizeof(unsigned long long));
+  if (e == cudaSuccess) e = w->hist.reserve(2 * bn::kSortBins * sizeof(unsigned));
+  if (e == cudaSuccess) e = w->off.reserve((bn::kSortBins + bn::kSortBins / 1024) * sizeof(unsigned));
+  if (e != cudaSuccess) w->paths.release();
+  return e;
 }
 
 // Path slots of a render that does not choose them: one per path, up to 64 M (16 GB).  Every path
@@ -184,9 +175,9 @@ int run(bn_context* ctx, WfState* w, const bn::DevScene& scene, const bn_render_
   p.max_iters = static_cast<int>(std::min<long long>(1LL << 30, ((end - first) / pool + 2) * (d->max_depth + 2) + 64));
   // bn_set_limits' cap is the wavefront mode's
   if (ctx->limit_iters > 0 && !ordered) p.max_iters = ctx->limit_iters;
-  p.slot = w->slot.as<float4>();
-  p.q_active = w->q_active.as<int>();
-  p.q_done = w->q_done.as<int>();
+  p.slot = w->paths.slot.as<float4>();
+  p.q_active = w->paths.q_active.as<int>();
+  p.q_done = w->paths.q_done.as<int>();
   p.sort = sort ? 1 : 0;
   p.sort_shadow = sort_shadow ? 1 : 0;
   {
@@ -200,14 +191,14 @@ int run(bn_context* ctx, WfState* w, const bn::DevScene& scene, const bn_render_
     p.key_scale = make_float4(sc[0], sc[1], sc[2], 0.f);
     p.key_bits = key_bits;
   }
-  p.q_key = w->q_key.as<int>();
-  p.q_ray = sort ? w->q_ray.as<int>() : w->q_active.as<int>();
-  p.sh_key = w->sh_key.as<int>();
-  p.q_shadow = w->q_shadow.as<int>();
+  p.q_key = w->paths.q_key.as<int>();
+  p.q_ray = sort ? w->paths.q_ray.as<int>() : w->paths.q_active.as<int>();
+  p.sh_key = w->paths.sh_key.as<int>();
+  p.q_shadow = w->paths.q_shadow.as<int>();
   p.hist = w->hist.as<unsigned>();
   p.off = w->off.as<unsigned>();
-  p.q_bins = w->q_bins.as<int>();
-  p.shadow = w->shadow.as<float4>();
+  p.q_bins = w->paths.q_bins.as<int>();
+  p.shadow = w->paths.shadow.as<float4>();
   p.counters = w->counters.as<int>();
   p.trace_counters = ctx->counters.ptr;
   p.work_next = w->work_next.as<unsigned long long>();
@@ -313,15 +304,15 @@ int run_mlt(bn_context* ctx, WfState* w, const bn_render_desc* d, const bn::MltP
   p.max_iters = static_cast<int>(std::min<long long>(
       1LL << 30, (static_cast<long long>(mp.mutations_per_chain) + 1) * (std::max(1, d->max_depth) + 1) + 64));
   if (ctx->limit_iters > 0) p.max_iters = ctx->limit_iters;
-  p.slot = w->slot.as<float4>();
-  p.q_active = w->q_active.as<int>();
-  p.q_done = w->q_done.as<int>();
+  p.slot = w->paths.slot.as<float4>();
+  p.q_active = w->paths.q_active.as<int>();
+  p.q_done = w->paths.q_done.as<int>();
   p.sort = 0;
   p.sort_shadow = 0;
   p.key_bits = 5;
-  p.q_ray = w->q_active.as<int>();
-  p.q_bins = w->q_bins.as<int>();
-  p.shadow = w->shadow.as<float4>();
+  p.q_ray = w->paths.q_active.as<int>();
+  p.q_bins = w->paths.q_bins.as<int>();
+  p.shadow = w->paths.shadow.as<float4>();
   p.counters = w->counters.as<int>();
   p.trace_counters = ctx->counters.ptr;
   p.work_next = w->work_next.as<unsigned long long>();
@@ -349,7 +340,7 @@ int run_mlt(bn_context* ctx, WfState* w, const bn_render_desc* d, const bn::MltP
   cudaStream_t st = ctx->stream;
   cudaMemcpyAsync(w->params.ptr, &p, sizeof(p), cudaMemcpyHostToDevice, st);
   cudaMemsetAsync(w->counters.ptr, 0, bn::kCntSize * sizeof(int), st);
-  cudaMemsetAsync(w->slot.ptr, 0, static_cast<size_t>(pool) * 8 * sizeof(float4), st);  // every chain unstarted
+  cudaMemsetAsync(w->paths.slot.ptr, 0, static_cast<size_t>(pool) * 8 * sizeof(float4), st);  // every chain unstarted
   // (checking the loop condition every 4 or 16 iterations instead of every one measured slower:
   // 499 and 510 against 450 ms)
   for (int it = 0; it < p.max_iters + 1; ++it) {
@@ -379,13 +370,18 @@ int render_pssmlt_wavefront(bn_context* ctx, const bn_render_desc* d, const bn::
   return rc;
 }
 
+void set_path_memory_limit(bn_context* ctx, size_t bytes) {
+  PathState& paths = state(ctx)->paths;
+  paths.limit = bytes;
+  if (bytes && paths.held() > bytes) paths.release();
+}
+
 int render_ordered(bn_context* ctx, const bn_render_desc* d, const bn::MegaParams& p, bool* ran) {
   // batches of whole pixels with at most 128 M paths (2 GB of radiances; half a second of work)
   const long long per = std::min<long long>(p.n_pixels, std::max<long long>(1, (1LL << 27) / d->spp));
   WfState* w = state(ctx);
   const int pool = std::max(default_pool(per * d->spp), 1024);
-  cudaError_t e = w->path_L.reserve(static_cast<size_t>(per) * d->spp * sizeof(float4));
-  if (e == cudaSuccess) e = ensure_pool(w, pool);
+  cudaError_t e = ensure_pool(w, pool, per * d->spp);
   if (e == cudaErrorMemoryAllocation) {
     cudaGetLastError();
     return BN_OK;  // *ran is false: the caller renders without path state
@@ -396,14 +392,14 @@ int render_ordered(bn_context* ctx, const bn_render_desc* d, const bn::MegaParam
   int launches = 0;
   for (long long first = 0; first < p.n_pixels; first += per) {
     const long long n = std::min(per, p.n_pixels - first);
-    const PathRecords out{w->path_L.as<float4>(), nullptr, nullptr};
+    const PathRecords out{w->paths.path_L.as<float4>(), nullptr, nullptr};
     const int rc = run(ctx, w, ctx->scene, d, p.n_pixels, first * d->spp, (first + n) * d->spp, p.n_views, pool, 0, true,
                        &out);
     if (rc) return rc;
     loop_ms += ctx->stats.last_dominant_ms;
     launches += ctx->stats.last_launches + 1;
     cudaEventRecord(ctx->ev0, ctx->stream);
-    if ((e = bn::launch_mega_chunks(p, w->path_L.as<float4>(), first, n, ctx->stream)) != cudaSuccess)
+    if ((e = bn::launch_mega_chunks(p, w->paths.path_L.as<float4>(), first, n, ctx->stream)) != cudaSuccess)
       return ctx->cuda_fail(e, "ordered sums");
     if (first + n == p.n_pixels) {
       ++launches;

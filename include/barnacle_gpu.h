@@ -316,6 +316,13 @@ int bn_reset_stats(bn_context* ctx);
  * BN_ERR_DEVICE and the context stays usable; tests lower them to drive those paths without
  * faulting the GPU.  The limits hold for the context until changed. */
 int bn_set_limits(bn_context* ctx, int32_t stack_entries, int32_t max_bounce_iterations);
+/* Device memory that the wavefront's path state may take in a context (240 B per slot, and 16 B per
+ * path of a batch in megakernel mode; 0 = what the GPU has).  What does not fit is done with less, as
+ * on a GPU whose memory others hold: a wavefront render that does not choose its slots halves them
+ * down to 1 M; megakernel-mode renders and the adjoint's paths run in the one kernel.  A render with
+ * a queue_capacity of its own, PSSMLT's chains in wavefront mode and fewer slots than that return
+ * BN_ERR_OUT_OF_MEMORY.  Memory held beyond the limit is given back at once. */
+int bn_set_memory_limit(bn_context* ctx, int64_t path_state_bytes);
 
 /* ---- differentiable materials (new; no reference counterpart) --------------------------
  * A parameter vector of n_slots material slots, each
