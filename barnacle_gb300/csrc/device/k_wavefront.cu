@@ -135,7 +135,11 @@ __global__ void __launch_bounds__(256) k_wf_regen(const WfParams* __restrict__ p
   const bool fresh = p.counters[kCntIter] == 0;  // every slot is free
   const int n = fresh ? p.pool : min(p.counters[kCntRetire], p.pool);
   const int rows = (n + 31) >> 5;
-  const long long claimed = fresh ? 0 : static_cast<long long>(*p.work_next);  // (by now, or more)
+  // claimed by now, or more.  Other warps count it up meanwhile, so one lane reads it for all: the warp
+  // leaves the loop below together.
+  long long claimed = 0;
+  if (!fresh && lane == 0) claimed = static_cast<long long>(*reinterpret_cast<volatile unsigned long long*>(p.work_next));
+  claimed = __shfl_sync(0xffffffffu, claimed, 0);
   if (fresh && warp == 0 && lane == 0) {
     const long long all = p.total_paths - p.first_path;
     const int got = static_cast<int>(all < p.pool ? all : p.pool);
