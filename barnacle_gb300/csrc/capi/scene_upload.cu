@@ -100,7 +100,8 @@ struct Collapse {
     float box[6][4];
     int ref[4] = {0, 0, 0, 0};
     for (int s = 0; s < 4; ++s) {
-      if (slot[s] < 0) {
+      // (an empty leaf, which an infinite extent splits off, has no code: nothing is there to enter)
+      if (slot[s] < 0 || (b[slot[s]].is_leaf && b[slot[s]].count == 0)) {
         for (int r = 0; r < 6; ++r) box[r][s] = nan;
         continue;
       }
@@ -111,7 +112,7 @@ struct Collapse {
       }
       if (n.is_leaf) {
         const int last = static_cast<uint8_t>(n.count) - 1;
-        codes = codes && last >= 0 && last < (1 << leaf_bits);
+        codes = codes && last < (1 << leaf_bits);
         ref[s] = static_cast<int>(~((static_cast<unsigned>(n.right_or_offset) << leaf_bits) | static_cast<unsigned>(last)));
       } else {
         ref[s] = emit(slot[s]);  // grows out: the record is written by index below
@@ -500,6 +501,14 @@ extern "C" int bn_scene_upload(bn_context* ctx, const bn_scene_desc* d) {
   for (int i = 0; i < d->n_meshes; ++i)
     if (!mp[i].on_device)
       for (size_t k = 0; k < mp[i].nodes.size(); ++k) put_node(&nodes[2 * (blas0 + mp[i].node_base + k)], mp[i].nodes[k]);
+  // A mesh without triangles is one empty leaf, which has no code to be entered by in the wide walk.  Its box
+  // is NaN on the device, which no ray passes; the counting walk counts it as before.
+  for (int i = 0; i < d->n_meshes; ++i)
+    if (d->meshes[i].n_triangles == 0) {
+      bn_bvh_node none = mp[i].nodes[0];
+      for (int a = 0; a < 3; ++a) none.bounds_min[a] = none.bounds_max[a] = std::numeric_limits<float>::quiet_NaN();
+      put_node(&nodes[2 * (blas0 + mp[i].node_base)], none);
+    }
   // wide records for every BVH with an interior root (the TLAS's first, at record 0) when the
   // scene is walked wide: asked for, or automatically for scenes of 1,024+ nodes
   if (d->bvh_width != BN_BVH_AUTO && d->bvh_width != BN_BVH_BINARY && d->bvh_width != BN_BVH_WIDE)

@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(128) k_wide_fill(WideParams p) {
   int ref[4] = {0, 0, 0, 0};
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    if (slot[k] < 0) {
+    if (slot[k] < 0 || (s[k].leaf() && ((s[k].bytes >> 16) & 0xffu) == 0)) {  // unused, or an empty leaf
 #pragma unroll
       for (int r = 0; r < 6; ++r) box[r][k] = __int_as_float(0x7fc00000);
       continue;
@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(128) k_wide_fill(WideParams p) {
     }
     if (s[k].leaf()) {
       const int last = static_cast<int>((s[k].bytes >> 16) & 0xffu) - 1;
-      if (last < 0 || last >= (1 << p.leaf_bits)) atomicOr(p.flags, 2);
+      if (last >= (1 << p.leaf_bits)) atomicOr(p.flags, 2);
       ref[k] = static_cast<int>(~((static_cast<unsigned>(s[k].link) << p.leaf_bits) | static_cast<unsigned>(last)));
     } else {
       ref[k] = record_of(p, slot[k] - p.base);
