@@ -149,6 +149,7 @@ extern "C" int bn_bvh_build_device(bn_context* ctx, const float* bounds, int32_t
     std::vector<bn_bvh_node> nv;
     std::vector<int32_t> pv;
     if (!bnh::bvh_build(bounds, n, &nv, &pv)) return ctx->fail(BN_ERR_UNSUPPORTED, "BVH leaf larger than 127 items");
+    if (!bnh::fits_two_n(nv, n)) return ctx->fail(BN_ERR_UNSUPPORTED, "BVH of more than 2 n nodes");
     std::copy(nv.begin(), nv.end(), nodes);
     *n_nodes = static_cast<int32_t>(nv.size());
     std::copy(pv.begin(), pv.end(), perm);

@@ -33,6 +33,7 @@ int bn_bvh_build(const float* bounds, int32_t n, bn_bvh_node* nodes_out, int32_t
   std::vector<int32_t> perm;
   const bool ok = bnh::bvh_build(bounds, n, &nodes, &perm);
   if (!ok) return host_fail(BN_ERR_UNSUPPORTED, "bn_bvh_build: a depth-capped leaf holds more than 127 items");
+  if (!bnh::fits_two_n(nodes, n)) return host_fail(BN_ERR_UNSUPPORTED, "bn_bvh_build: a tree of more than 2 n nodes");
   std::memcpy(nodes_out, nodes.data(), nodes.size() * sizeof(bn_bvh_node));
   if (n > 0) std::memcpy(perm_out, perm.data(), perm.size() * sizeof(int32_t));
   *n_nodes_out = static_cast<int32_t>(nodes.size());

@@ -363,12 +363,13 @@ typedef struct bn_bvh_node {
 } bn_bvh_node;
 
 /* BVHNode.Build (Util/BVH.fs:239-247): bounds = n * 6 floats (min xyz, max xyz).
- * nodes_out must hold 2n nodes; perm_out[k] = original index of the k-th item after the
- * in-place permutation. */
+ * nodes_out must hold 2n nodes (one for n = 0); perm_out[k] = original index of the k-th item after
+ * the in-place permutation.  A tree of more nodes, which boxes of infinite extent can make, is refused
+ * (BN_ERR_UNSUPPORTED). */
 int bn_bvh_build(const float* bounds, int32_t n, bn_bvh_node* nodes_out, int32_t* n_nodes_out,
                  int32_t* perm_out);
 /* The same build on the GPU of ctx, with the same nodes and permutation: node ranges above 256
- * items are split level by level on the device, smaller ones by one device thread each.  Boxes
+ * items are split level by level on the device, smaller ones by a warp each.  Boxes
  * with a NaN coordinate are built by the host builder. */
 int bn_bvh_build_device(bn_context* ctx, const float* bounds, int32_t n, bn_bvh_node* nodes_out,
                         int32_t* n_nodes_out, int32_t* perm_out);
