@@ -134,6 +134,7 @@ extern "C" int bn_bvh_build_device(bn_context* ctx, const float* bounds, int32_t
   if ((!bounds && n > 0) || !nodes || !n_nodes || (!perm && n > 0) || n < 0)
     return ctx->fail(BN_ERR_INVALID_ARG, "bn_bvh_build_device: null pointer or negative count");
   cudaSetDevice(ctx->device);
+  const bnc::TrimAtExit trim{ctx->bvh};
   cudaError_t e;
   bool nan = n == 0;
   int count = 0;
@@ -162,6 +163,5 @@ extern "C" int bn_bvh_build_device(bn_context* ctx, const float* bounds, int32_t
   cudaMemcpyAsync(perm, ctx->bvh.perm.ptr, static_cast<size_t>(n) * sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream);
   if ((e = cudaStreamSynchronize(ctx->stream)) != cudaSuccess) return ctx->cuda_fail(e, "BVH download");
   *n_nodes = count;
-  ctx->bvh.trim();
   return BN_OK;
 }

@@ -21,6 +21,11 @@ struct BvhWork {
   void trim();                    // frees what is too large to keep
   void release();
 };
+// trims a call's buffers however the call ends
+struct TrimAtExit {
+  BvhWork& work;
+  ~TrimAtExit() { work.trim(); }
+};
 }  // namespace bnc
 
 struct bn_context {

@@ -374,6 +374,7 @@ extern "C" int bn_scene_upload(bn_context* ctx, const bn_scene_desc* d) {
   if (!d) return ctx->fail(BN_ERR_INVALID_ARG, "bn_scene_upload: null scene");
   cudaSetDevice(ctx->device);
   ctx->has_scene = false;
+  const bnc::TrimAtExit trim{ctx->bvh};
   // ---- validation
   if (d->n_instances <= 0 || !d->instances) return ctx->fail(BN_ERR_INVALID_ARG, "scene has no instances");
   if (d->n_primitives < 0 || (d->n_primitives > 0 && !d->primitives)) return ctx->fail(BN_ERR_INVALID_ARG, "bad primitives");
@@ -677,7 +678,6 @@ extern "C" int bn_scene_upload(bn_context* ctx, const bn_scene_desc* d) {
   if ((e = upload(ctx->tri_pdf, tri_pdf, st)) != cudaSuccess) return ctx->cuda_fail(e, "upload triangle pdf");
   if ((e = upload(ctx->tri_lights, tl, st)) != cudaSuccess) return ctx->cuda_fail(e, "upload light table");
   if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return ctx->cuda_fail(e, "scene upload");
-  ctx->bvh.trim();
 
   bn::DevScene& s = ctx->scene;
   s.nodes = ctx->nodes.as<float4>();
