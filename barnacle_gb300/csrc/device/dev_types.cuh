@@ -127,4 +127,21 @@ __host__ __device__ inline int leaf_count_bits(long long n) {
   return bits;
 }
 
+// n / d for n >= 0: almost every n fits 32 bits, whose division is a fraction of the 64-bit one
+__host__ __device__ inline long long div_small(long long n, int d) {
+  if (n >> 32 == 0) return static_cast<unsigned>(n) / static_cast<unsigned>(d);
+  return n / d;
+}
+
+// Item `local` of a view of width x height pixels: items are chunk-major, pixels row-major inside a
+// chunk, and a view may have more pixels than an int counts.
+struct ItemPlace {
+  int chunk, x, y;
+};
+__host__ __device__ inline ItemPlace item_place(long long local, int width, int height) {
+  const long long npix = static_cast<long long>(width) * height, chunk = local / npix, pix = local - chunk * npix;
+  const long long y = div_small(pix, width);
+  return {static_cast<int>(chunk), static_cast<int>(pix - y * width), static_cast<int>(y)};
+}
+
 }  // namespace bn

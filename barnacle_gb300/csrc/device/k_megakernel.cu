@@ -34,13 +34,10 @@ struct MegaTask {
       if (item >= p.n_items) return false;
       vi = find_view(p.item_offsets, p.n_views, item);
       const DevView& v = p.views[vi];
-      const long long local = item - __ldg(&p.item_offsets[vi]);
-      const long long npix = static_cast<long long>(v.width) * v.height;
-      const int chunk = static_cast<int>(local / npix);
-      const int pix = static_cast<int>(local - chunk * npix);
-      y = pix / v.width;
-      x = pix - y * v.width;
-      sid = chunk * p.spc;
+      const ItemPlace at = item_place(item - __ldg(&p.item_offsets[vi]), v.width, v.height);
+      x = at.x;
+      y = at.y;
+      sid = at.chunk * p.spc;
       s1 = min(p.spp, sid + p.spc);
       acc = mk(0.f, 0.f, 0.f);
     }

@@ -115,12 +115,6 @@ __device__ __forceinline__ void put2(float4* p, float4 a, float4 b) {
                : "memory");
 }
 
-// n / d for n >= 0: almost every n fits 32 bits, whose division is a fraction of the 64-bit one
-__device__ __forceinline__ long long div_small(long long n, int d) {
-  if (n >> 32 == 0) return static_cast<unsigned>(n) / static_cast<unsigned>(d);
-  return n / d;
-}
-
 // One warp takes kRegenRows rows of 32 ended paths at a time: their records are loaded together, so a
 // warp has that many independent loads in flight instead of one dependent chain per row, and the
 // path claims and queue appends of all its rows share one atomic each.
