@@ -14,6 +14,7 @@ struct DevBuf {
     bytes = 0;
     cudaError_t e = cudaMalloc(&ptr, n);
     if (e == cudaSuccess) bytes = n;
+    else cudaGetLastError();  // reported here: the next launch's check would report it again
     return e;
   }
   void release() {
