@@ -20,12 +20,12 @@ int prepare(bn_context* ctx, const bn_adjoint_desc* d, const float* params, cons
   cudaError_t e;
   const size_t np = static_cast<size_t>(d->n_slots) * bn::kSlotParams;
   const long long pixels = static_cast<long long>(d->width) * d->height;
-  if ((e = ctx->adj_params.reserve(2 * np * sizeof(float))) != cudaSuccess) return ctx->cuda_fail(e, "adjoint params");
-  if ((e = ctx->adj_aux.reserve(static_cast<size_t>(pixels) * d->spp * sizeof(float4))) != cudaSuccess)
+  if ((e = ctx->reserve(ctx->adj_params, 2 * np * sizeof(float))) != cudaSuccess) return ctx->cuda_fail(e, "adjoint params");
+  if ((e = ctx->reserve(ctx->adj_aux, static_cast<size_t>(pixels) * d->spp * sizeof(float4))) != cudaSuccess)
     return ctx->cuda_fail(e, "adjoint path radiance");
-  if ((e = ctx->adj_image.reserve(static_cast<size_t>(pixels) * 3 * sizeof(float))) != cudaSuccess)
+  if ((e = ctx->reserve(ctx->adj_image, static_cast<size_t>(pixels) * 3 * sizeof(float))) != cudaSuccess)
     return ctx->cuda_fail(e, "adjoint image");
-  if ((e = ctx->views.reserve(sizeof(bn::DevView))) != cudaSuccess) return ctx->cuda_fail(e, "adjoint view");
+  if ((e = ctx->reserve(ctx->views, sizeof(bn::DevView))) != cudaSuccess) return ctx->cuda_fail(e, "adjoint view");
   bn_view v{};
   v.camera = d->camera;
   v.width = d->width;
@@ -73,12 +73,12 @@ bool patch_buffers(bn_context* ctx, const bn_adjoint_desc* d, bn::AdjParams* p, 
   const long long n = p->n_pixels * d->spp;
   const size_t mats = static_cast<size_t>(ctx->scene.n_mats + 1) * sizeof(bn::DevMaterial);
   const size_t lights = static_cast<size_t>(ctx->n_lights + 1) * sizeof(bn::DevLight);
-  cudaError_t e = ctx->adj_scene.reserve(mats + lights);
+  cudaError_t e = ctx->reserve(ctx->adj_scene, mats + lights);
   p->patched = ctx->scene;
   if (e == cudaSuccess && record) {
     // 17 bytes a vertex, up to 4 GB of them; longer paths are traced again in the adjoint
     if (n > (4LL << 30) / 17 / d->max_depth) return false;
-    e = ctx->adj_rec.reserve(static_cast<size_t>(n) * d->max_depth * (sizeof(float4) + 1));
+    e = ctx->reserve(ctx->adj_rec, static_cast<size_t>(n) * d->max_depth * (sizeof(float4) + 1));
     p->rec = ctx->adj_rec.as<float4>();
     p->lit = reinterpret_cast<unsigned char*>(p->rec + n * d->max_depth);
   }
@@ -175,9 +175,9 @@ extern "C" int bn_backward(bn_context* ctx, const bn_adjoint_desc* d, const floa
   if (rc) return rc;
   cudaError_t e;
   const size_t np = static_cast<size_t>(d->n_slots) * bn::kSlotParams;
-  if ((e = ctx->adj_target.reserve(static_cast<size_t>(p.n_pixels) * 3 * sizeof(float))) != cudaSuccess)
+  if ((e = ctx->reserve(ctx->adj_target, static_cast<size_t>(p.n_pixels) * 3 * sizeof(float))) != cudaSuccess)
     return ctx->cuda_fail(e, "adjoint target");
-  if ((e = ctx->adj_grad.reserve((np + 1) * sizeof(double))) != cudaSuccess) return ctx->cuda_fail(e, "adjoint gradient");
+  if ((e = ctx->reserve(ctx->adj_grad, (np + 1) * sizeof(double))) != cudaSuccess) return ctx->cuda_fail(e, "adjoint gradient");
   cudaStream_t st = ctx->stream;
   cudaMemcpyAsync(ctx->adj_target.ptr, target_image, static_cast<size_t>(p.n_pixels) * 3 * sizeof(float),
                   cudaMemcpyHostToDevice, st);

@@ -42,14 +42,14 @@ int gpu_bvh_build_resident(bn_context* ctx, const float* bounds_device, int32_t 
   const size_t top_b = up(tops * sizeof(bn::BvhTop)), small_b = up((tops + 1) * sizeof(bn::BvhSmallRange));
   const size_t acc_b = up(segs * sizeof(bn::BvhSegAcc)), bins_b = up(segs * bn::kBvhBins * sizeof(bn::BvhBin));
   const size_t cnt_b = up(chunks * bn::kBvhBins * sizeof(int));
-  if ((e = k.items.reserve(2 * N * sizeof(bn::BvhItem))) != cudaSuccess ||
-      (e = k.ranges.reserve(top_b + small_b)) != cudaSuccess ||
-      (e = k.level.reserve(acc_b + bins_b + cnt_b + chunks * sizeof(int))) != cudaSuccess ||
-      (e = k.nodes.reserve((2 * N + 160) * sizeof(bn_bvh_node))) != cudaSuccess ||
-      (e = k.out.reserve((2 * N + 160) * sizeof(bn_bvh_node))) != cudaSuccess ||
-      (e = k.perm.reserve(N * sizeof(int))) != cudaSuccess ||
-      (odd && (e = k.odd.reserve(2 * (2 * N + 160))) != cudaSuccess) ||
-      (e = k.counters.reserve(sizeof(bn::BvhCounters))) != cudaSuccess ||
+  if ((e = ctx->reserve(k.items, 2 * N * sizeof(bn::BvhItem))) != cudaSuccess ||
+      (e = ctx->reserve(k.ranges, top_b + small_b)) != cudaSuccess ||
+      (e = ctx->reserve(k.level, acc_b + bins_b + cnt_b + chunks * sizeof(int))) != cudaSuccess ||
+      (e = ctx->reserve(k.nodes, (2 * N + 160) * sizeof(bn_bvh_node))) != cudaSuccess ||
+      (e = ctx->reserve(k.out, (2 * N + 160) * sizeof(bn_bvh_node))) != cudaSuccess ||
+      (e = ctx->reserve(k.perm, N * sizeof(int))) != cudaSuccess ||
+      (odd && (e = ctx->reserve(k.odd, 2 * (2 * N + 160))) != cudaSuccess) ||
+      (e = ctx->reserve(k.counters, sizeof(bn::BvhCounters))) != cudaSuccess ||
       (!k.host_counters &&
        (e = cudaHostAlloc(&k.host_counters, sizeof(bn::BvhCounters), cudaHostAllocDefault)) != cudaSuccess))
     return ctx->cuda_fail(e, "BVH buffers");
@@ -106,7 +106,7 @@ int gpu_bvh_build(bn_context* ctx, const float* bounds, int32_t n, std::vector<b
   bool nan = n <= 0;
   int n_nodes = 0;
   if (!nan) {
-    cudaError_t e = ctx->bvh.bounds.reserve(6 * static_cast<size_t>(n) * sizeof(float));
+    cudaError_t e = ctx->reserve(ctx->bvh.bounds, 6 * static_cast<size_t>(n) * sizeof(float));
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(ctx->bvh.bounds.ptr, bounds, 6 * static_cast<size_t>(n) * sizeof(float), cudaMemcpyHostToDevice,
                           ctx->stream);
@@ -140,7 +140,7 @@ extern "C" int bn_bvh_build_device(bn_context* ctx, const float* bounds, int32_t
   int count = 0;
   if (n > 0) {
     const size_t bytes = 6 * static_cast<size_t>(n) * sizeof(float);
-    if ((e = ctx->bvh.bounds.reserve(bytes)) != cudaSuccess ||
+    if ((e = ctx->reserve(ctx->bvh.bounds, bytes)) != cudaSuccess ||
         (e = cudaMemcpyAsync(ctx->bvh.bounds.ptr, bounds, bytes, cudaMemcpyHostToDevice, ctx->stream)) != cudaSuccess)
       return ctx->cuda_fail(e, "BVH bounds");
     const int rc = bnc::gpu_bvh_build_resident(ctx, ctx->bvh.bounds.as<float>(), n, false, &nan, &count);

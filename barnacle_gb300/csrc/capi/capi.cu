@@ -119,9 +119,9 @@ int render_megakernel(bn_context* ctx, const bn_render_desc* d, const std::vecto
     items += static_cast<long long>(views[i].width) * views[i].height * ck.chunks;
   }
   cudaError_t e;
-  if ((e = ctx->item_offsets.reserve(item_off.size() * sizeof(long long))) != cudaSuccess)
+  if ((e = ctx->reserve(ctx->item_offsets, item_off.size() * sizeof(long long))) != cudaSuccess)
     return ctx->cuda_fail(e, "alloc item offsets");
-  if ((e = ctx->partial.reserve(static_cast<size_t>(items) * sizeof(float4))) != cudaSuccess)
+  if ((e = ctx->reserve(ctx->partial, static_cast<size_t>(items) * sizeof(float4))) != cudaSuccess)
     return ctx->cuda_fail(e, "alloc partial sums");
   cudaMemcpyAsync(ctx->item_offsets.ptr, item_off.data(), item_off.size() * sizeof(long long), cudaMemcpyHostToDevice,
                   ctx->stream);
@@ -229,8 +229,8 @@ int bn_trace(bn_context* ctx, const bn_ray* rays, int64_t n, uint32_t flags, bn_
   if (n == 0) return BN_OK;
   cudaSetDevice(ctx->device);
   cudaError_t e;
-  if ((e = ctx->q_in.reserve(n * sizeof(bn_ray))) != cudaSuccess) return ctx->cuda_fail(e, "alloc rays");
-  if ((e = ctx->q_out.reserve(n * sizeof(bn_hit))) != cudaSuccess) return ctx->cuda_fail(e, "alloc hits");
+  if ((e = ctx->reserve(ctx->q_in, n * sizeof(bn_ray))) != cudaSuccess) return ctx->cuda_fail(e, "alloc rays");
+  if ((e = ctx->reserve(ctx->q_out, n * sizeof(bn_hit))) != cudaSuccess) return ctx->cuda_fail(e, "alloc hits");
   if (flags & BN_TRACE_COUNT) cudaMemsetAsync(ctx->counters.ptr, 0, sizeof(bn::DevCounters), ctx->stream);
   cudaMemcpyAsync(ctx->q_in.ptr, rays, n * sizeof(bn_ray), cudaMemcpyHostToDevice, ctx->stream);
   cudaEventRecord(ctx->ev0, ctx->stream);
@@ -273,8 +273,8 @@ static int bsdf_common(bn_context* ctx, const bn_bsdf_query* q, int64_t n, bn_bs
   if (n == 0) return BN_OK;
   cudaSetDevice(ctx->device);
   cudaError_t e;
-  if ((e = ctx->q_in.reserve(n * sizeof(bn_bsdf_query))) != cudaSuccess) return ctx->cuda_fail(e, "alloc queries");
-  if ((e = ctx->q_out.reserve(n * sizeof(bn_bsdf_result))) != cudaSuccess) return ctx->cuda_fail(e, "alloc results");
+  if ((e = ctx->reserve(ctx->q_in, n * sizeof(bn_bsdf_query))) != cudaSuccess) return ctx->cuda_fail(e, "alloc queries");
+  if ((e = ctx->reserve(ctx->q_out, n * sizeof(bn_bsdf_result))) != cudaSuccess) return ctx->cuda_fail(e, "alloc results");
   cudaMemcpyAsync(ctx->q_in.ptr, q, n * sizeof(bn_bsdf_query), cudaMemcpyHostToDevice, ctx->stream);
   if ((e = bn::launch_bsdf(ctx->scene, ctx->q_in.as<bn_bsdf_query>(), ctx->q_out.as<bn_bsdf_result>(), n, sample,
                            ctx->stream)) != cudaSuccess)
@@ -298,8 +298,8 @@ int bn_sampler_stream(bn_context* ctx, const uint32_t* seeds, int64_t n_streams,
   if (n_streams == 0 || n_draws == 0) return BN_OK;
   cudaSetDevice(ctx->device);
   cudaError_t e;
-  if ((e = ctx->q_in.reserve(n_streams * 3 * sizeof(uint32_t))) != cudaSuccess) return ctx->cuda_fail(e, "alloc seeds");
-  if ((e = ctx->q_out.reserve(n_streams * n_draws * sizeof(float))) != cudaSuccess) return ctx->cuda_fail(e, "alloc draws");
+  if ((e = ctx->reserve(ctx->q_in, n_streams * 3 * sizeof(uint32_t))) != cudaSuccess) return ctx->cuda_fail(e, "alloc seeds");
+  if ((e = ctx->reserve(ctx->q_out, n_streams * n_draws * sizeof(float))) != cudaSuccess) return ctx->cuda_fail(e, "alloc draws");
   cudaMemcpyAsync(ctx->q_in.ptr, seeds, n_streams * 3 * sizeof(uint32_t), cudaMemcpyHostToDevice, ctx->stream);
   if ((e = bn::launch_sampler_stream(ctx->q_in.as<uint32_t>(), n_streams, n_draws, ctx->q_out.as<float>(), ctx->stream)) !=
       cudaSuccess)
@@ -325,8 +325,8 @@ int bn_render(bn_context* ctx, const bn_render_desc* d, const bn_view* views, in
     paths += static_cast<long long>(views[i].width) * views[i].height * d->spp;
   }
   cudaError_t e;
-  if ((e = ctx->views.reserve(dv.size() * sizeof(bn::DevView))) != cudaSuccess) return ctx->cuda_fail(e, "alloc views");
-  if ((e = ctx->film.reserve(static_cast<size_t>(pix) * 3 * sizeof(float))) != cudaSuccess)
+  if ((e = ctx->reserve(ctx->views, dv.size() * sizeof(bn::DevView))) != cudaSuccess) return ctx->cuda_fail(e, "alloc views");
+  if ((e = ctx->reserve(ctx->film, static_cast<size_t>(pix) * 3 * sizeof(float))) != cudaSuccess)
     return ctx->cuda_fail(e, "alloc film");
   ctx->film_floats = pix * 3;
   cudaMemcpyAsync(ctx->views.ptr, dv.data(), dv.size() * sizeof(bn::DevView), cudaMemcpyHostToDevice, ctx->stream);
@@ -378,7 +378,7 @@ int bn_film_tonemap(bn_context* ctx, int32_t tone_mapping, uint8_t* rgba, int64_
   if (n_pixels <= 0 || 3 * n_pixels > ctx->film_floats)
     return ctx->fail(BN_ERR_INVALID_ARG, "bn_film_tonemap: n_pixels must be 1 .. the last render's film pixels");
   cudaSetDevice(ctx->device);
-  cudaError_t e = ctx->rgba.reserve(static_cast<size_t>(n_pixels) * 4);
+  cudaError_t e = ctx->reserve(ctx->rgba, static_cast<size_t>(n_pixels) * 4);
   if (e != cudaSuccess) return ctx->cuda_fail(e, "alloc tone-mapped film");
   if ((e = bn::launch_film_tonemap(ctx->film.as<float>(), n_pixels, tone_mapping, ctx->rgba.ptr, ctx->stream)) !=
       cudaSuccess)

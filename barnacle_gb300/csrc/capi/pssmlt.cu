@@ -55,11 +55,11 @@ int render_pssmlt(bn_context* ctx, const bn_render_desc* d, const std::vector<bn
   if (mpc_ll > (1LL << 30)) return ctx->fail(BN_ERR_INVALID_ARG, "too many mutations per chain");
   cudaError_t e;
   cudaStream_t st = ctx->stream;
-  if ((e = ctx->mlt_boot.reserve(static_cast<size_t>(d->n_bootstrap) * sizeof(float))) != cudaSuccess)
+  if ((e = ctx->reserve(ctx->mlt_boot, static_cast<size_t>(d->n_bootstrap) * sizeof(float))) != cudaSuccess)
     return ctx->cuda_fail(e, "bootstrap weights");
-  if ((e = ctx->mlt_state.reserve(static_cast<size_t>(dims) * d->n_chains * sizeof(float4))) != cudaSuccess)
+  if ((e = ctx->reserve(ctx->mlt_state, static_cast<size_t>(dims) * d->n_chains * sizeof(float4))) != cudaSuccess)
     return ctx->cuda_fail(e, "primary-sample vectors");
-  if ((e = ctx->mlt_chain.reserve(256 + 2 * static_cast<size_t>(d->n_bootstrap) * sizeof(float))) != cudaSuccess)
+  if ((e = ctx->reserve(ctx->mlt_chain, 256 + 2 * static_cast<size_t>(d->n_bootstrap) * sizeof(float))) != cudaSuccess)
     return ctx->cuda_fail(e, "chain tables");
   bn::MltParams p{};
   p.scene = ctx->scene;

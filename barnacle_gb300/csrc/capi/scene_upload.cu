@@ -173,9 +173,9 @@ void build_vose(const std::vector<double>& w, std::vector<float>* prob, std::vec
 }
 
 template <class T>
-cudaError_t upload(DevBuf& b, const std::vector<T>& v, cudaStream_t st) {
+cudaError_t upload(bn_context* ctx, DevBuf& b, const std::vector<T>& v, cudaStream_t st) {
   const size_t bytes = std::max<size_t>(v.size() * sizeof(T), 16);
-  cudaError_t e = b.reserve(bytes);
+  cudaError_t e = ctx->reserve(b, bytes);
   if (e != cudaSuccess) return e;
   if (!v.empty()) e = cudaMemcpyAsync(b.ptr, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, st);
   return e;
@@ -213,10 +213,10 @@ void mesh_tris(const bn_mesh_desc& m, const std::vector<int32_t>& perm, std::vec
 }
 
 // n bytes of b with its first `used` kept
-cudaError_t grow(DevBuf& b, size_t used, size_t n, cudaStream_t st) {
+cudaError_t grow(bn_context* ctx, DevBuf& b, size_t used, size_t n, cudaStream_t st) {
   if (n <= b.bytes) return cudaSuccess;
   DevBuf bigger;
-  cudaError_t e = bigger.reserve(n);
+  cudaError_t e = ctx->reserve(bigger, n);
   if (e == cudaSuccess && used) e = cudaMemcpyAsync(bigger.ptr, b.ptr, used, cudaMemcpyDeviceToDevice, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) {
@@ -238,9 +238,9 @@ int device_blases(bn_context* ctx, const bn_scene_desc* d, const std::vector<int
   cudaError_t e;
   size_t est = tlas_room + *blas_nodes;
   for (int i : meshes) est += static_cast<size_t>(0.8 * d->meshes[i].n_triangles) + 200;  // leaves hold 2 to 3 boxes
-  if ((e = ctx->nodes.reserve(est * sizeof(bn_bvh_node))) != cudaSuccess ||
-      (e = ctx->tris.reserve(3 * n_tris * sizeof(float4))) != cudaSuccess ||
-      (e = ctx->tri_pdf.reserve(n_tris * sizeof(float))) != cudaSuccess)
+  if ((e = ctx->reserve(ctx->nodes, est * sizeof(bn_bvh_node))) != cudaSuccess ||
+      (e = ctx->reserve(ctx->tris, 3 * n_tris * sizeof(float4))) != cudaSuccess ||
+      (e = ctx->reserve(ctx->tri_pdf, n_tris * sizeof(float))) != cudaSuccess)
     return ctx->cuda_fail(e, "scene buffers");
   const size_t first_node = *blas_nodes;
   size_t tri_base = host_tris;
@@ -250,9 +250,9 @@ int device_blases(bn_context* ctx, const bn_scene_desc* d, const std::vector<int
     const bn_mesh_desc& m = d->meshes[i];
     MeshPrep& p = (*mp)[i];
     const size_t vb = 3 * static_cast<size_t>(m.n_vertices) * sizeof(float), ib = 3 * static_cast<size_t>(nt) * sizeof(int);
-    if ((e = k.vertices.reserve(vb)) != cudaSuccess || (e = k.indices.reserve(ib)) != cudaSuccess ||
-        (m.tri_material && (e = k.slots.reserve(nt * sizeof(int))) != cudaSuccess) ||
-        (e = k.bounds.reserve(6 * static_cast<size_t>(nt) * sizeof(float))) != cudaSuccess)
+    if ((e = ctx->reserve(k.vertices, vb)) != cudaSuccess || (e = ctx->reserve(k.indices, ib)) != cudaSuccess ||
+        (m.tri_material && (e = ctx->reserve(k.slots, nt * sizeof(int))) != cudaSuccess) ||
+        (e = ctx->reserve(k.bounds, 6 * static_cast<size_t>(nt) * sizeof(float))) != cudaSuccess)
       return ctx->cuda_fail(e, "mesh buffers");
     cudaMemcpyAsync(k.vertices.ptr, m.vertices, vb, cudaMemcpyHostToDevice, st);
     cudaMemcpyAsync(k.indices.ptr, m.indices, ib, cudaMemcpyHostToDevice, st);
@@ -276,8 +276,8 @@ int device_blases(bn_context* ctx, const bn_scene_desc* d, const std::vector<int
         if (!p.nodes[n].is_leaf) odd[n + 1] = odd[p.nodes[n].right_or_offset] = !odd[n];
     }
     const size_t at = tlas_room + *blas_nodes;
-    if ((e = grow(ctx->nodes, at * sizeof(bn_bvh_node), (at + n_nodes) * sizeof(bn_bvh_node), st)) != cudaSuccess ||
-        (e = grow(k.scene_odd, *blas_nodes - first_node,
+    if ((e = grow(ctx, ctx->nodes, at * sizeof(bn_bvh_node), (at + n_nodes) * sizeof(bn_bvh_node), st)) != cudaSuccess ||
+        (e = grow(ctx, k.scene_odd, *blas_nodes - first_node,
                   std::max(*blas_nodes - first_node + n_nodes, est - tlas_room - first_node), st)) != cudaSuccess)
       return ctx->cuda_fail(e, "scene nodes");
     // bn_bvh_node is the walk's two float4 (put_node)
@@ -286,7 +286,7 @@ int device_blases(bn_context* ctx, const bn_scene_desc* d, const std::vector<int
     if (nan) {
       cudaMemcpyAsync(dst, p.nodes.data(), n_nodes * sizeof(bn_bvh_node), cudaMemcpyHostToDevice, st);
       cudaMemcpyAsync(dst_odd, odd.data(), n_nodes, cudaMemcpyHostToDevice, st);
-      if ((e = k.perm.reserve(nt * sizeof(int))) != cudaSuccess) return ctx->cuda_fail(e, "mesh permutation");
+      if ((e = ctx->reserve(k.perm, nt * sizeof(int))) != cudaSuccess) return ctx->cuda_fail(e, "mesh permutation");
       cudaMemcpyAsync(k.perm.ptr, p.perm.data(), nt * sizeof(int), cudaMemcpyHostToDevice, st);
     } else {
       cudaMemcpyAsync(dst, k.out.ptr, n_nodes * sizeof(bn_bvh_node), cudaMemcpyDeviceToDevice, st);
@@ -334,7 +334,7 @@ int device_records(bn_context* ctx, const std::vector<int>& meshes, const std::v
   const int blocks = (w.n + 1023) / 1024;
   cudaError_t e;
   // rank | block sums | flag | roots | mesh bases
-  if ((e = k.wide.reserve((static_cast<size_t>(w.n) + blocks + 2 + 1 + 2 * nm) * sizeof(int))) != cudaSuccess)
+  if ((e = ctx->reserve(k.wide, (static_cast<size_t>(w.n) + blocks + 2 + 1 + 2 * nm) * sizeof(int))) != cudaSuccess)
     return ctx->cuda_fail(e, "wide-record buffers");
   w.rank = k.wide.as<int>();
   w.sums = w.rank + w.n;
@@ -351,7 +351,7 @@ int device_records(bn_context* ctx, const std::vector<int>& meshes, const std::v
       (e = cudaMemcpyAsync(&count, w.sums + blocks, sizeof(int), cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
       (e = cudaStreamSynchronize(st)) != cudaSuccess)
     return ctx->cuda_fail(e, "wide records");
-  if ((e = ctx->nodes4.reserve((*n_records + count + 1) * 8 * sizeof(float4))) != cudaSuccess)
+  if ((e = ctx->reserve(ctx->nodes4, (*n_records + count + 1) * 8 * sizeof(float4))) != cudaSuccess)
     return ctx->cuda_fail(e, "wide records");
   w.records = ctx->nodes4.as<float4>();
   w.first_record = static_cast<int>(*n_records);
@@ -668,15 +668,15 @@ extern "C" int bn_scene_upload(bn_context* ctx, const bn_scene_desc* d) {
   cudaStream_t st = ctx->stream;
   cudaError_t e;
   // (with meshes on the device these buffers hold them already, behind the host's parts)
-  if ((e = upload(ctx->nodes, nodes, st)) != cudaSuccess) return ctx->cuda_fail(e, "upload nodes");
-  if ((e = upload(ctx->nodes4, nodes4, st)) != cudaSuccess) return ctx->cuda_fail(e, "upload wide nodes");
-  if ((e = upload(ctx->tris, tris, st)) != cudaSuccess) return ctx->cuda_fail(e, "upload triangles");
-  if ((e = upload(ctx->inst, dinst, st)) != cudaSuccess) return ctx->cuda_fail(e, "upload instances");
-  if ((e = upload(ctx->mats, mats, st)) != cudaSuccess) return ctx->cuda_fail(e, "upload materials");
-  if ((e = upload(ctx->lights, lights, st)) != cudaSuccess) return ctx->cuda_fail(e, "upload lights");
-  if ((e = upload(ctx->light_inst, light_inst, st)) != cudaSuccess) return ctx->cuda_fail(e, "upload light list");
-  if ((e = upload(ctx->tri_pdf, tri_pdf, st)) != cudaSuccess) return ctx->cuda_fail(e, "upload triangle pdf");
-  if ((e = upload(ctx->tri_lights, tl, st)) != cudaSuccess) return ctx->cuda_fail(e, "upload light table");
+  if ((e = upload(ctx, ctx->nodes, nodes, st)) != cudaSuccess) return ctx->cuda_fail(e, "upload nodes");
+  if ((e = upload(ctx, ctx->nodes4, nodes4, st)) != cudaSuccess) return ctx->cuda_fail(e, "upload wide nodes");
+  if ((e = upload(ctx, ctx->tris, tris, st)) != cudaSuccess) return ctx->cuda_fail(e, "upload triangles");
+  if ((e = upload(ctx, ctx->inst, dinst, st)) != cudaSuccess) return ctx->cuda_fail(e, "upload instances");
+  if ((e = upload(ctx, ctx->mats, mats, st)) != cudaSuccess) return ctx->cuda_fail(e, "upload materials");
+  if ((e = upload(ctx, ctx->lights, lights, st)) != cudaSuccess) return ctx->cuda_fail(e, "upload lights");
+  if ((e = upload(ctx, ctx->light_inst, light_inst, st)) != cudaSuccess) return ctx->cuda_fail(e, "upload light list");
+  if ((e = upload(ctx, ctx->tri_pdf, tri_pdf, st)) != cudaSuccess) return ctx->cuda_fail(e, "upload triangle pdf");
+  if ((e = upload(ctx, ctx->tri_lights, tl, st)) != cudaSuccess) return ctx->cuda_fail(e, "upload light table");
   if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return ctx->cuda_fail(e, "scene upload");
 
   bn::DevScene& s = ctx->scene;

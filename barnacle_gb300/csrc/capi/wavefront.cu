@@ -58,6 +58,12 @@ WfState* state(bn_context* ctx) {
       s->release();
       delete s;
     };
+    ctx->wf_spare = [](void* p) {
+      auto* s = static_cast<WfState*>(p);
+      const bool held = s->paths.held() > 0;
+      s->paths.release();
+      return held;
+    };
   }
   return static_cast<WfState*>(ctx->wf);
 }

@@ -321,7 +321,9 @@ int bn_set_limits(bn_context* ctx, int32_t stack_entries, int32_t max_bounce_ite
  * on a GPU whose memory others hold: a wavefront render that does not choose its slots halves them
  * down to 1 M; megakernel-mode renders and the adjoint's paths run in the one kernel.  A render with
  * a queue_capacity of its own, PSSMLT's chains in wavefront mode and fewer slots than that return
- * BN_ERR_OUT_OF_MEMORY.  Memory held beyond the limit is given back at once. */
+ * BN_ERR_OUT_OF_MEMORY.  Memory held beyond the limit is given back at once.  (The state of a render
+ * stays with the context for the next one, up to 18 GB, and goes when another of the context's buffers
+ * finds no memory.) */
 int bn_set_memory_limit(bn_context* ctx, int64_t path_state_bytes);
 
 /* ---- differentiable materials (new; no reference counterpart) --------------------------

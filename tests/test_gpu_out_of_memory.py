@@ -29,3 +29,16 @@ def test_the_next_call_does_not_report_it_again():
         want = c.render(b.render, b.views)[0].copy()
         ask_too_much(c)
         np.testing.assert_array_equal(c.render(b.render, b.views)[0], want)
+
+
+def test_the_path_state_makes_room_for_other_buffers():
+    """What a render of 4 M paths leaves (1 GB) goes when another buffer finds no memory, and comes back."""
+    torch = pytest.importorskip("torch")
+    with Context(0) as c:
+        b = Bundle.generate("cornell", 1)
+        c.upload(b)
+        want = c.render(b.render, b.views)[0].copy()
+        held = torch.cuda.mem_get_info(0)[0]
+        ask_too_much(c)
+        assert torch.cuda.mem_get_info(0)[0] - held >= 0.9 * (256 * 256 * 64 * 256)
+        np.testing.assert_array_equal(c.render(b.render, b.views)[0], want)
