@@ -131,14 +131,17 @@ class _ResultMemory:
     """Host memory for a context's large results, used again once nobody holds an array in it.
 
     The driver copies into memory that is mapped already at 170 GB/s, into fresh pages at a tenth of
-    that (the hits of a million rays: 0.26 against 2 ms).  At most LIMIT bytes wait here unused; they go
+    that (the hits of a million rays: 0.26 against 2 ms).  A caller that keeps its results, and the first
+    call of a size, get fresh pages.  At most LIMIT bytes wait here unused; they go
     with the context.  Blocks come back in whatever thread drops the last array: the deque's appends
     and pops are atomic.
 
     A block handed out longer than `stale` seconds ago is let go instead: on some hosts the device's
     copy into memory that has lain mapped for a while is slower than into fresh pages (16 films, 176 MB
-    together, each written every 0.65 s: 1 ms on some hosts, 24 on average on others, fresh pages 7).  Films, whose
-    calls may be that far apart, ask for it (FILM_STALE)."""
+    together, each written every 0.65 s: 1 ms on some hosts, 24 on average on others, fresh pages 7).
+    render()'s films ask for it (FILM_STALE), of any size: only the large ones were measured, and a film
+    that gets fresh pages is copied as fast as before there was this memory.  forward()'s images do not:
+    a fit renders one every few milliseconds."""
 
     LIMIT = 512 << 20
     FILM_STALE = 0.1

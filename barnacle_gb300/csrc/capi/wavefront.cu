@@ -84,9 +84,9 @@ cudaError_t ensure_pool(WfState* w, int pool, long long paths = 0) {
 // then starts at once, the queues are as long and the sorted rays as coherent as they can be, and
 // a bounce is one iteration; fewer slots cost more, short iterations, more slots only add rows to
 // scan.  Measured (kernel ms by log2 of the slots, the render's paths in brackets): Cornell box
-// [2^22] 20: 7.04, 21: 6.47, 22: 6.17, 23: 6.70; Cornell with objects [2^23] 21: 25.2, 22: 23.1,
-// 23: 22.7, 24: 23.8; 16 instanced views [2^25.8] 23: 292, 24: 283, 25: 278, 26: 278.  A cap of 2
-// blocks per SM was 1.8 times slower at every one of them.
+// [2^22] 20: 6.07, 21: 5.43, 22: 4.90, 23: 5.00; Cornell with objects [2^23] 21: 20.8, 22: 18.5,
+// 23: 17.0, 24: 17.0; 16 instanced views [2^25.8] 22: 230.5, 23: 218.2, 24: 211.1, 25: 205.5, 26: 199.5.
+// A cap of 2 blocks per SM was 1.8 times slower at every one of them.
 int default_pool(long long paths) {
   return static_cast<int>(std::min<long long>(1LL << 26, (paths + 1023) / 1024 * 1024));
 }

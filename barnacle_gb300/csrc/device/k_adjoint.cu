@@ -18,8 +18,8 @@
 // run on the path machine or, from 0.8 M on, through the wavefront's queues, which leave each vertex's
 // hit (16 bytes) and whether its light sample was lit (a byte).  The adjoint then replays the paths
 // from those records without tracing a ray (k_adj_replay).  256^2, 16 spp, 32 slots, depth 8:
-// the gradient call 15.6 -> 4.7 ms (the adjoint's kernel 9.7 -> 0.85, the paths 5.9 -> 3.6), a forward
-// render of 128 spp 43.7 -> 13.4 ms.
+// the gradient call 15.6 -> 4.0 ms (the adjoint's kernel 9.7 -> 0.92, the paths 5.9 -> 3.0), a forward
+// render of 128 spp 43.7 -> 11.5 ms.
 #define BN_COMPACT
 #include <algorithm>
 

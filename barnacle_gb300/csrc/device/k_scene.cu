@@ -3,7 +3,7 @@
 //
 // Each kernel reads and writes its arrays once.  The same loops on one host core, with the copies
 // they needed, were 22 of the 28 ms in which the scene of 630,083 triangles was uploaded; it now takes
-// 5.4 ms, most of it the builds (k_bvh.cu) and the copies of vertices and indices.
+// 5.1 ms, most of it the builds (k_bvh.cu) and the copies of vertices and indices.
 #include <cstdint>
 
 #include "dev_geometry.cuh"

@@ -38,8 +38,9 @@ constexpr bool kWfInstRun = true;
 // Six instanced views of 4 spp took 82.2 ms; extend at 8 or 6 blocks with shadow at 8: 83.2 and 83.5, shadow
 // at 7 or 9 with extend at 7: 82.4 and 83.2.
 constexpr int kExtendBlocks = 7, kShadowBlocks = 8;
-// a traversal warp refills once at most this many of its lanes still walk (12 / 16 / 20 / 24 measured
-// 192.9 / 193.7 / 191.6 / 187.8 M paths/s on the instanced workload, when the mode vote came in)
+// A traversal warp refills once at most this many of its lanes still walk.  12 / 16 / 20 / 24: Cornell box
+// 4.81 / 4.89 / 5.00 / 5.14 ms, Cornell with objects 16.8 / 17.0 / 17.3 / 18.0, six instanced views of 4 spp
+// 70.3 / 70.7 / 71.9 / 74.0 (16 was the best, by 0.4 %, when the mode vote came in).
 constexpr int kWfRefill = 16;
 // stack entries per lane kept in shared memory (8 bytes each, x 128 lanes per block)
 constexpr int kWfSharedStack = 16;
@@ -436,7 +437,7 @@ __device__ __forceinline__ void tile_fetch(RecordTile& t, const float4* slots, i
 // Bound by the latency of its loads.  Each warp keeps two tiles: the records of its next 32 paths come
 // in while it shades the present 32.  Kernel time of a whole render, against reading the records lane by
 // lane: Cornell 5.95 -> 5.65 ms, the material scene 20.8 -> 19.8, instances 91.9 -> 89.2.  5 blocks per SM
-// (36 KB of tiles each); 4 measured the same, 6 slower.
+// (32 KB of tiles each); 4 measured the same, 6 slower.
 template <bool kWT>
 __global__ void __launch_bounds__(128, 5) k_wf_shade(const WfParams* __restrict__ pp) {
   const WfParams& p = *pp;

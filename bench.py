@@ -225,7 +225,8 @@ def run_extras(ctx, args, torch, flush):
     out["cornell"] = {"gpu_paths_per_s": gpu0, "gpu_ms": min(ms), "cpu_paths_per_s": pc / sc, "cpu_cores": threads,
                       "cpu_sample": f"{len(tiles)} 16x16 tiles x 64 spp (every cell of a 4x4 grid, twice)",
                       "gpu_over_cpu": gpu0 / (pc / sc)}
-    # PSSMLT: the chains one thread each in lockstep, and compacted every bounce in the wavefront
+    # PSSMLT: the chains a lane each on the path machine ("lockstep", the key of earlier runs), and compacted
+    # every bounce in the wavefront
     c3 = Bundle.generate("pssmlt", 1)
     ctx.upload(c3)
     out["pssmlt"] = {}
@@ -558,7 +559,7 @@ def main():
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": None if traffic is None else traffic["bytes_per_launch"],
                          "traffic_source": None if traffic is None else traffic["source"], "peak_kind": peak_kind,
-                         "kernel": "k_pt_mega" if args.mode == "megakernel" else
+                         "kernel": "k_pt_machine or k_pt_mega" if args.mode == "megakernel" and paths_per_step < 3 << 18 else
                                    "wavefront bounce loop (regen+sort+extend+shade+shadow, one graph launch)",
                          "alg_bytes_per_launch": int(alg_bytes), "l2": prof.get("l2", {}).get(args.mode)},
             "cpu_baseline": cpu,
